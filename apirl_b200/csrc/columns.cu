@@ -1,0 +1,579 @@
+// Kernels of the column walk (columns.cuh): projection, backprojection and the
+// fused EM pass of 3D sinograms with one float ray per bin, and the copies
+// between images and the column layout.
+//
+// A block takes one (angle, r) of the subset and all the sinograms of the
+// shard, 32 to a warp at a time.  Blocks run r first, then angle: neighbours
+// in r share columns in L1 and L2 (the listed pass of the 256 x 256 x 81 job
+// 1.19 ms, angle first 1.28 ms).
+//
+// Measured on that job's subset 0 of 21 (6.78 M bins, 2.14e9 segments forward,
+// 0.94e9 back, B200), the padded pair's kernels -> these: projection 3.59 ->
+// 1.15 ms, backprojection 4.07 -> 1.86, full pass 2.68 -> 1.77, listed pass
+// 1.76 -> 1.22.  The gathers are bound by instruction issue (70 % of the
+// slots; 8 warp instructions a step without z crossings, 22 in a batch with
+// one), the scatters by the SM-to-L2 path: 5.1 sectors a reduction of 32 lanes
+// (the pair's rays along r: 10.3), 217 G sectors/s.
+#include <cuda_runtime.h>
+#include <cmath>
+#include <cstdint>
+#include "bins.cuh"
+#include "columns.cuh"
+#include "internal.h"
+
+namespace apirl {
+
+namespace {
+
+// Eight warps, so that a list serves many sinograms, at 5 blocks an SM (48
+// registers): the full pass of that job 1.71 ms, against 1.80 / 1.79 / 1.77 /
+// 2.03 ms with 128 / 192 / 320 / 512 threads and 1.82 ms at 4 blocks (64
+// registers).
+constexpr int kColBlock = 256;
+constexpr int kColBlocks = 5;
+constexpr int kColWarps = kColBlock / 32;
+// Blocks of the LORs with few counts.
+constexpr int kColFewBlock = 64;
+constexpr int kColFewBlocks = 20;
+
+struct ColLor {
+  int k, l, a;  // subset angle, r, full angle
+};
+
+// LOR `at` of the subset, r first.
+__device__ __forceinline__ ColLor col_lor(const LorTable& t, const SubsetSel& s, unsigned at) {
+  ColLor c;
+  c.k = (int)(at / (unsigned)t.n_r);
+  c.l = (int)(at - (unsigned)c.k * (unsigned)t.n_r);
+  c.a = s.subset < 0 ? c.k : s.subset + s.nsub * c.k;
+  return c;
+}
+
+__global__ void __launch_bounds__(kColBlock, kColBlocks) k_project_cols(ImgGeom g, ColDims d, LorTable t, SubsetSel s,
+                                                            const float* __restrict__ img, float* __restrict__ out) {
+  const ColLor lor = col_lor(t, s, blockIdx.x);
+  const float4 P = __ldg(t.lor + (int64_t)lor.a * t.n_r + lor.l);
+  col_list(P, g, d);
+  const ColWalk& w = col_head();
+  for (int g0 = threadIdx.x & ~31; g0 < t.n_sinos; g0 += blockDim.x) {
+    const int gl = g0 + (threadIdx.x & 31);
+    const bool in = gl < t.n_sinos;
+    const float2 e = in ? __ldg(t.z + t.g0 + gl) : make_float2(0.f, 0.f);
+    ColGather sum;
+    if (w.listed) col_walk(in ? col_setup_z(e, w, g, d) : col_no_ray(), d, img, sum);
+    else if (in) col_walk_checked(P, e, g, d, img, sum);
+    if (in) out[((int64_t)gl * s.nk + lor.k) * t.n_r + lor.l] = sum.acc;
+  }
+}
+
+// A ray's adds where v / e would leave the float range: (seg * v) / e.
+struct ColScatterDivide {
+  float v, e;
+  __device__ __forceinline__ void operator()(float* p, float seg) const {
+    red_add_global(p, A_DIV(A_MUL(seg, v), e));
+  }
+};
+
+// acc += A_s^T v in the column layout: Backproject's rule (SiddonProjector.cpp:496,
+// bins with v == 0 add nothing) and, with vest, DivideAndBackproject's
+// (:669-683: (seg * v) / e where e != 0, else seg * v).  The ratio v / e is
+// formed once per bin where v and the ratio are far from the ends of the
+// float range, and per segment elsewhere.
+__global__ void __launch_bounds__(kColBlock, kColBlocks) k_scatter_cols(ImgGeom g, ColDims d, LorTable t, SubsetSel s,
+                                                                        const float* __restrict__ vin,
+                                                                        const float* __restrict__ vest,
+                                                                        float* __restrict__ acc) {
+  const ColLor lor = col_lor(t, s, blockIdx.x);
+  const float4 P = __ldg(t.lor + (int64_t)lor.a * t.n_r + lor.l);
+  col_list(P, g, d);
+  const ColWalk& w = col_head();
+  acc += w.xmain ? d.floats() : 0;
+  for (int g0 = threadIdx.x & ~31; g0 < t.n_sinos; g0 += blockDim.x) {
+    const int gl = g0 + (threadIdx.x & 31);
+    bool in = gl < t.n_sinos;
+    const int64_t b = ((int64_t)gl * s.nk + lor.k) * t.n_r + lor.l;
+    float v = 0.f, ends = 0.f;
+    if (in) {
+      v = __ldg(vin + b);
+      in = v != 0.f;
+      const float est = vest ? __ldg(vest + b) : 0.f;
+      if (in && est != 0.f) {
+        const float q = A_DIV(v, est), av = fabsf(v), aq = fabsf(q);
+        if (av >= 1e-30f && av <= 1e30f && aq >= 1e-30f && aq <= 1e30f) v = q;
+        else ends = est;
+      }
+    }
+    const float2 e = in ? __ldg(t.z + t.g0 + gl) : make_float2(0.f, 0.f);
+    if (ends != 0.f) {
+      ColScatterDivide add{v, ends};
+      col_walk_checked(P, e, g, d, acc, add);
+      in = false;
+    }
+    if (!__any_sync(0xffffffffu, in)) continue;
+    ColScatter add{in ? v : 0.f};
+    if (w.listed) col_walk(in ? col_setup_z(e, w, g, d) : col_no_ray(), d, acc, add);
+    else if (in) col_walk_checked(P, e, g, d, acc, add);
+  }
+}
+
+// The fused pass (k_em_pass_persist's steps, kernels.cu) of the warp's 32
+// rays: forward walk, additive term, likelihood term, ratio, and the ratio
+// scattered along the walk.  Returns the lane's likelihood term.
+template <typename CT>
+__device__ __forceinline__ double em_rays(const ImgGeom& g, const ColDims& d, const LorTable& t, const SubsetSel& s,
+                                          const ColLor& lor, const float4 P, int gl, bool in,
+                                          const CT* __restrict__ counts, int counts_packed,
+                                          const float* __restrict__ add, const float* __restrict__ img,
+                                          float* __restrict__ acc, int back, int skip_zero) {
+  const ColWalk& w = col_head();
+  acc += w.xmain ? d.floats() : 0;
+  const int64_t row = counts_packed ? (int64_t)gl * s.nk + lor.k : (int64_t)(t.g0 + gl) * t.n_proj + lor.a;
+  const int64_t ci = row * t.n_r + lor.l;
+  const float m = in ? load_count<CT>(counts, ci) : 0.f;
+  const float2 ez = in ? __ldg(t.z + t.g0 + gl) : make_float2(0.f, 0.f);
+  ColGather sum;
+  WalkZ r = col_no_ray();
+  if (w.listed) {
+    if (in) r = col_setup_z(ez, w, g, d);
+    col_walk(r, d, img, sum);
+  } else if (in) {
+    col_walk_checked(P, ez, g, d, img, sum);
+  }
+  double term = 0.0;
+  float q = 0.f;
+  if (in) {
+    float e = sum.acc;
+    if (add) e = A_ADD(e, __ldg(add + ci));
+    if (e != 0.f) term = lik_term(m, e, skip_zero);
+    q = (m != 0.f && e != 0.f && back) ? A_DIV(m, e) : 0.f;
+  }
+  if (__any_sync(0xffffffffu, q != 0.f)) {
+    ColScatter out{q};
+    if (w.listed) col_walk(q != 0.f ? r : col_no_ray(), d, acc, out);
+    else if (q != 0.f) col_walk_checked(P, ez, g, d, acc, out);
+  }
+  return term;
+}
+
+// The LOR's likelihood partial: the sum of the block's terms, warps in order.
+__device__ __forceinline__ void em_partial(double term, unsigned lor, double* __restrict__ partials) {
+  __shared__ double part[kColWarps];
+  #pragma unroll
+  for (int o = 16; o > 0; o >>= 1) term += __shfl_down_sync(0xffffffffu, term, o);
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = term;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    term = 0.0;
+    for (int w = 0; w < (int)(blockDim.x >> 5); w++) term += part[w];
+    partials[lor] = term;
+  }
+}
+
+// The fused pass over every bin of the subset.
+template <typename CT>
+__global__ void __launch_bounds__(kColBlock, kColBlocks) k_em_cols(
+    ImgGeom g, ColDims d, LorTable t, SubsetSel s, const CT* __restrict__ counts, int counts_packed,
+    const float* __restrict__ add, const float* __restrict__ img, float* __restrict__ acc, int back,
+    double* __restrict__ partials) {
+  const ColLor lor = col_lor(t, s, blockIdx.x);
+  const float4 P = __ldg(t.lor + (int64_t)lor.a * t.n_r + lor.l);
+  col_list(P, g, d);
+  double term = 0.0;
+  for (int g0 = threadIdx.x & ~31; g0 < t.n_sinos; g0 += blockDim.x) {
+    const int gl = g0 + (threadIdx.x & 31);
+    term += em_rays<CT>(g, d, t, s, lor, P, gl, gl < t.n_sinos, counts, counts_packed, add, img, acc, back, 0);
+  }
+  em_partial(term, blockIdx.x, partials);
+}
+
+// The block's list of a LOR's sinograms with counts, among kColWindow from
+// g0: list[0 .. n) in order, n returned to every thread.
+constexpr int kColWindow = 2048;
+struct ColActive {
+  unsigned mask[kColWindow / 32];
+  int first[kColWindow / 32];
+  int n;
+  uint16_t list[kColWindow];
+};
+template <typename CT>
+__device__ __forceinline__ int col_active(const LorTable& t, const SubsetSel& s, const ColLor& lor, int g0,
+                                          const CT* __restrict__ counts, int counts_packed, ColActive& act) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int left = min(t.n_sinos - g0, kColWindow), groups = (left + 31) >> 5;
+  const int64_t step = (int64_t)(counts_packed ? s.nk : t.n_proj) * t.n_r;  // from a sinogram to the next
+  const CT* const first = counts + (counts_packed ? (int64_t)g0 * s.nk + lor.k : (int64_t)(t.g0 + g0) * t.n_proj + lor.a) * t.n_r +
+                          lor.l;
+  const int warps = blockDim.x >> 5;
+  for (int q = warp; q < groups; q += 4 * warps) {  // four groups' counts in flight
+    float m[4];
+    #pragma unroll
+    for (int u = 0; u < 4; u++) {
+      const int i = (q + u * warps) * 32 + lane;
+      m[u] = i < left ? load_count<CT>(first, i * step) : 0.f;
+    }
+    #pragma unroll
+    for (int u = 0; u < 4; u++) {
+      const unsigned mask = __ballot_sync(0xffffffffu, m[u] != 0.f);
+      if (lane == 0 && q + u * warps < groups) act.mask[q + u * warps] = mask;
+    }
+  }
+  __syncthreads();
+  if (warp == 0) {
+    static_assert(kColWindow / 32 == 64, "two groups a lane");
+    const int a = 2 * lane < groups ? __popc(act.mask[2 * lane]) : 0;
+    const int b = 2 * lane + 1 < groups ? __popc(act.mask[2 * lane + 1]) : 0;
+    int incl = a + b;
+    #pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += u;
+    }
+    act.first[2 * lane] = incl - a - b;
+    act.first[2 * lane + 1] = incl - b;
+    if (lane == 31) act.n = incl;
+  }
+  __syncthreads();
+  for (int q = warp; q < groups; q += warps) {
+    const unsigned m = act.mask[q];
+    if (m >> lane & 1u) act.list[act.first[q] + __popc(m & ((1u << lane) - 1u))] = (uint16_t)(q * 32 + lane);
+  }
+  __syncthreads();
+  return act.n;
+}
+
+// The fused pass over the bins with counts: a block lists its LOR's
+// sinograms with counts and its warps take 32 of them at a time.  skip_zero
+// as lik_term.  A LOR with at most `few` (<= kColFew) counts would leave most
+// of the block's warps idle: it goes to the queue with its list, for the small
+// blocks of k_em_cols_few.
+template <typename CT>
+__global__ void __launch_bounds__(kColBlock, kColBlocks) k_em_cols_listed(
+    ImgGeom g, ColDims d, LorTable t, SubsetSel s, const CT* __restrict__ counts, int counts_packed,
+    const float* __restrict__ add, const float* __restrict__ img, float* __restrict__ acc, int back,
+    double* __restrict__ partials, int skip_zero, int few, ColQueue queue) {
+  __shared__ ColActive act;
+  __shared__ unsigned slot;
+  const ColLor lor = col_lor(t, s, blockIdx.x);
+  const float4 P = __ldg(t.lor + (int64_t)lor.a * t.n_r + lor.l);
+  bool listed = false;
+  double term = 0.0;
+  for (int g0 = 0; g0 < t.n_sinos; g0 += kColWindow) {
+    const int n = col_active<CT>(t, s, lor, g0, counts, counts_packed, act);
+    if (n <= few && t.n_sinos <= kColWindow) {
+      if (n == 0) {
+        if (threadIdx.x == 0) partials[blockIdx.x] = 0.0;
+        return;
+      }
+      if (threadIdx.x == 0) {
+        slot = atomicAdd(queue.n, 1u);
+        queue.item[slot] = make_uint2(blockIdx.x, (unsigned)n);
+      }
+      __syncthreads();
+      for (int i = threadIdx.x; i < n; i += blockDim.x) queue.list[(int64_t)slot * kColFew + i] = act.list[i];
+      return;
+    }
+    if (n > 0 && !listed) {
+      col_list(P, g, d);
+      listed = true;
+    }
+    for (int i0 = threadIdx.x & ~31; i0 < n; i0 += blockDim.x) {
+      const int i = i0 + (threadIdx.x & 31);
+      const bool in = i < n;
+      term += em_rays<CT>(g, d, t, s, lor, P, in ? g0 + act.list[i] : 0, in, counts, counts_packed, add, img, acc,
+                          back, skip_zero);
+    }
+    __syncthreads();
+  }
+  em_partial(term, blockIdx.x, partials);
+}
+
+template <typename CT>
+__global__ void __launch_bounds__(kColFewBlock, kColFewBlocks) k_em_cols_few(
+    ImgGeom g, ColDims d, LorTable t, SubsetSel s, const CT* __restrict__ counts, int counts_packed,
+    const float* __restrict__ add, const float* __restrict__ img, float* __restrict__ acc, int back,
+    double* __restrict__ partials, int skip_zero, ColQueue queue) {
+  const unsigned items = *queue.n;
+  for (unsigned q = blockIdx.x; q < items; q += gridDim.x) {
+    const uint2 item = queue.item[q];
+    const int n = (int)item.y;
+    const ColLor lor = col_lor(t, s, item.x);
+    const float4 P = __ldg(t.lor + (int64_t)lor.a * t.n_r + lor.l);
+    col_list(P, g, d);
+    double term = 0.0;
+    for (int i0 = threadIdx.x & ~31; i0 < n; i0 += blockDim.x) {
+      const int i = i0 + (threadIdx.x & 31);
+      const bool in = i < n;
+      const int gl = in ? queue.list[(int64_t)q * kColFew + i] : 0;
+      term += em_rays<CT>(g, d, t, s, lor, P, gl, in, counts, counts_packed, add, img, acc, back, skip_zero);
+    }
+    em_partial(term, item.x, partials);
+    __syncthreads();
+  }
+}
+
+// ---- images to and from the column layout -----------------------------------
+// A block works 32 x of one row y and 32 slices z0 .. z0 + 31, 32 x 8 threads;
+// tile[par * 16 + z / 2][x]: the slices in the order the columns store them.
+
+// img's interior <- x ([z][y][x]).  With gimg: dots[block] = - (x . gimg) over
+// the block's voxels where gimg != 0 (k_neg_dot's rule, kernels.cu), FP64.
+// queue_n (may be null) is set to 0.
+__global__ void __launch_bounds__(256) k_col_copy(ColDims d, const float* __restrict__ x, float* __restrict__ img,
+                                                  const float* __restrict__ gimg, double* __restrict__ dots,
+                                                  unsigned* __restrict__ queue_n) {
+  __shared__ float tile[32][33];
+  __shared__ double part[8];
+  const int lx = threadIdx.x, ly = threadIdx.y, x0 = blockIdx.x * 32, y = blockIdx.y, z0 = blockIdx.z * 32;
+  if (queue_n && (blockIdx.x | blockIdx.y | blockIdx.z) == 0 && (lx | ly) == 0) *queue_n = 0;
+  float v[4], gv[4];
+  #pragma unroll
+  for (int q = 0; q < 4; q++) {
+    const int z = z0 + ly + 8 * q;
+    const bool in = x0 + lx < d.nx && z < d.nz;
+    const int64_t i = ((int64_t)z * d.ny + y) * d.nx + x0 + lx;
+    v[q] = in ? x[i] : 0.f;
+    gv[q] = gimg && in ? gimg[i] : 0.f;
+  }
+  #pragma unroll
+  for (int q = 0; q < 4; q++) {
+    const int z = ly + 8 * q;
+    tile[(z & 1) * 16 + (z >> 1)][lx] = v[q];
+  }
+  if (gimg) {
+    double s = 0.0;
+    #pragma unroll
+    for (int q = 0; q < 4; q++)
+      if (gv[q] != 0.f) s += (double)v[q] * (double)gv[q];
+    #pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+    if (lx == 0) part[ly] = s;
+  }
+  __syncthreads();
+  const int par = lx >> 4, z = z0 + 2 * (lx & 15) + par;
+  #pragma unroll
+  for (int q = 0; q < 4; q++) {
+    const int xx = ly + 8 * q;
+    if (x0 + xx < d.nx && z < d.nz)
+      img[((int64_t)(y + kPad) * d.px() + x0 + xx + kPad) * d.stride() + par * d.half + ((z + d.z0) >> 1)] =
+          tile[lx][xx];
+  }
+  if (gimg && lx == 0 && ly == 0) {
+    double s = 0.0;
+    for (int i = 0; i < 8; i++) s += part[i];
+    dots[((int64_t)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x] = -s;
+  }
+}
+
+// mode 0: EM update of x from the column sums acc (rule ge / gt, as k_update);
+// mode 1: bp += acc.  acc's interior cleared, after the block's loads.  With
+// lik: one more layer of blocks (z = 0), whose first sums the n likelihood
+// partials in a fixed order, less *less (may be null), beside the others' work.
+__global__ void __launch_bounds__(256) k_col_reduce(ColDims d, float* __restrict__ acc, int mode,
+                                                    float* __restrict__ x, float* __restrict__ bp,
+                                                    const float* __restrict__ sens,
+                                                    const float* __restrict__ thr_ptr, float thr_value, int ge,
+                                                    const double* __restrict__ partials, int64_t n,
+                                                    const double* __restrict__ less, double* __restrict__ lik) {
+  __shared__ float tile[32][33];
+  if (lik && blockIdx.z == 0) {
+    if (blockIdx.x | blockIdx.y) return;
+    double* const part = reinterpret_cast<double*>(tile);
+    const int tid = threadIdx.y * 32 + threadIdx.x;
+    double v[8] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+    int64_t i = tid;
+    for (; i + 7 * 256 < n; i += 8 * 256) {
+      #pragma unroll
+      for (int u = 0; u < 8; u++) v[u] += partials[i + u * 256];
+    }
+    for (; i < n; i += 256) v[0] += partials[i];
+    double s = ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
+    #pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+    if (threadIdx.x == 0) part[threadIdx.y] = s;
+    __syncthreads();
+    if (tid == 0) {
+      s = 0.0;
+      for (int w = 0; w < 8; w++) s += part[w];
+      *lik = s - (less ? *less : 0.0);
+    }
+    return;
+  }
+  const float thr = (mode == 0 && thr_ptr) ? *thr_ptr : thr_value;
+  const int lx = threadIdx.x, ly = threadIdx.y, x0 = blockIdx.x * 32, y = blockIdx.y,
+            z0 = (lik ? blockIdx.z - 1 : blockIdx.z) * 32;
+  const int par = lx >> 4, zc = z0 + 2 * (lx & 15) + par;
+  float* out = mode == 0 ? x : bp;
+  float xv[4], sv[4];
+  #pragma unroll
+  for (int q = 0; q < 4; q++) {
+    const int xx = ly + 8 * q;
+    if (x0 + xx < d.nx && zc < d.nz) {
+      const float* a = acc + ((int64_t)(y + kPad) * d.px() + x0 + xx + kPad) * d.stride() + par * d.half +
+                       ((zc + d.z0) >> 1);
+      tile[lx][xx] = A_ADD(a[0], a[d.floats()]);
+    }
+  }
+  #pragma unroll
+  for (int q = 0; q < 4; q++) {
+    const int z = z0 + ly + 8 * q;
+    xv[q] = sv[q] = 0.f;
+    if (x0 + lx < d.nx && z < d.nz) {
+      const int64_t i = ((int64_t)z * d.ny + y) * d.nx + x0 + lx;
+      xv[q] = out[i];
+      if (mode == 0) sv[q] = sens[i];
+    }
+  }
+  __syncthreads();
+  #pragma unroll
+  for (int q = 0; q < 4; q++) {
+    const int xx = ly + 8 * q;
+    if (x0 + xx < d.nx && zc < d.nz) {
+      float* a = acc + ((int64_t)(y + kPad) * d.px() + x0 + xx + kPad) * d.stride() + par * d.half + ((zc + d.z0) >> 1);
+      a[0] = a[d.floats()] = 0.f;
+    }
+  }
+  #pragma unroll
+  for (int q = 0; q < 4; q++) {
+    const int zl = ly + 8 * q, z = z0 + zl;
+    if (x0 + lx >= d.nx || z >= d.nz) continue;
+    const int64_t i = ((int64_t)z * d.ny + y) * d.nx + x0 + lx;
+    const float b = tile[(zl & 1) * 16 + (zl >> 1)][lx];
+    if (mode == 0) {
+      const bool okv = ge ? (sv[q] >= thr) : (sv[q] > thr);
+      out[i] = okv ? A_DIV(A_MUL(xv[q], b), sv[q]) : 0.f;
+    } else {
+      out[i] = A_ADD(xv[q], b);
+    }
+  }
+}
+
+// Shared memory that a block may take without asking for more.
+constexpr size_t kColMaxSmem = 48 * 1024;
+
+ColDims dims_of(const ImgGeom& g, const ColBuffers& c) { return ColDims{g.nx, g.ny, g.nz, c.z0, c.half}; }
+
+dim3 voxel_grid(const ImgGeom& g) { return dim3((g.nx + 31) / 32, g.ny, (g.nz + 31) / 32); }
+
+// Warps of a block: up to 8, as few as give the same number of rounds over
+// the sinograms.
+int block_of(const LorTable& t) {
+  const int groups = (t.n_sinos + 31) / 32, rounds = (groups + kColBlock / 32 - 1) / (kColBlock / 32);
+  return (groups + rounds - 1) / rounds * 32;
+}
+
+int64_t lors_of(const LorTable& t, const SubsetSel& s) { return (int64_t)s.nk * t.n_r; }
+
+}  // namespace
+
+ColBuffers col_layout(const ImgGeom& g, const float* z_ends, int n_ends) {
+  // Slices that a ray between these end points can enter, and the spare ones.
+  float lo = z_ends[0], hi = z_ends[0];
+  for (int i = 1; i < n_ends; i++) {
+    lo = fminf(lo, z_ends[i]);
+    hi = fmaxf(hi, z_ends[i]);
+  }
+  ColBuffers c;
+  const double first = floor(((double)lo - g.offz) / g.dz) - 1 - kColSpare, end = floor(((double)hi - g.offz) / g.dz) + 2 + kColSpare;
+  const double z0 = ceil(fmax((double)kColSpare, -first) / 2) * 2, slices = fmax((double)g.nz + kColSpare, end) + z0;
+  const double floats = (double)(g.nx + 2 * kPad) * (g.ny + 2 * kPad) * (slices + 16);
+  // Bounded in bytes and against the image (a long scanner around a short
+  // image), in grid sizes and in the list's shared memory.
+  if (!(floats < (double)(1 << 30)) || floats > 4.0 * g.nx * g.ny * g.nz + (1 << 22) || g.ny > 65535 ||
+      g.nz > 65535 * 32 || col_smem(g.nx, g.ny) > kColMaxSmem)
+    return c;
+  c.z0 = (int)z0;
+  c.half = (((int)slices + 1) / 2 + 7) / 8 * 8;
+  c.floats = ColDims{g.nx, g.ny, g.nz, c.z0, c.half}.floats();
+  return c;
+}
+
+int64_t col_partials(const LorTable& t, SubsetSel s) { return lors_of(t, s); }
+
+int64_t col_dots(const ImgGeom& g) {
+  const dim3 v = voxel_grid(g);
+  return (int64_t)v.x * v.y * v.z;
+}
+
+cudaError_t launch_col_copy(const ImgGeom& g, const ColBuffers& c, const float* x, float* img, cudaStream_t st,
+                            const float* gimg, double* dots, unsigned* queue_n) {
+  k_col_copy<<<voxel_grid(g), dim3(32, 8), 0, st>>>(dims_of(g, c), x, img, gimg, dots, queue_n);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_col_reduce(const ImgGeom& g, const ColBuffers& c, float* acc, int mode, float* x, float* bp,
+                              const float* sens, const float* thr_ptr, float thr_value, int ge, cudaStream_t st,
+                              const double* partials, int64_t n, const double* less, double* lik) {
+  dim3 grid = voxel_grid(g);
+  if (lik) grid.z++;
+  k_col_reduce<<<grid, dim3(32, 8), 0, st>>>(dims_of(g, c), acc, mode, x, bp, sens, thr_ptr, thr_value, ge, partials, n,
+                                             less, lik);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_project_cols(const ImgGeom& g, const ColBuffers& c, const LorTable& t, SubsetSel s,
+                                const float* img, float* out, cudaStream_t st) {
+  if (lors_of(t, s) == 0) return cudaSuccess;
+  k_project_cols<<<(unsigned)lors_of(t, s), block_of(t), col_smem(g.nx, g.ny), st>>>(g, dims_of(g, c), t, s, img, out);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_scatter_cols(const ImgGeom& g, const ColBuffers& c, const LorTable& t, SubsetSel s,
+                                const float* vin, const float* vest, float* acc, cudaStream_t st) {
+  if (lors_of(t, s) == 0) return cudaSuccess;
+  k_scatter_cols<<<(unsigned)lors_of(t, s), block_of(t), col_smem(g.nx, g.ny), st>>>(g, dims_of(g, c), t, s, vin, vest,
+                                                                                    acc);
+  return cudaGetLastError();
+}
+
+template <typename CT>
+static cudaError_t em_cols(const ImgGeom& g, const ColBuffers& c, const LorTable& t, SubsetSel s, const CT* counts,
+                           int counts_packed, const float* add, int back, double* partials, int skip_zero,
+                           const ColQueue& queue, cudaStream_t st) {
+  const ColDims d = dims_of(g, c);
+  const unsigned grid = (unsigned)lors_of(t, s);
+  const size_t smem = col_smem(g.nx, g.ny);
+  if (!skip_zero) {
+    k_em_cols<CT><<<grid, block_of(t), smem, st>>>(g, d, t, s, counts, counts_packed, add, c.img, c.acc, back,
+                                                   partials);
+    return cudaGetLastError();
+  }
+  int dev = 0, sms = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
+  // Up to two waves of blocks the idle warps cost nothing, and a second
+  // kernel's latency would follow the first's (747 LORs of a 64 x 64 x 41 job,
+  // most with few counts: 29 + 31 us, in one kernel 40 us).  Above, the small
+  // blocks walk the few counts faster (5376 LORs of the 256 x 256 x 81 job at
+  // 1 % bins with counts: the pass 500 -> 444 us; 3984 LORs of a 128 x 128 x
+  // 41 job: 141 -> 128 us).
+  // With so few sinograms that a block has few warps anyway (37 and 19 of a
+  // 128 x 128 image: 388 and 358 us with the queue, 304 and 181 without) there
+  // is nothing to defer either.
+  const int few = lors_of(t, s) > 2 * sms * kColBlocks && t.n_sinos > 4 * kColFew && t.n_sinos <= kColWindow ? kColFew
+                                                                                                            : 0;
+  k_em_cols_listed<CT><<<grid, block_of(t), smem, st>>>(g, d, t, s, counts, counts_packed, add, c.img, c.acc, back,
+                                                       partials, skip_zero, few, queue);
+  if ((e = cudaGetLastError()) != cudaSuccess || !few) return e;
+  const unsigned resident = (unsigned)(sms * kColFewBlocks);
+  k_em_cols_few<CT><<<grid < resident ? grid : resident, kColFewBlock, smem, st>>>(g, d, t, s, counts, counts_packed, add, c.img,
+                                                                        c.acc, back, partials, skip_zero, queue);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_em_cols(const ImgGeom& g, const ColBuffers& c, const LorTable& t, SubsetSel s, const void* counts,
+                           int counts_dtype, int counts_packed, const float* add, int back, double* partials,
+                           int skip_zero, const ColQueue& queue, cudaStream_t st) {
+  if (lors_of(t, s) == 0) return cudaSuccess;
+  switch (counts_dtype) {
+    case APIRL_F32:
+      return em_cols(g, c, t, s, (const float*)counts, counts_packed, add, back, partials, skip_zero, queue, st);
+    case APIRL_U32:
+      return em_cols(g, c, t, s, (const uint32_t*)counts, counts_packed, add, back, partials, skip_zero, queue, st);
+    case APIRL_U16:
+      return em_cols(g, c, t, s, (const uint16_t*)counts, counts_packed, add, back, partials, skip_zero, queue, st);
+    default: return cudaErrorInvalidValue;
+  }
+}
+
+}  // namespace apirl

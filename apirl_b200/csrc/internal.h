@@ -3,6 +3,7 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <cstdint>
+#include <mutex>
 #include <vector>
 #include "geom_types.h"
 
@@ -114,6 +115,56 @@ struct PadBuffers {
   // 6 or 8; 0 = the pass kind's default).
   int unroll = 0;
 };
+// The column layout of the 3D passes (columns.cuh): an image copy and two
+// backprojection sums one behind the other, whose interiors are zero between
+// passes: the rays that run mostly along x add into the second, the others
+// into the first, as into the padded pair (the rounding error of a voxel's
+// float sum grows with the sum: with one sum it measured twice the pair's).
+// half = 0: the volume has none (col_layout's bounds).
+struct ColBuffers {
+  float* img = nullptr;
+  float* acc = nullptr;
+  int z0 = 0, half = 0;
+  int64_t floats = 0;
+};
+// Sinograms (of the shard) from which the column walk serves the 3D passes: a
+// warp holds 32.  Measured on a 128 x 128 image, 166 x 166 bins, us for
+// project / backproject / full pass, padded pair -> column walk: 10 sinograms
+// 98 / 128 / 150 -> 120 / 97 / 176, 19: 155 / 186 / 219 -> 123 / 112 / 187,
+// 44: 315 / 398 / 405 -> 179 / 237 / 311, 91: 616 / 787 / 764 -> 247 / 374 / 474.
+constexpr int kColMinSinos = 16;
+// Sizes only; z_ends: the axial end points of the scanner's LORs.
+ColBuffers col_layout(const ImgGeom& g, const float* z_ends, int n_ends);
+// Likelihood partials of a column pass.
+int64_t col_partials(const LorTable& t, SubsetSel s);
+// A listed column pass's LORs with few counts: item (LOR of the subset, count)
+// and list (kColFew sinograms of each); room for every LOR.
+constexpr int kColFew = 64;
+struct ColQueue {
+  unsigned* n = nullptr;
+  uint2* item = nullptr;
+  uint16_t* list = nullptr;
+};
+// Partials of -x . gimg (launch_col_copy).
+int64_t col_dots(const ImgGeom& g);
+cudaError_t launch_col_copy(const ImgGeom& g, const ColBuffers& c, const float* x, float* img, cudaStream_t st,
+                            const float* gimg = nullptr, double* dots = nullptr, unsigned* queue_n = nullptr);
+// mode 0: EM update of x from acc (threshold rule); mode 1: bp += acc.  Clears
+// acc.  lik set: *lik = the sum of the n partials, less *less.
+cudaError_t launch_col_reduce(const ImgGeom& g, const ColBuffers& c, float* acc, int mode, float* x, float* bp,
+                              const float* sens, const float* thr_ptr, float thr_value, int ge, cudaStream_t st,
+                              const double* partials = nullptr, int64_t n = 0, const double* less = nullptr,
+                              double* lik = nullptr);
+cudaError_t launch_project_cols(const ImgGeom& g, const ColBuffers& c, const LorTable& t, SubsetSel s,
+                                const float* img, float* out, cudaStream_t st);
+// acc += A_s^T v (a subset sinogram); vest: DivideAndBackproject's rule.
+cudaError_t launch_scatter_cols(const ImgGeom& g, const ColBuffers& c, const LorTable& t, SubsetSel s,
+                                const float* vin, const float* vest, float* acc, cudaStream_t st);
+// The fused kernels, one partial per col_partials.  skip_zero as the kernels'
+// (0: every bin is walked); else queue.n is 0 before (launch_col_copy).
+cudaError_t launch_em_cols(const ImgGeom& g, const ColBuffers& c, const LorTable& t, SubsetSel s, const void* counts,
+                           int counts_dtype, int counts_packed, const float* add, int back, double* partials,
+                           int skip_zero, const ColQueue& queue, cudaStream_t st);
 // Bins per tile of the list building (one block each).
 constexpr int kNzTile = 2048;
 // Room for the list of a subset's bins with counts (sparse passes of the
@@ -126,6 +177,10 @@ struct NzList {
   int64_t cap = 0;
   int order = 0;  // APIRL_OPT_LIST_ORDER: 0 = bin order, else groups of this size by walk length
 };
+// *lik = the fixed-order sum of the n partials (room for 2 kSumLevel2 more
+// behind them), less x . zimg + *zero_add when zimg is given.
+cudaError_t launch_lik_sum(const ImgGeom& g, double* partials, int64_t n, const float* x, const float* zimg,
+                           const double* zero_add, double* lik, cudaStream_t st);
 // lik_mode: 0 = over e != 0, 1 = over e > 0, 2 = over ratio > 0.  back = 0: no backprojection.
 cudaError_t launch_em_pass(const ImgGeom& g, const LorTable& t, SubsetSel s, const void* counts, int counts_dtype,
                            int counts_packed, const float* add, const float* x, float* bp, int back, int lik_mode,
@@ -291,6 +346,21 @@ struct apirl_projector {
   unsigned long long* d_chunk = nullptr;  // chunk counter of the persistent pass
   int sparse_image = 0;          // APIRL_OPT_SPARSE_IMAGE: 0 = zero-count image Z_s, 1 = geometry image G_s
   apirl::NzList nz;              // list of a subset's bins with counts (sparse passes), grown on demand
+  // The column layout (half = 0: none): the fused pass's and the
+  // backprojections' image copy and sums, used by one stream at a time.
+  apirl::ColBuffers cols;
+  apirl::ColQueue queue;         // LORs with few counts of a listed pass
+  // Column images and sums of the calls that keep no other state in the
+  // projector (apirl_project, apirl_divide_and_backproject) and may run on
+  // several streams and threads at once: a call takes one under the lock and
+  // its stream waits for the work that last used it.
+  struct ColSlot {
+    float* buf = nullptr;
+    cudaEvent_t done = nullptr;
+    cudaStream_t last = nullptr;
+    unsigned long long use = 0;
+  } col_img[2], col_sum[1];
+  std::mutex col_mu;
   apirl::PadBuffers pad2;        // second padded backprojection pair (bA, bT only), on first use
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   // Counts staged ahead of apirl_em_pass_host (apirl_stage_counts): copied on

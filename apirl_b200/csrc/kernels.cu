@@ -18,6 +18,7 @@
 #include <mutex>
 #include <utility>
 #include <vector>
+#include "bins.cuh"
 #include "internal.h"
 #include "siddon.cuh"
 #include "../../include/apirl_b200.h"
@@ -64,31 +65,6 @@ constexpr int kEmMinBlocks = APIRL_EM_MIN_BLOCKS;
 #ifndef APIRL_EM_RESETUP
 #define APIRL_EM_RESETUP 1
 #endif
-
-struct BinPos {
-  int g, k, l, a;  // sinogram, subset angle, r, full angle
-};
-
-__device__ __forceinline__ BinPos decode(int64_t b, const LorTable& t, const SubsetSel& s) {
-  BinPos p;
-  const int64_t per = (int64_t)s.nk * t.n_r;
-  const int gl = (int)(b / per);  // sinogram within the shard
-  const int rem = (int)(b - (int64_t)gl * per);
-  p.g = t.g0 + gl;
-  p.k = rem / t.n_r;
-  p.l = rem - p.k * t.n_r;
-  p.a = s.subset < 0 ? p.k : s.subset + s.nsub * p.k;
-  return p;
-}
-
-template <typename CT> __device__ __forceinline__ float load_count(const CT* p, int64_t i);
-template <> __device__ __forceinline__ float load_count<float>(const float* p, int64_t i) { return __ldg(p + i); }
-template <> __device__ __forceinline__ float load_count<uint32_t>(const uint32_t* p, int64_t i) {
-  return (float)__ldg(p + i);
-}
-template <> __device__ __forceinline__ float load_count<uint16_t>(const uint16_t* p, int64_t i) {
-  return (float)__ldg(p + i);
-}
 
 // Forward projection of one bin (3D), masked gather of the image.
 __device__ __forceinline__ float ray_sum3(const ImgGeom& g, const float4 L, const float2 z, const float* __restrict__ img,
@@ -317,16 +293,6 @@ __global__ void __launch_bounds__(kBlock) k_count_steps(ImgGeom g, LorTable t, S
     if (t.ok[p.l]) siddon2_setup(L.x, L.y, A_SUB(L.z, L.x), A_SUB(L.w, L.y), g, w);
     steps[b] = w.n;
   }
-}
-
-// A walked bin's likelihood term (Sinogram3D::getLikelihoodValue,
-// data/src/Sinogram3D.cpp:584-606: m log e - e over e != 0).  skip_zero:
-// 0 = every bin walked; 1 = zero-count bins not walked, their -e supplied by
-// -x . Z_s (Z_s = A_s^T 1[m == 0]); 2 = zero-count bins not walked and the
-// -e of every bin supplied by -x . G_s - sum(add) (G_s = A_s^T 1, a
-// geometry image), so a walked bin adds m log e alone.
-__device__ __forceinline__ double lik_term(float m, float e, int skip_zero) {
-  return skip_zero == 2 ? (double)m * log((double)e) : (double)m * log((double)e) - (double)e;
 }
 
 // ---------------------------------------------------------------------------
@@ -1582,6 +1548,17 @@ cudaError_t prepare_em_kernels(int block) {
 }
 
 
+cudaError_t launch_lik_sum(const ImgGeom& g, double* partials, int64_t n, const float* x, const float* zimg,
+                           const double* zero_add, double* lik, cudaStream_t st) {
+  if (zimg) {
+    // - sum of the bins' estimates that were not walked: - x . zimg - their additive terms.
+    const int64_t nv = (int64_t)g.nx * g.ny * g.nz;
+    k_neg_dot<<<kSumLevel2, kBlock, 0, st>>>(x, zimg, nv, zero_add, partials + n);
+    n += kSumLevel2;
+  }
+  return launch_sum(partials, n, lik, st);
+}
+
 int64_t em_pass_blocks(const LorTable& t, SubsetSel s) {
   // One likelihood partial per warp for any block size of 32..256 threads
   // (ceil(total / b) * b / 32 <= total / 32 + 8), the zero-count image's
@@ -1795,13 +1772,7 @@ cudaError_t launch_em_pass(const ImgGeom& g, const LorTable& t, SubsetSel s, con
     if (le != cudaSuccess) return le;
     cudaError_t pe = cudaGetLastError();
     if (pe != cudaSuccess || !lik) return pe;
-    int64_t np = chunks;
-    if (zimg) {
-      const int64_t nv = (int64_t)g.nx * g.ny * g.nz;
-      k_neg_dot<<<kSumLevel2, kBlock, 0, st>>>(x, zimg, nv, zero_add, partials + np);
-      np += kSumLevel2;
-    }
-    return launch_sum(partials, np, lik, st);
+    return launch_lik_sum(g, partials, chunks, x, zimg, zero_add, lik, st);
   }
   if (cudaError_t le = prefer_l1()) return le;
   switch (counts_dtype) {
@@ -1815,14 +1786,7 @@ cudaError_t launch_em_pass(const ImgGeom& g, const LorTable& t, SubsetSel s, con
   if (e != cudaSuccess || !lik) return e;
   // One partial per 32 bins, whatever the block size (warps past the last
   // bin wrote zeros behind them): the same sum for every block size.
-  int64_t np = (total + 31) / 32;
-  if (zimg) {
-    // - sum of the zero-count bins' estimates: - x . zimg - sum of their additive terms.
-    const int64_t nv = (int64_t)g.nx * g.ny * g.nz;
-    k_neg_dot<<<kSumLevel2, kBlock, 0, st>>>(x, zimg, nv, zero_add, partials + np);
-    np += kSumLevel2;
-  }
-  return launch_sum(partials, np, lik, st);
+  return launch_lik_sum(g, partials, (total + 31) / 32, x, zimg, zero_add, lik, st);
 }
 
 cudaError_t launch_zero_bins(const ImgGeom& g, const LorTable& t, SubsetSel s, const void* counts, int counts_dtype,

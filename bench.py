@@ -275,11 +275,11 @@ def run_sharded(args):
                        "pass": ("nonzero: each shard walks its bins with counts, its likelihood part from its "
                                 "geometry images A_s^T 1 (set-up)") if nonzero else "full: every bin walked",
                        "update": "x*bp/sens where sens > 0"},
-            "roofline": {"bound": "hbm", "kernel": "k_em_pass on rank 0's shard",
+            "roofline": {"bound": "hbm", "kernel": "k_em_cols on rank 0's shard",
                          "kernel_ms": statistics.mean(kern), "peak": peak, "unit": "GB/s",
                          "peak_source": f"{peak_kind} hbm_gbs",
                          "achieved": achieved, "frac": achieved / peak, "traffic": None},
-            "e2e": None, "cpu_baseline": None, "gpu_launches": (9 if nonzero else 5) * args.steps, "clocks": clock,
+            "e2e": None, "cpu_baseline": None, "gpu_launches": (4 if nonzero else 3) * args.steps, "clocks": clock,
         }
         print(json.dumps(line), flush=True)
     if world > 1:
@@ -441,6 +441,11 @@ def run_gpu(args):
     value, total_ms = whole_job_value(args.steps, sum(step_ms) + pre_ms, world, dist if world > 1 else None, dev)
 
     kb = [step_bytes(w, s, skipz) for s in subs]
+    # The kernel that walks: the column walk, or the padded pair's where an
+    # option keeps to it (csrc/capi.cu, pass_cols).
+    pair = args.l2_persist or args.list_order or args.accumulate != "atomic"
+    kernel = ("k_em_pass" if args.alpha != "f32" else "k_em_pass_persist" if pair else
+              "k_em_cols" if args.pass_form == "full" else "k_em_cols_listed")
     kern_bytes = statistics.mean(k for k, _ in kb)
     kern_s = statistics.mean(kern_ms) / 1e3
     peak, peak_kind = peaks()
@@ -571,19 +576,17 @@ def run_gpu(args):
                          "traffic": args.traffic_bytes if args.traffic_bytes is not None else
                          ({"full": FULL_TRAFFIC_BYTES, "nonzero": NONZERO_TRAFFIC_BYTES}.get(args.pass_form)
                           if args.max_ring_diff is None else None),
-                         "kernel": ("k_em_pass_persist" if args.persistent and args.alpha == "f32" else "k_em_pass")
-                                   + " (fused projection / ratio / backprojection)",
+                         "kernel": kernel + " (fused projection / ratio / backprojection)",
                          "timing": "CUDA events recorded by the library on the launching stream around the fused "
-                                   "kernel and its two small likelihood-sum kernels",
+                                   "kernels",
                          "algorithmic_bytes_per_launch": kern_bytes, "kernel_ms": kern_s * 1e3,
                          "peak_source": f"{peak_kind} hbm_gbs"},
             "e2e": e2e,
             "cpu_baseline": cpu,
-            # per step: layout copy, fused kernel, (zero-count dot,) two-level
-            # likelihood sum, reduce/update; plus one zero-count kernel per subset
-            # per pass: layout copy, [list: tiles, scan, write], fused kernel,
-            # [dot product], two-level sum, update
-            "gpu_launches": (9 * args.steps + NSUB) if sparse else (9 * args.steps if nonzero else 5 * args.steps),
+            # per pass on the column layout: copy, fused kernel (listed: and
+            # the one of the LORs with few counts), update; else at least copy,
+            # fused kernel, two-level sum, update; zero-count images once
+            "gpu_launches": (4 if sparse or nonzero else 3) * args.steps + (NSUB if sparse else 0),
             "clocks": clock,
         }
         if mixed:

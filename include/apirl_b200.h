@@ -178,7 +178,15 @@ apirl_status apirl_projector_set_shard(apirl_projector* p, int first_sinogram, i
  *   running mostly along x in the [z][x][y] one, so that a warp's 32
  *   neighbouring rays touch contiguous memory; rays that stay within the
  *   border skip the per-step bounds tests.  Results equal the 0 setting up to
- *   the order of fp32 additions in the backprojection.
+ *   the order of fp32 additions in the backprojection.  Projectors of 16 or
+ *   more sinograms (the shard's) run their passes, projections and
+ *   backprojections on a third, column layout instead, [y][x][z], in which a
+ *   block walks one (angle, r) for all sinograms (7 more images); sensitivities
+ *   and geometry images, and passes with an option that speaks of the padded
+ *   layouts (L2 window, list order, another accumulation form than plain
+ *   atomics), keep to the two.  The launch options below (block size,
+ *   persistent, gather segments) shape the two layouts' kernel; the column
+ *   layout's has one shape and takes any setting.
  * APIRL_OPT_KERNEL_TIMING (default 0): record CUDA events around the fused
  *   kernel of every pass; apirl_projector_kernel_ms returns the last one.
  * APIRL_OPT_EM_BLOCK (default 128): threads per block of the fused kernel
