@@ -299,6 +299,17 @@ apirl_status finish_create(apirl_projector* p, apirl_projector** out) {
     if (!st) st = alloc_cols(p);
     if (st) return st;
   }
+  if (!p->is3d && apirl::planar_lim(p->g) && (int64_t)p->t.n_proj * p->t.n_r < INT_MAX) {
+    apirl::PlanarBuffers& pl = p->planar;
+    const size_t lim = apirl::planar_lim(p->g);
+    constexpr int copies = apirl::kPlanarCopies;
+    CK(cudaMalloc(&pl.img, 2 * (1 + copies) * lim * sizeof(float)));
+    CK(cudaMemset(pl.img, 0, 2 * (1 + copies) * lim * sizeof(float)));
+    pl.imgT = pl.img + lim;
+    pl.sum = pl.imgT + lim;
+    pl.sumT = pl.sum + copies * lim;
+    pl.lim = (unsigned)lim;
+  }
   *out = p;
   return APIRL_OK;
 }
@@ -475,6 +486,7 @@ void apirl_projector_destroy(apirl_projector* p) {
   }
   cudaFree(p->cols.img);  // the block of all column buffers
   cudaFree(p->queue.n);
+  cudaFree(p->planar.img);
   for (auto& c : p->col_img)
     if (c.done) cudaEventDestroy(c.done);
   for (auto& c : p->col_sum)
@@ -797,6 +809,8 @@ apirl_status fused(apirl_projector* p, SubsetSel ss, const void* d_counts, int d
   if (dual && pass_cols(p)) {
     CK(apirl::launch_em_cols(p->g, p->cols, p->t, ss, d_counts, dtype, packed, d_add, 1, p->d_partials,
                              d_zimg ? (p->sparse_image ? 2 : 1) : 0, p->queue, s));
+  } else if (p->planar.lim) {
+    CK(apirl::launch_planar_pass(p->g, p->t, ss, d_counts, dtype, packed, d_add, d_x, p->planar, 1, 1, p->d_partials, s));
   } else {
     CK(apirl::launch_em_pass(p->g, p->t, ss, d_counts, dtype, packed, d_add, d_x, d_bp, 1, p->is3d ? 0 : 1,
                              p->d_partials, d_lik, s, p->pg, dual ? p->pad : apirl::PadBuffers(), p->em_block,
@@ -839,7 +853,11 @@ apirl_status apirl_em_pass(apirl_projector* p, const void* d_counts, int counts_
   }
   st = fused(p, ss, d_counts, counts_dtype, counts_packed, d_add, d_x, d_bp, false, d_lik, s);
   if (st) return st;
-  CK(apirl::launch_update(nv, d_x, d_bp, d_sens, d_thr, thr_value, ge, 1, s));
+  if (p->planar.lim)
+    CK(apirl::launch_planar_update(p->g, p->planar, 0, d_x, nullptr, d_sens, d_thr, thr_value, ge, p->d_partials,
+                                   ((int64_t)ss.nk * p->t.n_r + 31) / 32, d_lik, s));
+  else
+    CK(apirl::launch_update(nv, d_x, d_bp, d_sens, d_thr, thr_value, ge, 1, s));
   return APIRL_OK;
 }
 
@@ -932,7 +950,12 @@ apirl_status apirl_em_project_backproject(apirl_projector* p, const void* d_coun
     if (st) return st;
     return pass_end(p, ss, 1, nullptr, d_bp, nullptr, nullptr, 0.f, 0, nullptr, nullptr, d_lik, s);
   }
-  return fused(p, ss, d_counts, counts_dtype, counts_packed, d_add, d_x, d_bp, false, d_lik, s);
+  st = fused(p, ss, d_counts, counts_dtype, counts_packed, d_add, d_x, d_bp, false, d_lik, s);
+  if (st) return st;
+  if (p->planar.lim)
+    CK(apirl::launch_planar_update(p->g, p->planar, 1, nullptr, d_bp, nullptr, nullptr, 0.f, 0, p->d_partials,
+                                   ((int64_t)ss.nk * p->t.n_r + 31) / 32, d_lik, s));
+  return APIRL_OK;
 }
 
 apirl_status apirl_projector_set_option(apirl_projector* p, int option, int value) {

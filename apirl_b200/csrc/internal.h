@@ -127,6 +127,24 @@ struct ColBuffers {
   int z0 = 0, half = 0;
   int64_t floats = 0;
 };
+// The 2D pass's padded layouts (planar.cu): the slice as [y][x] and [x][y],
+// and kPlanarCopies sums of each, one behind the other, interiors zero between
+// passes; lim = floats of one, 0: none.
+constexpr int kPlanarCopies = 2;
+struct PlanarBuffers {
+  float *img = nullptr, *imgT = nullptr, *sum = nullptr, *sumT = nullptr;
+  unsigned lim = 0;
+};
+// Floats of one padded slice; 0: too large, the slice keeps to the unpadded pass.
+unsigned planar_lim(const ImgGeom& g);
+// Copies x and runs the fused 2D pass; one partial per 32 bins.
+cudaError_t launch_planar_pass(const ImgGeom& g, const LorTable& t, SubsetSel s, const void* counts, int counts_dtype,
+                               int counts_packed, const float* add, const float* x, const PlanarBuffers& pl, int back,
+                               int lik_mode, double* partials, cudaStream_t st);
+// mode 0: EM update of x, mode 1: bp += the sums; clears them.  lik: the sum of the n partials.
+cudaError_t launch_planar_update(const ImgGeom& g, const PlanarBuffers& pl, int mode, float* x, float* bp,
+                                 const float* sens, const float* thr_ptr, float thr_value, int ge,
+                                 const double* partials, int64_t n, double* lik, cudaStream_t st);
 // Sinograms (of the shard) from which the column walk serves the 3D passes: a
 // warp holds 32.  Measured on a 128 x 128 image, 166 x 166 bins, us for
 // project / backproject / full pass, padded pair -> column walk: 10 sinograms
@@ -349,6 +367,7 @@ struct apirl_projector {
   // The column layout (half = 0: none): the fused pass's and the
   // backprojections' image copy and sums, used by one stream at a time.
   apirl::ColBuffers cols;
+  apirl::PlanarBuffers planar;   // 2D
   apirl::ColQueue queue;         // LORs with few counts of a listed pass
   // Column images and sums of the calls that keep no other state in the
   // projector (apirl_project, apirl_divide_and_backproject) and may run on

@@ -394,6 +394,7 @@ __device__ __forceinline__ void siddon3_walk(Walk3 w, const ImgGeom& g, V&& visi
 struct Walk2 {
   float ax, ay, axu, ayu, ac, L;
   int i, j, iinc, jinc, n;
+  int guarded;  // entry and exit voxels within one of the image
 };
 
 __device__ __forceinline__ void siddon2_setup(float p0x, float p0y, float vx, float vy, const ImgGeom& g, Walk2& w) {
@@ -423,6 +424,7 @@ __device__ __forceinline__ void siddon2_setup(float p0x, float p0y, float vx, fl
     return;
   }
   w.n = abs(imax - imin) + abs(jmax - jmin);
+  w.guarded = (min(imin, imax) >= -1) & (max(imin, imax) <= g.nx) & (min(jmin, jmax) >= -1) & (max(jmin, jmax) <= g.ny);
   w.iinc = vx > 0.f ? 1 : (vx < 0.f ? -1 : 0);
   w.jinc = vy > 0.f ? 1 : (vy < 0.f ? -1 : 0);
   const float ex = A_SUB(A_ADD(p0x, vx), p0x), ey = A_SUB(A_ADD(p0y, vy), p0y);
