@@ -103,6 +103,25 @@ def test_against_oracle(oracle, name):
             assert abs(lik.item() - want_lik) <= (1e-6 if listed else 1e-9) * abs(want_lik)
 
 
+@pytest.mark.parametrize("n", [1016, 1024, 1160, 1230])
+def test_widest_lists(oracle, n):
+    """Images around the widest whose crossing list fits a block's shared
+    memory (and wider: the padded pair): the listed pass and a projection."""
+    ig, sg = ImageGeom(n, n, 2, 0.4, 0.4, 4.0), Sino3DGeom.span1(3, 200, 16, 0.2 * n, 16 * 0.5, 400.0, 0)
+    rng = np.random.default_rng(n)
+    x0 = (rng.random(ig.n_voxels, dtype=np.float32) + 0.5).astype(np.float32)
+    est = oracle.project_3d(sg, ig, x0)
+    P = ap.SiddonProjector(ig, sg)
+    assert bits_equal(P.project(t(x0), zeros(est.size)).cpu().numpy(), est)
+    P.set_option(_lib.APIRL_OPT_SPARSE_IMAGE, _lib.APIRL_SPARSE_GEOMETRY)
+    meas = rng.poisson(est * 0.05).astype(np.float32)
+    G = P.backproject_ones(zeros(ig.n_voxels))
+    sens = np.ones(ig.n_voxels, np.float32)
+    x = P.em_pass_sparse(t(meas), t(x0), zeros(ig.n_voxels), t(sens), G)
+    bp = oracle.backproject_3d(sg, ig, oracle.inverse_divide(meas, est), threads=1)
+    assert rel(x.cpu().numpy(), oracle.update(x0, bp, sens, np.float32(0), True)) <= 1e-5
+
+
 def test_divide_at_the_ends_of_the_float_range(oracle):
     """Values and estimates whose ratio, or whose products with a segment,
     leave the float range: the same finite, infinite and NaN voxels as the
