@@ -4,20 +4,22 @@
 // downloading -> done.  apirl_batch_step takes each transition once the GPU
 // work of the previous stage has finished (per-job events; the engine never
 // synchronises its streams while jobs run), then launches one batched EM step:
-// one pass of every running job, or its final likelihood, in four launches
-// whatever the number of jobs (padded image copies and image dot products; a
-// persistent walk over the concatenated lists of all jobs' bins with counts;
-// the likelihood sums; the EM updates).
+// one pass of every running job, or its final likelihood, in four or five
+// launches whatever the number of jobs (image copies and image dot products;
+// the column walk of the jobs with 16 and more sinograms, a block per LOR,
+// beside a persistent walk over the concatenated lists of the other jobs'
+// bins with counts; the likelihood sums; the EM updates).
 //
 // * Device memory comes from a private stream-ordered pool that keeps what it
 //   has reserved, so jobs coming and going allocate nothing from the driver
 //   once the pool has grown to the working set.
 // * Counts, factors and initial images go up from a worker thread on a copy
 //   stream, so that a large job's upload overlaps the other jobs' steps.
-// * Each job's lists of bins with counts (one per subset) are built once, when
-//   its counts arrive; its passes walk only those bins (the geometry form of
-//   the sparse pass: the likelihood's sum over the other bins comes from the
-//   image dot product with G_s = A_s^T 1).
+// * The passes walk only the bins with counts (the geometry form of the sparse
+//   pass: the likelihood's sum over the other bins comes from the image dot
+//   product with G_s = A_s^T 1).  The column walk finds them in each block; the
+//   lists of the other jobs (one per subset) are built once, when their counts
+//   arrive.
 // * Geometry products are shared between jobs of the same image and sinogram
 //   geometry: the LOR tables, and A_a^T 1 for every angle a, from which the
 //   sensitivity images of any subset split (without a multiplicative term,
@@ -43,7 +45,9 @@
 #include "../../include/apirl_b200.h"
 
 using apirl::ImgGeom;
+using apirl::ColBuffers;
 using apirl::LorTable;
+using apirl::MultiCols;
 using apirl::MultiSeg;
 using apirl::MultiVox;
 using apirl::PadBuffers;
@@ -76,8 +80,15 @@ int64_t padded_voxels(const apirl_image_geom& g) {
 }
 int n_tiles_of(int64_t bins) { return (int)((bins + apirl::kNzTile - 1) / apirl::kNzTile); }
 
-// Device bytes a job holds while active, its lists at their largest (every
-// bin with counts) and its subset split's sensitivity images included.
+// Device bytes of a job's padded copies and backprojection pair, and of its
+// lists at their largest (every bin with counts).
+int64_t pads_and_lists(const apirl_image_geom& img, int64_t nbins) {
+  return 4 * align256(padded_voxels(img) * 4) + align256(nbins * 4);
+}
+
+// Device bytes a job holds while active, at most: as if it kept the padded
+// copies and its lists at their largest, its subset split's sensitivity
+// images included.
 int64_t footprint_of(const apirl_image_geom& img, const apirl_sino3d_geom& sino, int dtype, bool mult, bool add,
                      int nsub, int64_t nbins, int iters) {
   const int64_t nv = (int64_t)img.nx * img.ny * img.nz;
@@ -86,8 +97,7 @@ int64_t footprint_of(const apirl_image_geom& img, const apirl_sino3d_geom& sino,
   if (mult) b += align256(nbins * 4) + align256(nv * 4 * ns);  // factors, own sensitivity images
   if (add) b += align256(nbins * 4);
   b += align256(nv * 4);                                       // image
-  b += 4 * align256(padded_voxels(img) * 4);                   // padded copies and backprojection pair
-  b += align256(nbins * 4);                                    // lists of the bins with counts (at most every bin)
+  b += pads_and_lists(img, nbins);
   b += align256(((int64_t)ns * (nbins / (sino.n_proj > 0 ? sino.n_proj : 1) * ((sino.n_proj + ns - 1) / ns) /
                  apirl::kNzTile + 2)) * 4);                     // list tiles
   b += align256(((int64_t)iters * ns + 1) * 8) + align256(ns * 12);
@@ -225,6 +235,7 @@ struct Geom {
   ImgGeom g{};                   // the image geometry as the walk takes it
   LorTable t{};                  // LOR end points and end-point z, on the device (pool)
   std::vector<float> host_lor;   // the LOR table on the host, [angle][r] (p1x, p1y, p2x, p2y)
+  ColBuffers cols;               // the column layout's sizes (half 0: jobs keep to the padded copies)
   void* h_tables = nullptr;      // page-locked copy of the tables, the source of their upload
   int64_t nvox = 0, nbins = 0;
   // A_a^T 1 of every angle a (padded images of pv voxels, [z][x][y] where
@@ -268,6 +279,7 @@ struct Job {
   int* d_nlist = nullptr;
   int* d_list = nullptr;
   PadBuffers pad;
+  ColBuffers cols;               // or these, without lists (cols.half)
   std::vector<int64_t> tile_off, list_off;
   std::vector<int> n_list;
   std::vector<double> zero_add;
@@ -450,6 +462,8 @@ struct apirl_batch {
   int64_t next_id = 0;
   uint64_t clock = 0;
   cudaStream_t st = nullptr;  // compute
+  cudaStream_t side = nullptr;  // a step's lists, beside its columns on st
+  cudaEvent_t fork_ev = nullptr, join_ev = nullptr;
   Pool pool;
   PinnedPool pinned;
   Uploader up;
@@ -460,16 +474,18 @@ struct apirl_batch {
   // batched-step scratch
   int walk_blocks = 0;
   unsigned long long* d_counter = nullptr;
-  double* d_chunk_part = nullptr;
-  int64_t cap_chunks = 0;
+  double* d_part = nullptr;
+  int64_t cap_part = 0;
   double* d_tile_part = nullptr;
   int64_t cap_tiles = 0;
   MultiVox* d_vox = nullptr;
   MultiSeg* d_segs = nullptr;
-  int cap_vox = 0, cap_segs = 0;
+  MultiCols* d_cols = nullptr;
+  int64_t cap_vox = 0, cap_segs = 0, cap_cols = 0;
   MultiVox* h_vox[2] = {nullptr, nullptr};
   MultiSeg* h_segs[2] = {nullptr, nullptr};
-  int h_cap_vox = 0, h_cap_segs = 0;
+  MultiCols* h_cols[2] = {nullptr, nullptr};
+  int h_cap_vox = 0, h_cap_segs = 0, h_cap_cols = 0;
   cudaEvent_t step_ev[2] = {nullptr, nullptr};
   int64_t n_steps = 0;
 };
@@ -550,6 +566,13 @@ apirl_status geom_for(apirl_batch* b, Job& j, Geom** out) {
     g->nvox = j.nvox;
     g->nbins = j.nbins;
     g->pv = padded_voxels(j.img);
+    // The column layout, as a projector's, where a job's image copy and two
+    // sums in it take no more memory than its footprint counts.
+    if (g->t.n_sinos >= apirl::kColMinSinos) {
+      const float2* z = reinterpret_cast<const float2*>((const char*)g->h_tables + g->host_lor.size() * sizeof(float));
+      g->cols = apirl::col_layout(g->g, &z->x, 2 * g->t.n_sinos);
+      if (3 * align256(g->cols.floats * 4) > pads_and_lists(j.img, j.nbins)) g->cols = ColBuffers();
+    }
     // Rays of one angle are parallel in x-y: the angle's middle ray decides
     // its image layout (the layout is a matter of speed, not of results).
     const int np = g->key.n_proj, nr = g->key.n_r;
@@ -655,6 +678,8 @@ void release_job(apirl_batch* b, Job& j) {
   b->pool.release(j.pad.pT, s);
   b->pool.release(j.pad.bA, s);
   b->pool.release(j.pad.bT, s);
+  b->pool.release(j.cols.img, s);
+  b->pool.release(j.cols.acc, s);
   if (j.set) { j.set->refs--; j.set = nullptr; }
   if (j.geom) { j.geom->refs--; j.geom->last_use = ++b->clock; j.geom = nullptr; }
   b->pinned.put(j.h_stage); j.h_stage = nullptr;
@@ -691,19 +716,27 @@ apirl_status admit(apirl_batch* b, Job& j) {
   BK(b->pool.alloc(&j.d_x, j.nvox, s));
   BK(b->pool.alloc(&j.d_lik, (int64_t)j.iters * j.nsub + 1, s));
   BK(b->pool.alloc(&j.d_zero_add, j.nsub, s));
-  BK(b->pool.alloc(&j.d_nlist, j.nsub, s));
-  j.tile_off.assign(j.nsub + 1, 0);
-  for (int k = 0; k < j.nsub; k++)
-    j.tile_off[k + 1] = j.tile_off[k] + n_tiles_of((int64_t)j.geom->t.n_sinos *
-                                                   apirl::subset_nproj(j.sino.n_proj, k, j.nsub) * j.sino.n_r);
-  BK(b->pool.alloc(&j.d_tiles, std::max<int64_t>(j.tile_off[j.nsub], 1), s));
-  float* pads[4];
-  for (int k = 0; k < 4; k++) {
-    BK(b->pool.alloc(&pads[k], pv, s));
-    BK(cudaMemsetAsync(pads[k], 0, (size_t)pv * 4, s));
+  if (j.geom->cols.half) {
+    j.cols = j.geom->cols;
+    BK(b->pool.alloc(&j.cols.img, j.cols.floats, s));
+    BK(b->pool.alloc(&j.cols.acc, 2 * j.cols.floats, s));
+    BK(cudaMemsetAsync(j.cols.img, 0, (size_t)j.cols.floats * 4, s));
+    BK(cudaMemsetAsync(j.cols.acc, 0, (size_t)j.cols.floats * 8, s));
+  } else {
+    BK(b->pool.alloc(&j.d_nlist, j.nsub, s));
+    j.tile_off.assign(j.nsub + 1, 0);
+    for (int k = 0; k < j.nsub; k++)
+      j.tile_off[k + 1] = j.tile_off[k] + n_tiles_of((int64_t)j.geom->t.n_sinos *
+                                                     apirl::subset_nproj(j.sino.n_proj, k, j.nsub) * j.sino.n_r);
+    BK(b->pool.alloc(&j.d_tiles, std::max<int64_t>(j.tile_off[j.nsub], 1), s));
+    float* pads[4];
+    for (int k = 0; k < 4; k++) {
+      BK(b->pool.alloc(&pads[k], pv, s));
+      BK(cudaMemsetAsync(pads[k], 0, (size_t)pv * 4, s));
+    }
+    j.pad.pA = pads[0]; j.pad.pT = pads[1]; j.pad.bA = pads[2]; j.pad.bT = pads[3];
+    j.pad.lim = (unsigned)pv;
   }
-  j.pad.pA = pads[0]; j.pad.pT = pads[1]; j.pad.bA = pads[2]; j.pad.bT = pads[3];
-  j.pad.lim = (unsigned)pv;
   BK(cudaMemsetAsync(j.d_lik, 0, ((size_t)j.iters * j.nsub + 1) * 8, s));
   BK(cudaMemsetAsync(j.d_zero_add, 0, (size_t)j.nsub * 8, s));
   j.h_stage = b->pinned.get(stage_bytes(j.nsub));
@@ -718,21 +751,22 @@ apirl_status admit(apirl_batch* b, Job& j) {
   return APIRL_OK;
 }
 
-// Counts arrived: the initial image, the per-subset list lengths and
-// additive sums (read back), the own sensitivity of a job with factors.
+// Counts arrived: the initial image, the per-subset list lengths (of a job
+// that walks lists) and additive sums (read back), the own sensitivity of a
+// job with factors.
 apirl_status start_counting(apirl_batch* b, Job& j) {
   cudaStream_t s = b->st;
   BK(cudaStreamWaitEvent(s, j.up_ev, 0));
   if (!j.h_init) BK(apirl::launch_fill(j.nvox, j.d_x, 1.f, s));
   const LorTable& t = j.geom->t;
-  for (int k = 0; k < j.nsub; k++) {
+  for (int k = 0; k < j.nsub && !j.cols.half; k++) {
     SubsetSel ss;
     ss.subset = k; ss.nsub = j.nsub; ss.nk = apirl::subset_nproj(j.sino.n_proj, k, j.nsub);
     BK(apirl::launch_nz_count(t, ss, j.d_counts, j.dtype, (int64_t)t.n_sinos * ss.nk * t.n_r,
                               j.d_tiles + j.tile_off[k], j.d_nlist + k, s));
   }
   if (j.d_add) BK(apirl::launch_subset_sums(t, j.nsub, j.d_add, j.d_zero_add, s));
-  BK(cudaMemcpyAsync(j.h_stage, j.d_nlist, (size_t)j.nsub * 4, cudaMemcpyDeviceToHost, s));
+  if (!j.cols.half) BK(cudaMemcpyAsync(j.h_stage, j.d_nlist, (size_t)j.nsub * 4, cudaMemcpyDeviceToHost, s));
   BK(cudaMemcpyAsync((char*)j.h_stage + stage_zero_add_off(j.nsub), j.d_zero_add, (size_t)j.nsub * 8,
                      cudaMemcpyDeviceToHost, s));
   if (j.d_mult) {
@@ -749,23 +783,29 @@ apirl_status start_counting(apirl_batch* b, Job& j) {
 // List lengths known: the lists themselves, and the shared sensitivity.
 apirl_status start_running(apirl_batch* b, Job& j) {
   cudaStream_t s = b->st;
-  j.n_list.assign((const int*)j.h_stage, (const int*)j.h_stage + j.nsub);
   const double* za = (const double*)((char*)j.h_stage + stage_zero_add_off(j.nsub));
   j.zero_add.assign(za, za + j.nsub);
-  j.list_off.assign(j.nsub + 1, 0);
-  for (int k = 0; k < j.nsub; k++) j.list_off[k + 1] = j.list_off[k] + j.n_list[k];
-  BK(b->pool.alloc(&j.d_list, std::max<int64_t>(j.list_off[j.nsub], 1), s));
-  // the lists' reservation shrinks from every bin to the bins with counts
-  const int64_t unused = align256(j.nbins * 4) - align256(std::max<int64_t>(j.list_off[j.nsub], 1) * 4);
+  int64_t unused;
+  if (j.cols.half) {
+    // the columns in place of the padded copies and lists
+    unused = pads_and_lists(j.img, j.nbins) - 3 * align256(j.cols.floats * 4);
+  } else {
+    j.n_list.assign((const int*)j.h_stage, (const int*)j.h_stage + j.nsub);
+    j.list_off.assign(j.nsub + 1, 0);
+    for (int k = 0; k < j.nsub; k++) j.list_off[k + 1] = j.list_off[k] + j.n_list[k];
+    BK(b->pool.alloc(&j.d_list, std::max<int64_t>(j.list_off[j.nsub], 1), s));
+    // the lists' reservation shrinks from every bin to the bins with counts
+    unused = align256(j.nbins * 4) - align256(std::max<int64_t>(j.list_off[j.nsub], 1) * 4);
+    const LorTable& t = j.geom->t;
+    for (int k = 0; k < j.nsub; k++) {
+      SubsetSel ss;
+      ss.subset = k; ss.nsub = j.nsub; ss.nk = apirl::subset_nproj(j.sino.n_proj, k, j.nsub);
+      BK(apirl::launch_nz_write(t, ss, j.d_counts, j.dtype, (int64_t)t.n_sinos * ss.nk * t.n_r,
+                                j.d_tiles + j.tile_off[k], j.d_list + j.list_off[k], s));
+    }
+  }
   j.charged -= unused;
   b->used -= unused;
-  const LorTable& t = j.geom->t;
-  for (int k = 0; k < j.nsub; k++) {
-    SubsetSel ss;
-    ss.subset = k; ss.nsub = j.nsub; ss.nk = apirl::subset_nproj(j.sino.n_proj, k, j.nsub);
-    BK(apirl::launch_nz_write(t, ss, j.d_counts, j.dtype, (int64_t)t.n_sinos * ss.nk * t.n_r,
-                              j.d_tiles + j.tile_off[k], j.d_list + j.list_off[k], s));
-  }
   BS(ensure_sensitivity(b, j));
   j.stage = j.iters * j.nsub > 0 ? Stage::Running : Stage::Final;
   return APIRL_OK;
@@ -781,30 +821,28 @@ apirl_status grow(apirl_batch* b, T** d, int64_t* cap, int64_t need) {
   return APIRL_OK;
 }
 
-// Room for nv job and ns segment descriptors in both page-locked slots.  The
-// old blocks go back to the pool only once no copy from either slot is in
-// flight (the other slot's was queued one step ago).
-apirl_status grow_host(apirl_batch* b, int nv, int ns) {
-  if (nv <= b->h_cap_vox && ns <= b->h_cap_segs) return APIRL_OK;
+template <typename T>
+apirl_status grow_slots(apirl_batch* b, T* (&slots)[2], int* cap, int need) {
+  if (need <= *cap) return APIRL_OK;
+  for (int k = 0; k < 2; k++) {
+    b->pinned.put(slots[k]);
+    slots[k] = (T*)b->pinned.get((size_t)(2 * need) * sizeof(T));
+    if (!slots[k]) return bfail(APIRL_ERR_OOM, "page-locked step descriptors");
+  }
+  *cap = 2 * need;
+  return APIRL_OK;
+}
+
+// Room for nv job, ns list and nc column segment descriptors in both
+// page-locked slots.  The old blocks go back to the pool only once no copy
+// from either slot is in flight (the other slot's was queued one step ago).
+apirl_status grow_host(apirl_batch* b, int nv, int ns, int nc) {
+  if (nv <= b->h_cap_vox && ns <= b->h_cap_segs && nc <= b->h_cap_cols) return APIRL_OK;
   BK(cudaEventSynchronize(b->step_ev[0]));
   BK(cudaEventSynchronize(b->step_ev[1]));
-  if (nv > b->h_cap_vox) {
-    for (int k = 0; k < 2; k++) {
-      b->pinned.put(b->h_vox[k]);
-      b->h_vox[k] = (MultiVox*)b->pinned.get((size_t)(2 * nv) * sizeof(MultiVox));
-      if (!b->h_vox[k]) return bfail(APIRL_ERR_OOM, "page-locked step descriptors");
-    }
-    b->h_cap_vox = 2 * nv;
-  }
-  if (ns > b->h_cap_segs) {
-    for (int k = 0; k < 2; k++) {
-      b->pinned.put(b->h_segs[k]);
-      b->h_segs[k] = (MultiSeg*)b->pinned.get((size_t)(2 * ns) * sizeof(MultiSeg));
-      if (!b->h_segs[k]) return bfail(APIRL_ERR_OOM, "page-locked step descriptors");
-    }
-    b->h_cap_segs = 2 * ns;
-  }
-  return APIRL_OK;
+  BS(grow_slots(b, b->h_vox, &b->h_cap_vox, nv));
+  BS(grow_slots(b, b->h_segs, &b->h_cap_segs, ns));
+  return grow_slots(b, b->h_cols, &b->h_cap_cols, nc);
 }
 
 // One batched EM step over `jobs` (running: their next pass; final: their
@@ -813,16 +851,21 @@ apirl_status grow_host(apirl_batch* b, int nv, int ns) {
 apirl_status launch_step(apirl_batch* b, std::vector<Job*>& jobs) {
   if (jobs.empty()) return APIRL_OK;
   std::stable_sort(jobs.begin(), jobs.end(), [](const Job* a, const Job* c) { return a->nvox > c->nvox; });
-  int nsegs = 0;
-  for (Job* j : jobs) nsegs += j->stage == Stage::Final ? j->nsub : 1;
+  int nsegs = 0, ncols = 0;
+  for (Job* j : jobs) {
+    if (j->cols.half) ncols++;
+    else nsegs += j->stage == Stage::Final ? j->nsub : 1;
+  }
   const int slot = (int)(b->n_steps & 1);
   // the page-locked slot was last copied from two steps ago
   BK(cudaEventSynchronize(b->step_ev[slot]));
-  BS(grow_host(b, (int)jobs.size(), nsegs));
+  BS(grow_host(b, (int)jobs.size(), nsegs, ncols));
   MultiVox* hv = b->h_vox[slot];
   MultiSeg* hs = b->h_segs[slot];
-  int64_t tiles = 0, chunks = 0;
-  int si = 0;
+  MultiCols* hc = b->h_cols[slot];
+  int64_t tiles = 0, chunks = 0, lors = 0;
+  size_t col_smem = 0;
+  int si = 0, ci = 0;
   for (size_t q = 0; q < jobs.size(); q++) {
     Job& j = *jobs[q];
     const bool fin = j.stage == Stage::Final;
@@ -831,18 +874,39 @@ apirl_status launch_step(apirl_batch* b, std::vector<Job*>& jobs) {
     MultiVox& V = hv[q];
     V.g = gm.g;
     V.pad = j.pad;
+    V.cols = j.cols;
     V.x = j.d_x;
     V.sens = fin ? nullptr : (j.d_sens ? j.d_sens + (int64_t)sub * j.nvox : j.set->g + (int64_t)sub * j.nvox);
     V.gimg = fin ? j.geom->g_total : j.set->g + (int64_t)sub * j.nvox;
     V.lik = j.d_lik + (fin ? (int64_t)j.iters * j.nsub : j.pass);
     V.tile_begin = tiles;
     V.tiles_x = (gm.g.nx + 31) / 32;
-    V.tiles_y = (gm.g.ny + 31) / 32;
-    tiles += apirl::multi_tiles(gm.g);
-    V.chunk_begin = chunks;
+    V.tiles_y = j.cols.half ? gm.g.ny : (gm.g.ny + 31) / 32;
+    V.tiles_z = j.cols.half ? (gm.g.nz + 31) / 32 : gm.g.nz;
+    tiles += (int64_t)V.tiles_x * V.tiles_y * V.tiles_z;
+    V.part_begin = chunks;
     V.update = fin ? 0 : 1;
     V.ge = j.positive ? 0 : 1;  // OsemSinogram3d's rule: sens >= 0 (threshold 0), or sens > 0
     V.zero_add = 0.0;
+    for (int k = fin ? 0 : sub; k < (fin ? j.nsub : sub + 1); k++) V.zero_add += j.zero_add[k];
+    if (j.cols.half) {
+      MultiCols& S = hc[ci++];
+      S.g = gm.g;
+      S.t = gm.t;
+      S.s.subset = fin ? -1 : sub; S.s.nsub = j.nsub;
+      S.s.nk = fin ? j.sino.n_proj : apirl::subset_nproj(j.sino.n_proj, sub, j.nsub);
+      S.counts = j.d_counts;
+      S.counts_dtype = j.dtype;
+      S.add = j.d_add;
+      S.cols = j.cols;
+      S.lor_begin = lors;
+      S.back = fin ? 0 : 1;
+      V.part_begin = lors;  // behind the chunks', below
+      V.n_parts = (int64_t)S.s.nk * j.sino.n_r;
+      lors += V.n_parts;
+      col_smem = std::max(col_smem, apirl::col_list_bytes(gm.g));
+      continue;
+    }
     for (int k = fin ? 0 : sub; k < (fin ? j.nsub : sub + 1); k++) {
       MultiSeg& S = hs[si++];
       S.g = gm.g;
@@ -857,21 +921,22 @@ apirl_status launch_step(apirl_batch* b, std::vector<Job*>& jobs) {
       S.chunk_begin = chunks;
       S.back = fin ? 0 : 1;
       chunks += (S.n_list + 31) / 32;
-      V.zero_add += j.zero_add[k];
     }
-    V.n_chunks = chunks - V.chunk_begin;
+    V.n_parts = chunks - V.part_begin;
   }
-  int64_t cv = b->cap_vox, cs = b->cap_segs;
-  BS(grow(b, &b->d_vox, &cv, (int64_t)jobs.size()));
-  BS(grow(b, &b->d_segs, &cs, nsegs));
-  b->cap_vox = (int)cv;
-  b->cap_segs = (int)cs;
-  BS(grow(b, &b->d_chunk_part, &b->cap_chunks, std::max<int64_t>(chunks, 1)));
+  for (size_t q = 0; q < jobs.size(); q++)
+    if (hv[q].cols.half) hv[q].part_begin += chunks;
+  BS(grow(b, &b->d_vox, &b->cap_vox, (int64_t)jobs.size()));
+  BS(grow(b, &b->d_segs, &b->cap_segs, nsegs));
+  BS(grow(b, &b->d_cols, &b->cap_cols, ncols));
+  BS(grow(b, &b->d_part, &b->cap_part, std::max<int64_t>(chunks + lors, 1)));
   BS(grow(b, &b->d_tile_part, &b->cap_tiles, tiles));
   BK(cudaMemcpyAsync(b->d_vox, hv, jobs.size() * sizeof(MultiVox), cudaMemcpyHostToDevice, b->st));
-  BK(cudaMemcpyAsync(b->d_segs, hs, (size_t)nsegs * sizeof(MultiSeg), cudaMemcpyHostToDevice, b->st));
-  BK(apirl::launch_multi_step(b->d_vox, (int)jobs.size(), tiles, b->d_segs, nsegs, chunks, b->walk_blocks,
-                              b->d_counter, b->d_chunk_part, b->d_tile_part, b->st));
+  if (nsegs) BK(cudaMemcpyAsync(b->d_segs, hs, (size_t)nsegs * sizeof(MultiSeg), cudaMemcpyHostToDevice, b->st));
+  if (ncols) BK(cudaMemcpyAsync(b->d_cols, hc, (size_t)ncols * sizeof(MultiCols), cudaMemcpyHostToDevice, b->st));
+  const apirl::MultiStep m{b->d_vox, (int)jobs.size(), tiles, b->d_segs, nsegs, chunks, b->d_cols, ncols, lors, col_smem,
+                           b->walk_blocks, b->d_counter, b->d_part, b->d_tile_part};
+  BK(apirl::launch_multi_step(m, b->st, b->side, b->fork_ev, b->join_ev));
   BK(cudaEventRecord(b->step_ev[slot], b->st));
   b->n_steps++;
   for (Job* j : jobs) {
@@ -919,6 +984,9 @@ apirl_status apirl_batch_create(int device, int64_t budget, apirl_batch** out) {
   b->device = device;
   b->budget = budget;
   BK(cudaStreamCreateWithFlags(&b->st, cudaStreamNonBlocking));
+  BK(cudaStreamCreateWithFlags(&b->side, cudaStreamNonBlocking));
+  BK(cudaEventCreateWithFlags(&b->fork_ev, cudaEventDisableTiming));
+  BK(cudaEventCreateWithFlags(&b->join_ev, cudaEventDisableTiming));
   const unsigned hw = std::thread::hardware_concurrency();
   BK(b->up.init(device, hw >= 8 ? 4 : (hw >= 2 ? 2 : 1)));
   BK(b->pool.create(device));
@@ -956,6 +1024,7 @@ void apirl_batch_destroy(apirl_batch* b) {
   cudaSetDevice(b->device);
   b->up.shutdown();
   cudaStreamSynchronize(b->up.st);
+  cudaStreamSynchronize(b->side);
   cudaStreamSynchronize(b->st);
   for (auto& j : b->active) { release_job(b, *j); destroy_events(*j); }
   for (auto& j : b->queue) destroy_events(*j);
@@ -971,20 +1040,25 @@ void apirl_batch_destroy(apirl_batch* b) {
     b->pool.release(z, b->st);
   }
   b->pool.release(b->d_counter, b->st);
-  b->pool.release(b->d_chunk_part, b->st);
+  b->pool.release(b->d_part, b->st);
   b->pool.release(b->d_tile_part, b->st);
   b->pool.release(b->d_vox, b->st);
   b->pool.release(b->d_segs, b->st);
+  b->pool.release(b->d_cols, b->st);
   cudaStreamSynchronize(b->st);
   for (auto& kv : b->geoms) b->pinned.put(kv.second->h_tables);
   for (int k = 0; k < 2; k++) {
     b->pinned.put(b->h_vox[k]);
     b->pinned.put(b->h_segs[k]);
+    b->pinned.put(b->h_cols[k]);
     if (b->step_ev[k]) cudaEventDestroy(b->step_ev[k]);
   }
   if (b->pool.pool) cudaMemPoolDestroy(b->pool.pool);
   b->up.release();
   cudaStreamDestroy(b->st);
+  cudaStreamDestroy(b->side);
+  cudaEventDestroy(b->fork_ev);
+  cudaEventDestroy(b->join_ev);
   cudaSetDevice(prev);
   delete b;
 }

@@ -43,4 +43,22 @@ __device__ __forceinline__ double lik_term(float m, float e, int skip_zero) {
   return skip_zero == 2 ? (double)m * log((double)e) : (double)m * log((double)e) - (double)e;
 }
 
+__device__ __forceinline__ float load_count_any(const void* p, int dtype, int64_t i) {
+  if (dtype == APIRL_U32) return (float)__ldg((const uint32_t*)p + i);
+  if (dtype == APIRL_U16) return (float)__ldg((const uint16_t*)p + i);
+  return __ldg((const float*)p + i);
+}
+
+// The last of n entries whose first (block, tile or chunk) key(e) is <= k;
+// entries are ordered by key.
+template <typename J, class Key>
+__device__ __forceinline__ int find_entry(const J* __restrict__ e, int n, int64_t k, Key key) {
+  int lo = 0, hi = n - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (key(e[mid]) <= k) lo = mid; else hi = mid - 1;
+  }
+  return lo;
+}
+
 }  // namespace apirl

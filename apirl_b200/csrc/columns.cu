@@ -17,8 +17,7 @@
 #include <cuda_runtime.h>
 #include <cmath>
 #include <cstdint>
-#include "bins.cuh"
-#include "columns.cuh"
+#include "columns_em.cuh"
 #include "internal.h"
 
 namespace apirl {
@@ -35,19 +34,12 @@ constexpr int kColWarps = kColBlock / 32;
 // Blocks of the LORs with few counts.
 constexpr int kColFewBlock = 64;
 constexpr int kColFewBlocks = 20;
-
-struct ColLor {
-  int k, l, a;  // subset angle, r, full angle
-};
-
-// LOR `at` of the subset, r first.
-__device__ __forceinline__ ColLor col_lor(const LorTable& t, const SubsetSel& s, unsigned at) {
-  ColLor c;
-  c.k = (int)(at / (unsigned)t.n_r);
-  c.l = (int)(at - (unsigned)c.k * (unsigned)t.n_r);
-  c.a = s.subset < 0 ? c.k : s.subset + s.nsub * c.k;
-  return c;
-}
+// Blocks of the batched pass, whose LORs have from a few to hundreds of
+// counts: ten mixed jobs of 64 - 128 x 1 - 41 slices in 16.7 ms, against 18.0 /
+// 17.6 / 17.8 / 20.4 ms with 64 / 96 / 160 / 256 threads and 18.1 ms at 8 blocks
+// (64 registers).
+constexpr int kMultiColBlock = 128;
+constexpr int kMultiColBlocks = 10;
 
 __global__ void __launch_bounds__(kColBlock, kColBlocks) k_project_cols(ImgGeom g, ColDims d, LorTable t, SubsetSel s,
                                                             const float* __restrict__ img, float* __restrict__ out) {
@@ -116,43 +108,9 @@ __global__ void __launch_bounds__(kColBlock, kColBlocks) k_scatter_cols(ImgGeom 
   }
 }
 
-// The fused pass (k_em_pass_persist's steps, kernels.cu) of the warp's 32
-// rays: forward walk, additive term, likelihood term, ratio, and the ratio
-// scattered along the walk.  Returns the lane's likelihood term.
-template <typename CT>
-__device__ __forceinline__ double em_rays(const ImgGeom& g, const ColDims& d, const LorTable& t, const SubsetSel& s,
-                                          const ColLor& lor, const float4 P, int gl, bool in,
-                                          const CT* __restrict__ counts, int counts_packed,
-                                          const float* __restrict__ add, const float* __restrict__ img,
-                                          float* __restrict__ acc, int back, int skip_zero) {
-  const ColWalk& w = col_head();
-  acc += w.xmain ? d.floats() : 0;
-  const int64_t row = counts_packed ? (int64_t)gl * s.nk + lor.k : (int64_t)(t.g0 + gl) * t.n_proj + lor.a;
-  const int64_t ci = row * t.n_r + lor.l;
-  const float m = in ? load_count<CT>(counts, ci) : 0.f;
-  const float2 ez = in ? __ldg(t.z + t.g0 + gl) : make_float2(0.f, 0.f);
-  ColGather sum;
-  WalkZ r = col_no_ray();
-  if (w.listed) {
-    if (in) r = col_setup_z(ez, w, g, d);
-    col_walk(r, d, img, sum);
-  } else if (in) {
-    col_walk_checked(P, ez, g, d, img, sum);
-  }
-  double term = 0.0;
-  float q = 0.f;
-  if (in) {
-    float e = sum.acc;
-    if (add) e = A_ADD(e, __ldg(add + ci));
-    if (e != 0.f) term = lik_term(m, e, skip_zero);
-    q = (m != 0.f && e != 0.f && back) ? A_DIV(m, e) : 0.f;
-  }
-  if (__any_sync(0xffffffffu, q != 0.f)) {
-    ColScatter out{q};
-    if (w.listed) col_walk(q != 0.f ? r : col_no_ray(), d, acc, out);
-    else if (q != 0.f) col_walk_checked(P, ez, g, d, acc, out);
-  }
-  return term;
+// Place of a bin (sinogram gl of the shard) in the counts / additive layout.
+__device__ __forceinline__ int64_t bin_of(const LorTable& t, const SubsetSel& s, const ColLor& lor, int gl, int packed) {
+  return (packed ? (int64_t)gl * s.nk + lor.k : (int64_t)(t.g0 + gl) * t.n_proj + lor.a) * t.n_r + lor.l;
 }
 
 // The LOR's likelihood partial: the sum of the block's terms, warps in order.
@@ -181,64 +139,11 @@ __global__ void __launch_bounds__(kColBlock, kColBlocks) k_em_cols(
   double term = 0.0;
   for (int g0 = threadIdx.x & ~31; g0 < t.n_sinos; g0 += blockDim.x) {
     const int gl = g0 + (threadIdx.x & 31);
-    term += em_rays<CT>(g, d, t, s, lor, P, gl, gl < t.n_sinos, counts, counts_packed, add, img, acc, back, 0);
+    const bool in = gl < t.n_sinos;
+    const int64_t ci = bin_of(t, s, lor, gl, counts_packed);
+    term += em_rays(g, d, t, P, gl, in, in ? load_count<CT>(counts, ci) : 0.f, ci, add, img, acc, back, 0);
   }
   em_partial(term, blockIdx.x, partials);
-}
-
-// The block's list of a LOR's sinograms with counts, among kColWindow from
-// g0: list[0 .. n) in order, n returned to every thread.
-constexpr int kColWindow = 2048;
-struct ColActive {
-  unsigned mask[kColWindow / 32];
-  int first[kColWindow / 32];
-  int n;
-  uint16_t list[kColWindow];
-};
-template <typename CT>
-__device__ __forceinline__ int col_active(const LorTable& t, const SubsetSel& s, const ColLor& lor, int g0,
-                                          const CT* __restrict__ counts, int counts_packed, ColActive& act) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int left = min(t.n_sinos - g0, kColWindow), groups = (left + 31) >> 5;
-  const int64_t step = (int64_t)(counts_packed ? s.nk : t.n_proj) * t.n_r;  // from a sinogram to the next
-  const CT* const first = counts + (counts_packed ? (int64_t)g0 * s.nk + lor.k : (int64_t)(t.g0 + g0) * t.n_proj + lor.a) * t.n_r +
-                          lor.l;
-  const int warps = blockDim.x >> 5;
-  for (int q = warp; q < groups; q += 4 * warps) {  // four groups' counts in flight
-    float m[4];
-    #pragma unroll
-    for (int u = 0; u < 4; u++) {
-      const int i = (q + u * warps) * 32 + lane;
-      m[u] = i < left ? load_count<CT>(first, i * step) : 0.f;
-    }
-    #pragma unroll
-    for (int u = 0; u < 4; u++) {
-      const unsigned mask = __ballot_sync(0xffffffffu, m[u] != 0.f);
-      if (lane == 0 && q + u * warps < groups) act.mask[q + u * warps] = mask;
-    }
-  }
-  __syncthreads();
-  if (warp == 0) {
-    static_assert(kColWindow / 32 == 64, "two groups a lane");
-    const int a = 2 * lane < groups ? __popc(act.mask[2 * lane]) : 0;
-    const int b = 2 * lane + 1 < groups ? __popc(act.mask[2 * lane + 1]) : 0;
-    int incl = a + b;
-    #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int u = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += u;
-    }
-    act.first[2 * lane] = incl - a - b;
-    act.first[2 * lane + 1] = incl - b;
-    if (lane == 31) act.n = incl;
-  }
-  __syncthreads();
-  for (int q = warp; q < groups; q += warps) {
-    const unsigned m = act.mask[q];
-    if (m >> lane & 1u) act.list[act.first[q] + __popc(m & ((1u << lane) - 1u))] = (uint16_t)(q * 32 + lane);
-  }
-  __syncthreads();
-  return act.n;
 }
 
 // The fused pass over the bins with counts: a block lists its LOR's
@@ -255,10 +160,12 @@ __global__ void __launch_bounds__(kColBlock, kColBlocks) k_em_cols_listed(
   __shared__ unsigned slot;
   const ColLor lor = col_lor(t, s, blockIdx.x);
   const float4 P = __ldg(t.lor + (int64_t)lor.a * t.n_r + lor.l);
+  const int64_t step = (int64_t)(counts_packed ? s.nk : t.n_proj) * t.n_r;  // from a sinogram to the next
   bool listed = false;
   double term = 0.0;
   for (int g0 = 0; g0 < t.n_sinos; g0 += kColWindow) {
-    const int n = col_active<CT>(t, s, lor, g0, counts, counts_packed, act);
+    const int64_t first = bin_of(t, s, lor, g0, counts_packed);
+    const int n = col_active(t.n_sinos, g0, [&](int i) { return load_count<CT>(counts, first + i * step); }, act);
     if (n <= few && t.n_sinos <= kColWindow) {
       if (n == 0) {
         if (threadIdx.x == 0) partials[blockIdx.x] = 0.0;
@@ -279,8 +186,9 @@ __global__ void __launch_bounds__(kColBlock, kColBlocks) k_em_cols_listed(
     for (int i0 = threadIdx.x & ~31; i0 < n; i0 += blockDim.x) {
       const int i = i0 + (threadIdx.x & 31);
       const bool in = i < n;
-      term += em_rays<CT>(g, d, t, s, lor, P, in ? g0 + act.list[i] : 0, in, counts, counts_packed, add, img, acc,
-                          back, skip_zero);
+      const int gl = in ? g0 + act.list[i] : 0;
+      const int64_t ci = bin_of(t, s, lor, gl, counts_packed);
+      term += em_rays(g, d, t, P, gl, in, in ? load_count<CT>(counts, ci) : 0.f, ci, add, img, acc, back, skip_zero);
     }
     __syncthreads();
   }
@@ -304,70 +212,85 @@ __global__ void __launch_bounds__(kColFewBlock, kColFewBlocks) k_em_cols_few(
       const int i = i0 + (threadIdx.x & 31);
       const bool in = i < n;
       const int gl = in ? queue.list[(int64_t)q * kColFew + i] : 0;
-      term += em_rays<CT>(g, d, t, s, lor, P, gl, in, counts, counts_packed, add, img, acc, back, skip_zero);
+      const int64_t ci = bin_of(t, s, lor, gl, counts_packed);
+      term += em_rays(g, d, t, P, gl, in, in ? load_count<CT>(counts, ci) : 0.f, ci, add, img, acc, back, skip_zero);
     }
     em_partial(term, item.x, partials);
     __syncthreads();
   }
 }
 
-// ---- images to and from the column layout -----------------------------------
-// A block works 32 x of one row y and 32 slices z0 .. z0 + 31, 32 x 8 threads;
-// tile[par * 16 + z / 2][x]: the slices in the order the columns store them.
+// The listed pass of many jobs (geometry form of the likelihood): LORs
+// lor_begin .. of the segments, a block each, whose descriptor stays in shared
+// memory.  Bound by the gathers' latency and the issue slots, as the single
+// pass.  Ten mixed jobs of two iterations (single-slice ones on lists): walks
+// 11.2 -> 8.5 + 1.0 ms, bin lists 2.1 -> 0.4 ms, the whole 20.6 -> 17.1 ms.
+__global__ void __launch_bounds__(kMultiColBlock, kMultiColBlocks) k_em_multi_cols(const MultiCols* __restrict__ segs,
+                                                                                  int nseg,
+                                                                                  double* __restrict__ partials) {
+  __shared__ ColActive act;
+  static_assert(sizeof(MultiCols) % 8 == 0, "segment copy");
+  __shared__ __align__(16) int seg_raw[sizeof(MultiCols) / 4];
+  __shared__ int sk;
+  const MultiCols& S = *reinterpret_cast<const MultiCols*>(seg_raw);
+  if (threadIdx.x == 0) sk = find_entry(segs, nseg, blockIdx.x, [](const MultiCols& e) { return e.lor_begin; });
+  __syncthreads();
+  for (int i = threadIdx.x; i < (int)(sizeof(MultiCols) / 4); i += blockDim.x)
+    seg_raw[i] = __ldg(reinterpret_cast<const int*>(segs + sk) + i);
+  __syncthreads();
+  const ColLor lor = col_lor(S.t, S.s, blockIdx.x - (unsigned)S.lor_begin);
+  const ColDims d{S.g.nx, S.g.ny, S.g.nz, S.cols.z0, S.cols.half};
+  const float4 P = __ldg(S.t.lor + (int64_t)lor.a * S.t.n_r + lor.l);
+  const int64_t step = (int64_t)S.t.n_proj * S.t.n_r;
+  bool listed = false;
+  double term = 0.0;
+  for (int g0 = 0; g0 < S.t.n_sinos; g0 += kColWindow) {
+    const int64_t first = bin_of(S.t, S.s, lor, g0, 0);
+    const int n = col_active(S.t.n_sinos, g0, [&](int i) {
+      return load_count_any(S.counts, S.counts_dtype, first + i * step); }, act);
+    if (n > 0 && !listed) {
+      col_list(P, S.g, d);
+      listed = true;
+    }
+    for (int i0 = threadIdx.x & ~31; i0 < n; i0 += blockDim.x) {
+      const int i = i0 + (threadIdx.x & 31);
+      const bool in = i < n;
+      const int gl = in ? g0 + act.list[i] : 0;
+      const int64_t ci = bin_of(S.t, S.s, lor, gl, 0);
+      term += em_rays(S.g, d, S.t, P, gl, in, in ? load_count_any(S.counts, S.counts_dtype, ci) : 0.f, ci, S.add,
+                      S.cols.img, S.cols.acc, S.back, 2);
+    }
+    __syncthreads();
+  }
+  em_partial(term, blockIdx.x, partials);
+}
 
-// img's interior <- x ([z][y][x]).  With gimg: dots[block] = - (x . gimg) over
-// the block's voxels where gimg != 0 (k_neg_dot's rule, kernels.cu), FP64.
-// queue_n (may be null) is set to 0.
+// ---- images to and from the column layout -----------------------------------
+// img's interior <- x; with gimg: dots[block] = - (x . gimg) over the block's
+// voxels.  queue_n (may be null) is set to 0.
 __global__ void __launch_bounds__(256) k_col_copy(ColDims d, const float* __restrict__ x, float* __restrict__ img,
                                                   const float* __restrict__ gimg, double* __restrict__ dots,
                                                   unsigned* __restrict__ queue_n) {
   __shared__ float tile[32][33];
   __shared__ double part[8];
-  const int lx = threadIdx.x, ly = threadIdx.y, x0 = blockIdx.x * 32, y = blockIdx.y, z0 = blockIdx.z * 32;
+  const int lx = threadIdx.x, ly = threadIdx.y;
   if (queue_n && (blockIdx.x | blockIdx.y | blockIdx.z) == 0 && (lx | ly) == 0) *queue_n = 0;
-  float v[4], gv[4];
+  double s = col_copy_tile(d, x, img, gimg, blockIdx.x * 32, blockIdx.y, blockIdx.z * 32, lx, ly, tile);
+  if (!gimg) return;
   #pragma unroll
-  for (int q = 0; q < 4; q++) {
-    const int z = z0 + ly + 8 * q;
-    const bool in = x0 + lx < d.nx && z < d.nz;
-    const int64_t i = ((int64_t)z * d.ny + y) * d.nx + x0 + lx;
-    v[q] = in ? x[i] : 0.f;
-    gv[q] = gimg && in ? gimg[i] : 0.f;
-  }
-  #pragma unroll
-  for (int q = 0; q < 4; q++) {
-    const int z = ly + 8 * q;
-    tile[(z & 1) * 16 + (z >> 1)][lx] = v[q];
-  }
-  if (gimg) {
-    double s = 0.0;
-    #pragma unroll
-    for (int q = 0; q < 4; q++)
-      if (gv[q] != 0.f) s += (double)v[q] * (double)gv[q];
-    #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-    if (lx == 0) part[ly] = s;
-  }
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+  if (lx == 0) part[ly] = s;
   __syncthreads();
-  const int par = lx >> 4, z = z0 + 2 * (lx & 15) + par;
-  #pragma unroll
-  for (int q = 0; q < 4; q++) {
-    const int xx = ly + 8 * q;
-    if (x0 + xx < d.nx && z < d.nz)
-      img[((int64_t)(y + kPad) * d.px() + x0 + xx + kPad) * d.stride() + par * d.half + ((z + d.z0) >> 1)] =
-          tile[lx][xx];
-  }
-  if (gimg && lx == 0 && ly == 0) {
-    double s = 0.0;
+  if (lx == 0 && ly == 0) {
+    s = 0.0;
     for (int i = 0; i < 8; i++) s += part[i];
     dots[((int64_t)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x] = -s;
   }
 }
 
-// mode 0: EM update of x from the column sums acc (rule ge / gt, as k_update);
-// mode 1: bp += acc.  acc's interior cleared, after the block's loads.  With
-// lik: one more layer of blocks (z = 0), whose first sums the n likelihood
-// partials in a fixed order, less *less (may be null), beside the others' work.
+// The update of x (mode 0) or bp (mode 1) from the column sums.  With lik: one
+// more layer of blocks (z = 0), whose first sums the n likelihood partials in a
+// fixed order, less *less (may be null), beside the others' work.
 __global__ void __launch_bounds__(256) k_col_reduce(ColDims d, float* __restrict__ acc, int mode,
                                                     float* __restrict__ x, float* __restrict__ bp,
                                                     const float* __restrict__ sens,
@@ -399,52 +322,8 @@ __global__ void __launch_bounds__(256) k_col_reduce(ColDims d, float* __restrict
     return;
   }
   const float thr = (mode == 0 && thr_ptr) ? *thr_ptr : thr_value;
-  const int lx = threadIdx.x, ly = threadIdx.y, x0 = blockIdx.x * 32, y = blockIdx.y,
-            z0 = (lik ? blockIdx.z - 1 : blockIdx.z) * 32;
-  const int par = lx >> 4, zc = z0 + 2 * (lx & 15) + par;
-  float* out = mode == 0 ? x : bp;
-  float xv[4], sv[4];
-  #pragma unroll
-  for (int q = 0; q < 4; q++) {
-    const int xx = ly + 8 * q;
-    if (x0 + xx < d.nx && zc < d.nz) {
-      const float* a = acc + ((int64_t)(y + kPad) * d.px() + x0 + xx + kPad) * d.stride() + par * d.half +
-                       ((zc + d.z0) >> 1);
-      tile[lx][xx] = A_ADD(a[0], a[d.floats()]);
-    }
-  }
-  #pragma unroll
-  for (int q = 0; q < 4; q++) {
-    const int z = z0 + ly + 8 * q;
-    xv[q] = sv[q] = 0.f;
-    if (x0 + lx < d.nx && z < d.nz) {
-      const int64_t i = ((int64_t)z * d.ny + y) * d.nx + x0 + lx;
-      xv[q] = out[i];
-      if (mode == 0) sv[q] = sens[i];
-    }
-  }
-  __syncthreads();
-  #pragma unroll
-  for (int q = 0; q < 4; q++) {
-    const int xx = ly + 8 * q;
-    if (x0 + xx < d.nx && zc < d.nz) {
-      float* a = acc + ((int64_t)(y + kPad) * d.px() + x0 + xx + kPad) * d.stride() + par * d.half + ((zc + d.z0) >> 1);
-      a[0] = a[d.floats()] = 0.f;
-    }
-  }
-  #pragma unroll
-  for (int q = 0; q < 4; q++) {
-    const int zl = ly + 8 * q, z = z0 + zl;
-    if (x0 + lx >= d.nx || z >= d.nz) continue;
-    const int64_t i = ((int64_t)z * d.ny + y) * d.nx + x0 + lx;
-    const float b = tile[(zl & 1) * 16 + (zl >> 1)][lx];
-    if (mode == 0) {
-      const bool okv = ge ? (sv[q] >= thr) : (sv[q] > thr);
-      out[i] = okv ? A_DIV(A_MUL(xv[q], b), sv[q]) : 0.f;
-    } else {
-      out[i] = A_ADD(xv[q], b);
-    }
-  }
+  col_reduce_tile(d, acc, mode, x, bp, sens, thr, ge, blockIdx.x * 32, blockIdx.y,
+                  (lik ? blockIdx.z - 1 : blockIdx.z) * 32, threadIdx.x, threadIdx.y, tile);
 }
 
 // The list's shared memory: with the kernels' own (the listed pass's 4.7 KB)
@@ -486,6 +365,20 @@ ColBuffers col_layout(const ImgGeom& g, const float* z_ends, int n_ends) {
   c.half = (((int)slices + 1) / 2 + 7) / 8 * 8;
   c.floats = ColDims{g.nx, g.ny, g.nz, c.z0, c.half}.floats();
   return c;
+}
+
+size_t col_list_bytes(const ImgGeom& g) { return col_smem(g.nx, g.ny); }
+
+cudaError_t launch_multi_cols(const MultiStep& m, cudaStream_t st) {
+  if (m.total_lors == 0) return cudaSuccess;
+  k_em_multi_cols<<<(unsigned)m.total_lors, kMultiColBlock, m.col_smem, st>>>(m.cols, m.n_cols,
+                                                                             m.partials + m.total_chunks);
+  return cudaGetLastError();
+}
+
+cudaError_t load_multi_cols() {
+  cudaFuncAttributes a;
+  return cudaFuncGetAttributes(&a, k_em_multi_cols);
 }
 
 int64_t col_partials(const LorTable& t, SubsetSel s) { return lors_of(t, s); }

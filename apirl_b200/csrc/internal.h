@@ -260,24 +260,41 @@ struct MultiSeg {
   int counts_dtype;
   int back;
 };
-// One job's voxel work in a batched step, in 32 x 32 tiles of its slices:
-// before the walk, x into the padded copies and -x . gimg; after it, with
-// `update`, the EM update of x from the padded backprojection pair; the
-// likelihood = the job's chunk partials + its -x . gimg partials - zero_add.
+// The same of a job in the column layout: a subset's (angle, r) LORs (or, for
+// its final likelihood, all of them: subset -1), lor_begin .. of the step;
+// segments are ordered by lor_begin.
+struct MultiCols {
+  ImgGeom g;
+  LorTable t;
+  SubsetSel s;
+  const void* counts;
+  const float* add;
+  ColBuffers cols;
+  int64_t lor_begin;
+  int counts_dtype;
+  int back;
+};
+// One job's voxel work in a batched step, in tiles (32 x 32 of a slice, or a
+// row's 32 x by 32 slices where cols.half): before the walk, x into the
+// copies and -x . gimg; after it, with `update`, the EM update of x from the
+// backprojection sums; the likelihood = the job's walk partials (of its
+// chunks or LORs) + its -x . gimg partials - zero_add.
 struct MultiVox {
   ImgGeom g;
   PadBuffers pad;
+  ColBuffers cols;
   float* x;
   const float* sens;     // the pass's subset sensitivity (update)
   const float* gimg;     // G_s of the pass's subset, or A^T 1 of all subsets (final likelihood)
   double* lik;           // the likelihood's slot
   int64_t tile_begin;    // first tile of the job in the step's tile launches
-  int64_t chunk_begin, n_chunks;  // the job's chunk partials in the walk
+  int64_t part_begin, n_parts;  // the job's partials of the walk
   double zero_add;       // sum over all walked subsets' bins of the additive term
-  int tiles_x, tiles_y;
+  int tiles_x, tiles_y, tiles_z;
   int update, ge;
 };
-// Tiles (blocks of the copy / update launches) of a job: ceil(nx/32) x ceil(ny/32) x nz.
+// Tiles (blocks of the copy / update launches) of a padded job: ceil(nx/32) x
+// ceil(ny/32) x nz.  (A job in the column layout: col_dots.)
 inline int64_t multi_tiles(const ImgGeom& g) {
   return (int64_t)((g.nx + 31) / 32) * ((g.ny + 31) / 32) * g.nz;
 }
@@ -286,12 +303,34 @@ cudaError_t multi_walk_grid(int* blocks);
 // Loads the batch engine's kernels into the context (instead of at their
 // first launch).
 cudaError_t load_batch_kernels();
-// One batched step: copies and dot products, the walk over every segment's
-// list (counter reset here), the likelihood sums, the updates.
-// chunk_partials: >= total_chunks doubles; tile_partials: >= total_tiles.
-cudaError_t launch_multi_step(const MultiVox* d_vox, int n_vox, int64_t total_tiles, const MultiSeg* d_segs,
-                              int n_segs, int64_t total_chunks, int walk_blocks, unsigned long long* counter,
-                              double* chunk_partials, double* tile_partials, cudaStream_t st);
+// A step's work: the walk over n_segs lists (total_chunks chunks) and over
+// n_cols segments of columns (total_lors LORs, col_smem bytes of lists).
+struct MultiStep {
+  const MultiVox* vox;
+  int n_vox;
+  int64_t total_tiles;
+  const MultiSeg* segs;
+  int n_segs;
+  int64_t total_chunks;
+  const MultiCols* cols;
+  int n_cols;
+  int64_t total_lors;
+  size_t col_smem;
+  int walk_blocks;              // multi_walk_grid
+  unsigned long long* counter;  // reset here
+  double* partials;             // total_chunks, then total_lors
+  double* tile_partials;        // total_tiles
+};
+// One batched step: copies and dot products, the walks, the likelihood sums,
+// the updates.  Where it has both kinds of segments the lists are walked on
+// `side` beside the columns (between `fork` and `join`, events of the caller).
+cudaError_t launch_multi_step(const MultiStep& m, cudaStream_t st, cudaStream_t side, cudaEvent_t fork,
+                              cudaEvent_t join);
+// The walk of a step's column segments (columns.cu), a block a LOR.
+cudaError_t launch_multi_cols(const MultiStep& m, cudaStream_t st);
+cudaError_t load_multi_cols();
+// Shared memory of the LOR lists of an image in the column layout.
+size_t col_list_bytes(const ImgGeom& g);
 // List of the bins with counts of subset s (bin numbers of the subset, in bin
 // order), in two launches per subset: count (tiles: ceil(total / kNzTile)
 // ints kept for the write; *n_list) then write.

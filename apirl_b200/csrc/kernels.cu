@@ -19,6 +19,7 @@
 #include <utility>
 #include <vector>
 #include "bins.cuh"
+#include "columns_em.cuh"
 #include "internal.h"
 #include "siddon.cuh"
 #include "../../include/apirl_b200.h"
@@ -1012,24 +1013,6 @@ __global__ void k_fill(int64_t n, float* __restrict__ x, float v) {
 
 // ---------------------------------------------------------------------------
 // Batched work over many independent jobs in one launch.
-__device__ __forceinline__ float load_count_any(const void* p, int dtype, int64_t i) {
-  if (dtype == APIRL_U32) return (float)__ldg((const uint32_t*)p + i);
-  if (dtype == APIRL_U16) return (float)__ldg((const uint16_t*)p + i);
-  return __ldg((const float*)p + i);
-}
-
-// The last of n entries whose first (block, tile or chunk) key(e) is <= k;
-// entries are ordered by key.
-template <typename J, class Key>
-__device__ __forceinline__ int find_entry(const J* __restrict__ e, int n, int64_t k, Key key) {
-  int lo = 0, hi = n - 1;
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (key(e[mid]) <= k) lo = mid; else hi = mid - 1;
-  }
-  return lo;
-}
-
 template <typename J>
 __device__ __forceinline__ int find_job(const J* __restrict__ jobs, int njobs, int64_t blk) {
   return find_entry(jobs, njobs, blk, [](const J& j) { return j.blk_begin; });
@@ -1203,9 +1186,9 @@ __global__ void __launch_bounds__(256) k_pad_reduce(PadDims d, float* __restrict
 }
 
 // ---- batched reconstructions: one step for many jobs ----------------------------
-// Before the walk: every job's image into its padded copies, and the FP64
-// partial -x . gimg of every tile (the likelihood's sum over the bins the
-// walk leaves out).  One block per tile; tiles of a job are consecutive.
+// Before the walk: every job's image into its padded or column copies, and
+// the FP64 partial -x . gimg of every tile (the likelihood's sum over the bins
+// the walk leaves out).  One block per tile; tiles of a job are consecutive.
 __global__ void __launch_bounds__(256) k_multi_copy(const MultiVox* __restrict__ jobs, int njobs,
                                                     double* __restrict__ tile_partials) {
   __shared__ float tile[32][33];
@@ -1214,12 +1197,17 @@ __global__ void __launch_bounds__(256) k_multi_copy(const MultiVox* __restrict__
   __syncthreads();
   const MultiVox& J = jobs[sj];
   const int64_t tl = (int64_t)blockIdx.x - J.tile_begin;
-  const int tx = (int)(tl % J.tiles_x);
+  const int tx = (int)(tl % J.tiles_x), lx = threadIdx.x & 31, ly = threadIdx.x >> 5;
   const int64_t q = tl / J.tiles_x;
   const int ty = (int)(q % J.tiles_y), z = (int)(q / J.tiles_y);
-  const PadDims d{J.g.nx, J.g.ny, J.g.nz};
-  const double dot = pad_copy_tile(d, J.x, J.pad.pA, J.pad.pT, J.gimg, tx * 32, ty * 32, z, threadIdx.x & 31,
-                                   threadIdx.x >> 5, tile);
+  double dot;
+  if (J.cols.half) {
+    const ColDims d{J.g.nx, J.g.ny, J.g.nz, J.cols.z0, J.cols.half};
+    dot = col_copy_tile(d, J.x, J.cols.img, J.gimg, tx * 32, ty, z * 32, lx, ly, tile);
+  } else {
+    const PadDims d{J.g.nx, J.g.ny, J.g.nz};
+    dot = pad_copy_tile(d, J.x, J.pad.pA, J.pad.pT, J.gimg, tx * 32, ty * 32, z, lx, ly, tile);
+  }
   const double sum = block_sum(dot);
   if (threadIdx.x == 0) tile_partials[blockIdx.x] = -sum;
 }
@@ -1268,22 +1256,22 @@ __global__ void __launch_bounds__(kBlock, kMultiMinBlocks) k_em_multi(const Mult
   }
 }
 
-// One block per job: its likelihood, the fixed-order sum of its chunk
-// partials and its tile partials, minus its additive sum.
+// One block per job: its likelihood, the fixed-order sum of its walk partials
+// and its tile partials, minus its additive sum.
 __global__ void __launch_bounds__(256) k_multi_sum(const MultiVox* __restrict__ jobs,
-                                                   const double* __restrict__ chunk_partials,
+                                                   const double* __restrict__ partials,
                                                    const double* __restrict__ tile_partials) {
   const MultiVox& J = jobs[blockIdx.x];
-  const int64_t ntiles = (int64_t)J.tiles_x * J.tiles_y * J.g.nz;
+  const int64_t ntiles = (int64_t)J.tiles_x * J.tiles_y * J.tiles_z;
   double v = 0.0;
-  for (int64_t i = threadIdx.x; i < J.n_chunks; i += blockDim.x) v += chunk_partials[J.chunk_begin + i];
+  for (int64_t i = threadIdx.x; i < J.n_parts; i += blockDim.x) v += partials[J.part_begin + i];
   for (int64_t i = threadIdx.x; i < ntiles; i += blockDim.x) v += tile_partials[J.tile_begin + i];
   const double s = block_sum(v);
   if (threadIdx.x == 0 && J.lik) *J.lik = s - J.zero_add;
 }
 
-// After the walk: the EM update of every job with `update` from its padded
-// backprojection pair (threshold 0, rule ge), the pair cleared.
+// After the walk: the EM update of every job with `update` from its
+// backprojection sums (threshold 0, rule ge), the sums cleared.
 __global__ void __launch_bounds__(256) k_multi_update(const MultiVox* __restrict__ jobs, int njobs) {
   __shared__ float tile[32][33];
   __shared__ int sj;
@@ -1292,12 +1280,16 @@ __global__ void __launch_bounds__(256) k_multi_update(const MultiVox* __restrict
   const MultiVox& J = jobs[sj];
   if (!J.update) return;
   const int64_t tl = (int64_t)blockIdx.x - J.tile_begin;
-  const int tx = (int)(tl % J.tiles_x);
+  const int tx = (int)(tl % J.tiles_x), lx = threadIdx.x & 31, ly = threadIdx.x >> 5;
   const int64_t q = tl / J.tiles_x;
   const int ty = (int)(q % J.tiles_y), z = (int)(q / J.tiles_y);
-  const PadDims d{J.g.nx, J.g.ny, J.g.nz};
-  pad_reduce_tile(d, J.pad.bA, J.pad.bT, 0, J.x, nullptr, J.sens, 0.f, J.ge, tx * 32, ty * 32, z, threadIdx.x & 31,
-                  threadIdx.x >> 5, tile);
+  if (J.cols.half) {
+    const ColDims d{J.g.nx, J.g.ny, J.g.nz, J.cols.z0, J.cols.half};
+    col_reduce_tile(d, J.cols.acc, 0, J.x, nullptr, J.sens, 0.f, J.ge, tx * 32, ty, z * 32, lx, ly, tile);
+  } else {
+    const PadDims d{J.g.nx, J.g.ny, J.g.nz};
+    pad_reduce_tile(d, J.pad.bA, J.pad.bT, 0, J.x, nullptr, J.sens, 0.f, J.ge, tx * 32, ty * 32, z, lx, ly, tile);
+  }
 }
 
 // per_angle[a] += A_a^T 1 (Backproject of ones, SiddonProjector.cpp:444-568)
@@ -1910,7 +1902,7 @@ cudaError_t load_batch_kernels() {
     const cudaError_t e = cudaFuncGetAttributes(&a, f);
     if (e != cudaSuccess) return e;
   }
-  return cudaSuccess;
+  return load_multi_cols();
 }
 
 cudaError_t multi_walk_grid(int* blocks) {
@@ -1924,23 +1916,33 @@ cudaError_t multi_walk_grid(int* blocks) {
   return cudaSuccess;
 }
 
-cudaError_t launch_multi_step(const MultiVox* d_vox, int n_vox, int64_t total_tiles, const MultiSeg* d_segs,
-                              int n_segs, int64_t total_chunks, int walk_blocks, unsigned long long* counter,
-                              double* chunk_partials, double* tile_partials, cudaStream_t st) {
-  if (n_vox == 0 || total_tiles == 0) return cudaSuccess;
+cudaError_t launch_multi_step(const MultiStep& m, cudaStream_t st, cudaStream_t side, cudaEvent_t fork,
+                              cudaEvent_t join) {
+  if (m.n_vox == 0 || m.total_tiles == 0) return cudaSuccess;
   cudaError_t e;
-  k_multi_copy<<<(unsigned)total_tiles, 256, 0, st>>>(d_vox, n_vox, tile_partials);
+  k_multi_copy<<<(unsigned)m.total_tiles, 256, 0, st>>>(m.vox, m.n_vox, m.tile_partials);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  if (total_chunks > 0 && n_segs > 0) {
-    if ((e = cudaMemsetAsync(counter, 0, sizeof(unsigned long long), st)) != cudaSuccess) return e;
-    const int64_t need = (total_chunks * 32 + kBlock - 1) / kBlock;
-    const unsigned grid = (unsigned)(need < walk_blocks ? need : walk_blocks);
-    k_em_multi<<<grid, kBlock, 0, st>>>(d_segs, n_segs, total_chunks, counter, chunk_partials);
+  const bool lists = m.total_chunks > 0, both = lists && m.total_lors > 0;
+  if (both) {
+    if ((e = cudaEventRecord(fork, st)) != cudaSuccess) return e;
+    if ((e = cudaStreamWaitEvent(side, fork, 0)) != cudaSuccess) return e;
+  }
+  if (lists) {
+    cudaStream_t ls = both ? side : st;
+    if ((e = cudaMemsetAsync(m.counter, 0, sizeof(unsigned long long), ls)) != cudaSuccess) return e;
+    const int64_t need = (m.total_chunks * 32 + kBlock - 1) / kBlock;
+    const unsigned grid = (unsigned)(need < m.walk_blocks ? need : m.walk_blocks);
+    k_em_multi<<<grid, kBlock, 0, ls>>>(m.segs, m.n_segs, m.total_chunks, m.counter, m.partials);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
   }
-  k_multi_sum<<<n_vox, 256, 0, st>>>(d_vox, chunk_partials, tile_partials);
+  if ((e = launch_multi_cols(m, st)) != cudaSuccess) return e;
+  if (both) {
+    if ((e = cudaEventRecord(join, side)) != cudaSuccess) return e;
+    if ((e = cudaStreamWaitEvent(st, join, 0)) != cudaSuccess) return e;
+  }
+  k_multi_sum<<<m.n_vox, 256, 0, st>>>(m.vox, m.partials, m.tile_partials);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  k_multi_update<<<(unsigned)total_tiles, 256, 0, st>>>(d_vox, n_vox);
+  k_multi_update<<<(unsigned)m.total_tiles, 256, 0, st>>>(m.vox, m.n_vox);
   return cudaGetLastError();
 }
 

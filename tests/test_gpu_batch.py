@@ -225,3 +225,42 @@ def test_sensitivity_images_returned_as_asked(small_jobs):
     assert s0.shape == sall[0].shape and s0.any()
     assert rel(s0, sall[0]) <= 1e-6
     assert rel(img1, img2) <= 1e-6 and np.allclose(lik1, lik2, rtol=1e-7)
+
+
+@pytest.mark.parametrize("rings,max_rd", [(16, 0), (15, 0), (9, 4), (21, 20)])
+def test_batch_column_walk(rings, max_rd):
+    """Jobs whose walk is a block per (angle, r) over 16 and more sinograms,
+    one count type each, with factors, an additive term and an initial image
+    (and 15 sinograms, which keep the lists of bins): each equals its solo run,
+    beside a single-slice job whose list is walked in the same steps.  A
+    width that is no multiple of a tile's 32."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    ig = ap.ImageGeom(41, 41, 2 * rings - 1, 2.08, 2.08, 2.03)
+    sg = ap.Sino3DGeom.span1(54, 53, rings, 53 * 2.08 / 2, rings * 4.06, 443.0, max_rd)
+    rng = np.random.default_rng(rings)
+    x = workloads.random_phantom(ig, rng)
+    P = ap.SiddonProjector(ig, sg)
+    est = torch.empty(P.num_bins(), dtype=torch.float32, device=DEV)
+    P.project(torch.from_numpy(x).to(DEV), est)
+    est = est.cpu().numpy()
+    P.close()
+    jobs = []
+    for k, dt in enumerate((np.uint16, np.uint32, np.float32)):
+        counts = workloads.poisson_counts(est, 0.2 * est.size if k else 5.0 * est.size, seed=k).astype(dt)
+        mult = (rng.random(est.size, dtype=np.float32) * 0.5 + 0.5) if k == 1 else None
+        add = (rng.random(est.size, dtype=np.float32) * 0.1) if k == 2 else None
+        init = (rng.random(ig.n_voxels, dtype=np.float32) + 0.5) if k == 2 else None
+        jobs.append(Job(ig, sg, counts, 2, 4, mult=mult, add=add, init=init, tag=dt))
+    jobs += make_jobs([dict(n=32, z=1, seed=5, counts=1e5, iters=2, nsubsets=4)])
+    b = Batch(0, budget_bytes=8 << 30)
+    res = b.run_all(jobs)
+    b.close()
+    for j, (img, lik) in zip(jobs, res):
+        init = np.ones(j.image_geom.n_voxels, np.float32) if j.init is None else j.init
+        solo, solo_lik, _ = ap.osem_3d(j.image_geom, j.sino_geom, j.counts.astype(np.float32), init, j.iters,
+                                       j.nsubsets, mult=j.mult, add=j.add)
+        finite = np.isfinite(solo)
+        assert np.array_equal(np.isfinite(img), finite), j.tag
+        assert rel(img[finite], solo[finite]) <= 1e-4, j.tag
+        assert np.allclose(lik[:-1], solo_lik[:-1], rtol=1e-6), j.tag
