@@ -111,6 +111,13 @@ bool use_cols(const apirl_projector* p) {
          p->t.n_sinos >= apirl::kColMinSinos;
 }
 
+// The fused passes with several rays a bin: on their own column layout where
+// set_sampling made it, from the sinograms on that pay in the plain passes.
+bool use_ray_cols(const apirl_projector* p) {
+  return p->t.lor_s && p->dual_layout && !p->pg.enabled && p->ray_cols.half && p->pad.acc == APIRL_ACC_ATOMIC &&
+         p->t.n_sinos >= apirl::kColMinSinos;
+}
+
 // A slot for work queued on s until slot_done, which the lock covers: the one
 // s used last, else the one unused the longest; s waits for its last use.
 // (No event is queried: a query in one thread breaks a global-mode capture in
@@ -270,6 +277,24 @@ apirl_status alloc_cols(apirl_projector* p) {
     CK(cudaEventCreateWithFlags(&p->col_img[k].done, cudaEventDisableTiming));
   }
   return APIRL_OK;
+}
+
+// The column layout of a sampled table, whose end points lie up to half a ring
+// beyond the rings': image copy and the two sums.  Without room for it the
+// passes walk bin by bin.
+void alloc_ray_cols(apirl_projector* p, const apirl::RayTables& rt) {
+  if (p->host.n_sinos < apirl::kColMinSinos || !apirl::col_rays_fit(p->g, rt.n_rs)) return;
+  apirl::ColBuffers c = apirl::col_layout(p->g, rt.zs.data(), (int)rt.zs.size());
+  if (!c.half) return;
+  const size_t bytes = 3 * (size_t)c.floats * sizeof(float);
+  cudaError_t e = cudaMalloc(&c.img, bytes);
+  if (e == cudaSuccess && (e = cudaMemset(c.img, 0, bytes)) != cudaSuccess) cudaFree(c.img);
+  if (e != cudaSuccess) {
+    (void)cudaGetLastError();  // handled here
+    return;
+  }
+  c.acc = c.img + c.floats;
+  p->ray_cols = c;
 }
 
 apirl_status finish_create(apirl_projector* p, apirl_projector** out) {
@@ -485,6 +510,7 @@ void apirl_projector_destroy(apirl_projector* p) {
     cudaFree(p->d_zoff[k]);
   }
   cudaFree(p->cols.img);  // the block of all column buffers
+  cudaFree(p->ray_cols.img);
   cudaFree(p->queue.n);
   cudaFree(p->planar.img);
   for (auto& c : p->col_img)
@@ -574,6 +600,8 @@ apirl_status apirl_projector_set_sampling(apirl_projector* p, int n_samples, int
     p->d_zs[k] = nullptr;
     p->d_zoff[k] = nullptr;
   }
+  cudaFree(p->ray_cols.img);
+  p->ray_cols = apirl::ColBuffers();
   p->t.lor_s = nullptr; p->t.zs = nullptr; p->t.zoff = nullptr; p->t.n_rs = 1; p->t.n_as = 1;
   p->t_dab = p->t;
   p->n_samples = 1; p->n_axial_samples = 1; p->multi_lors = 0;
@@ -585,6 +613,7 @@ apirl_status apirl_projector_set_sampling(apirl_projector* p, int n_samples, int
                               (int)p->min_rd.size(), p->min_rd.data(), p->max_rd.data(), n_samples, n_axial_samples,
                               multiple_lors_per_bin != 0, k == 1, rt))
       return fail(APIRL_ERR_INVALID, "a sampled ray end point is not finite (sample outside the scanner radius)");
+    if (k == 0) alloc_ray_cols(p, rt);
     if ((int)rt.zoff.size() != p->t.n_sinos + 1) return fail(APIRL_ERR_INVALID, "ring-pair table mismatch");
     CK(cudaMalloc(&p->d_lor_s[k], rt.lor.size() * sizeof(float)));
     CK(cudaMemcpy(p->d_lor_s[k], rt.lor.data(), rt.lor.size() * sizeof(float), cudaMemcpyHostToDevice));
@@ -765,7 +794,8 @@ namespace {
 // The padded pass on the column layout.  It has one launch form: the options
 // of the padded pair's launch (persistent, block size, gather segments) do not
 // change it, an ordered list keeps to the pair.
-bool pass_cols(const apirl_projector* p) { return use_cols(p) && !p->nz.order; }
+bool pass_cols(const apirl_projector* p) { return (use_cols(p) && !p->nz.order) || use_ray_cols(p); }
+const apirl::ColBuffers& pass_layout(const apirl_projector* p) { return p->t.lor_s ? p->ray_cols : p->cols; }
 
 // Before the padded pass: the image into its copy.  After it: the update of x
 // (mode 0), or bp += the backprojection (mode 1).  On the column layout they
@@ -773,7 +803,7 @@ bool pass_cols(const apirl_projector* p) { return use_cols(p) && !p->nz.order; }
 apirl_status pass_begin(apirl_projector* p, SubsetSel ss, const float* d_x, const float* d_zimg, double* d_lik,
                         cudaStream_t s) {
   if (pass_cols(p))
-    CK(apirl::launch_col_copy(p->g, p->cols, d_x, p->cols.img, s, d_lik ? d_zimg : nullptr,
+    CK(apirl::launch_col_copy(p->g, pass_layout(p), d_x, pass_layout(p).img, s, d_lik ? d_zimg : nullptr,
                               p->d_partials + apirl::col_partials(p->t, ss), d_zimg ? p->queue.n : nullptr));
   else
     CK(apirl::launch_pad_copy(p->g, d_x, p->pad, s));
@@ -785,7 +815,7 @@ apirl_status pass_end(apirl_projector* p, SubsetSel ss, int mode, float* d_x, fl
   if (pass_cols(p)) {
     const int64_t lors = (int64_t)ss.nk * p->t.n_r;  // no LORs: no partials written
     const int64_t n = lors ? apirl::col_partials(p->t, ss) + (d_zimg ? apirl::col_dots(p->g) : 0) : 0;
-    CK(apirl::launch_col_reduce(p->g, p->cols, p->cols.acc, mode, d_x, d_bp, d_sens, d_thr, thr_value, ge, s,
+    CK(apirl::launch_col_reduce(p->g, pass_layout(p), pass_layout(p).acc, mode, d_x, d_bp, d_sens, d_thr, thr_value, ge, s,
                                 p->d_partials, n, d_zimg ? d_zero_add : nullptr, lors ? d_lik : nullptr));
   } else {
     CK(apirl::launch_pad_reduce(p->g, p->pad, mode, d_x, d_bp, d_sens, d_thr, thr_value, ge, s));
@@ -806,7 +836,9 @@ apirl_status fused(apirl_projector* p, SubsetSel ss, const void* d_counts, int d
     }
     CK(cudaEventRecord(p->ev0, s));
   }
-  if (dual && pass_cols(p)) {
+  if (dual && p->t.lor_s) {
+    CK(apirl::launch_em_cols_rays(p->g, p->ray_cols, p->t, ss, d_counts, dtype, packed, d_add, 1, p->d_partials, s));
+  } else if (dual && pass_cols(p)) {
     CK(apirl::launch_em_cols(p->g, p->cols, p->t, ss, d_counts, dtype, packed, d_add, 1, p->d_partials,
                              d_zimg ? (p->sparse_image ? 2 : 1) : 0, p->queue, s));
   } else if (p->planar.lim) {
@@ -845,7 +877,7 @@ apirl_status apirl_em_pass(apirl_projector* p, const void* d_counts, int counts_
   cudaStream_t s = (cudaStream_t)stream;
   SubsetSel ss = make_subset(p, subset, nsubsets);
   const int64_t nv = (int64_t)p->g.nx * p->g.ny * p->g.nz;
-  if (use_dual(p)) {
+  if (use_dual(p) || use_ray_cols(p)) {
     if ((st = pass_begin(p, ss, d_x, nullptr, d_lik, s))) return st;
     st = fused(p, ss, d_counts, counts_dtype, counts_packed, d_add, d_x, d_bp, true, d_lik, s);
     if (st) return st;
@@ -944,7 +976,7 @@ apirl_status apirl_em_project_backproject(apirl_projector* p, const void* d_coun
   DEVICE_SCOPE(p->device);
   cudaStream_t s = (cudaStream_t)stream;
   SubsetSel ss = make_subset(p, subset, nsubsets);
-  if (use_dual(p)) {
+  if (use_dual(p) || use_ray_cols(p)) {
     if ((st = pass_begin(p, ss, d_x, nullptr, d_lik, s))) return st;
     st = fused(p, ss, d_counts, counts_dtype, counts_packed, d_add, d_x, d_bp, true, d_lik, s);
     if (st) return st;

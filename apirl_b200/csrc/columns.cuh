@@ -65,21 +65,22 @@ struct ColWalk {
 // an[j - 1], the columns (int bits) and the crossing parameters an[j].  One
 // address register reads a whole record.  Behind them lie the x and y chains
 // that the list is merged from, and in their place then (an[j], column) step
-// by step.
+// by step.  A block may keep several lists: `at`, here and below, is the first
+// float4 of one.
 extern __shared__ __align__(16) float4 col_smem4[];
 constexpr int kColHead = (sizeof(ColWalk) + 15) / 16;  // float4s before the list
 // Steps a list can need on this image (guarded walks: at most nx + 2 and
 // ny + 2 crossings, two spare entries a chain), in whole records.
 __host__ __device__ inline int col_cap(int nx, int ny) { return (nx + ny + 8 + kColBatch - 1) / kColBatch * kColBatch; }
 __host__ __device__ inline size_t col_smem(int nx, int ny) {
-  return (size_t)kColHead * 16 + (size_t)col_cap(nx, ny) * 20;
+  return (size_t)kColHead * 16 + (size_t)col_cap(nx, ny) * 20;  // whole float4s
 }
-__device__ __forceinline__ ColWalk& col_head() { return *reinterpret_cast<ColWalk*>(col_smem4); }
+__device__ __forceinline__ ColWalk& col_head(int at = 0) { return *reinterpret_cast<ColWalk*>(col_smem4 + at); }
 // Float offset of what lies behind the records.
 __device__ __forceinline__ int col_behind(const ColDims& d) { return kColHead * 4 + col_cap(d.nx, d.ny) * 3; }
 // Step j's field f (0 length, 1 column, 2 crossing parameter).
-__device__ __forceinline__ float& col_field(int j, int f) {
-  return reinterpret_cast<float*>(col_smem4)[kColHead * 4 + (j >> 2) * 12 + f * 4 + (j & 3)];
+__device__ __forceinline__ float& col_field(int j, int f, int at) {
+  return reinterpret_cast<float*>(col_smem4 + at)[kColHead * 4 + (j >> 2) * 12 + f * 4 + (j & 3)];
 }
 
 __device__ __forceinline__ void col_setup_xy(const float4 P, const ImgGeom& g, const ColDims& d, ColWalk& w) {
@@ -130,10 +131,10 @@ __device__ __forceinline__ void col_setup_xy(const float4 P, const ImgGeom& g, c
 // on return.  The crossing parameters are the reference's running sums: two
 // threads add the x and the y chain up, then every thread places entries at
 // their rank among both (x before y on ties, Siddon.cpp:317-339).
-__device__ __forceinline__ void col_list(const float4 P, const ImgGeom& g, const ColDims& d) {
+__device__ __forceinline__ void col_list(const float4 P, const ImgGeom& g, const ColDims& d, int at = 0) {
   const int tid = threadIdx.x;
-  ColWalk& h = col_head();
-  float* const chain = reinterpret_cast<float*>(col_smem4) + col_behind(d);
+  ColWalk& h = col_head(at);
+  float* const chain = reinterpret_cast<float*>(col_smem4 + at) + col_behind(d);
   if (tid < 32) {
     ColWalk w;
     col_setup_xy(P, g, d, w);
@@ -168,8 +169,8 @@ __device__ __forceinline__ void col_list(const float4 P, const ImgGeom& g, const
       }
       const int p = i + lo;
       if (p < n) {
-        col_field(p, 2) = v;
-        col_field(p, 1) = __int_as_float((int)min((unsigned)(col + (isx ? i * sx + lo * sy : lo * sx + i * sy)), last));
+        col_field(p, 2, at) = v;
+        col_field(p, 1, at) = __int_as_float((int)min((unsigned)(col + (isx ? i * sx + lo * sy : lo * sx + i * sy)), last));
         // The chain's last spare entry taken: the chain may be too short.
         if (i == (isx ? nx : ny) - 1) h.listed = 0;
       }
@@ -177,11 +178,11 @@ __device__ __forceinline__ void col_list(const float4 P, const ImgGeom& g, const
   }
   __syncthreads();
   if (listed) {
-    float2* const by_step = reinterpret_cast<float2*>(reinterpret_cast<float*>(col_smem4) + col_behind(d));
+    float2* const by_step = reinterpret_cast<float2*>(reinterpret_cast<float*>(col_smem4 + at) + col_behind(d));
     for (int p = tid; p < h.n; p += blockDim.x) {
-      const float an = col_field(p, 2);
-      col_field(p, 0) = A_SUB(an, p ? col_field(p - 1, 2) : h.amin);
-      by_step[p] = make_float2(an, col_field(p, 1));
+      const float an = col_field(p, 2, at);
+      col_field(p, 0, at) = A_SUB(an, p ? col_field(p - 1, 2, at) : h.amin);
+      by_step[p] = make_float2(an, col_field(p, 1, at));
     }
   }
   __syncthreads();
@@ -226,8 +227,8 @@ __device__ __forceinline__ WalkZ col_setup_z(const float2 e, const ColWalk& w, c
 // Warps with a ray whose z crossings lie so close that a batch could hold two
 // merge z crossings and list segment by segment, each lane at its own step.
 template <class T, class V>
-__device__ __forceinline__ void col_walk(WalkZ r, const ColDims& d, T* base, V&& visit) {
-  const int n = col_head().n;
+__device__ __forceinline__ void col_walk(WalkZ r, const ColDims& d, T* base, V&& visit, int list_at = 0) {
+  const int n = col_head(list_at).n;
   T* p = base + r.at;
   // One z crossing of the lane's ray, from lo, in the column at `col`.
   auto cross = [&](int col, float& lo) {
@@ -239,15 +240,15 @@ __device__ __forceinline__ void col_walk(WalkZ r, const ColDims& d, T* base, V&&
     r.az = A_ADD(r.az, r.azu);
     r.rem--;
   };
-  float before = col_head().amin;  // the crossing before the batch
+  float before = col_head(list_at).amin;  // the crossing before the batch
   // rem >= -kPad: up to the list's last kPad steps no walk has recorded all
   // its crossings, so only the steps after this loop ask.
   const int batches = (n - kPad) / kColBatch;
   // Four steps span at most four gaps of the denser of the x and y crossings:
   // where every lane's z crossings lie further apart, a batch holds one at most.
-  const bool single = !__any_sync(0xffffffffu, r.azu != 0.f && r.azu < 4.01f * fminf(col_head().axu, col_head().ayu));
+  const bool single = !__any_sync(0xffffffffu, r.azu != 0.f && r.azu < 4.01f * fminf(col_head(list_at).axu, col_head(list_at).ayu));
   if (!single && batches > 0) {
-    const float2* const list = reinterpret_cast<const float2*>(reinterpret_cast<float*>(col_smem4) + col_behind(d));
+    const float2* const list = reinterpret_cast<const float2*>(reinterpret_cast<float*>(col_smem4 + list_at) + col_behind(d));
     const float2* at = list;
     const float2* const stop = list + batches * kColBatch;
     float2 next = *at;
@@ -278,7 +279,7 @@ __device__ __forceinline__ void col_walk(WalkZ r, const ColDims& d, T* base, V&&
     p = base + r.at;
     before = list[batches * kColBatch - 1].x;
   }
-  unsigned rec = (unsigned)__cvta_generic_to_shared(col_smem4 + kColHead);
+  unsigned rec = (unsigned)__cvta_generic_to_shared(col_smem4 + list_at + kColHead);
   const unsigned stop = rec + (single ? max(batches, 0) * 48u : 0u);
   #pragma unroll 1
   for (; rec != stop; rec += 48) {
@@ -314,8 +315,8 @@ __device__ __forceinline__ void col_walk(WalkZ r, const ColDims& d, T* base, V&&
   }
   #pragma unroll 1
   for (int j = max(batches, 0) * kColBatch; j < n; j++) {
-    const float an = col_field(j, 2);
-    const int col = __float_as_int(col_field(j, 1)), left = n - j;
+    const float an = col_field(j, 2, list_at);
+    const int col = __float_as_int(col_field(j, 1, list_at)), left = n - j;
     float lo = before;
     while (r.az < an && r.rem + left > 0 && r.rem > -kPad) cross(col, lo);
     if (r.rem + left > 0) visit(p + col, A_MUL(A_SUB(an, lo), r.len));
@@ -324,7 +325,7 @@ __device__ __forceinline__ void col_walk(WalkZ r, const ColDims& d, T* base, V&&
   // z crossings still to record after the list, with the x and y ones that
   // come before them: the x/y chains are added up again to the list's end.
   if (r.rem > 0) {
-    const ColWalk& h = col_head();
+    const ColWalk& h = col_head(list_at);
     float ax = h.ax, ay = h.ay, lo = h.amin;
     int col = h.col;
     auto next_xy = [&]() {

@@ -183,6 +183,12 @@ cudaError_t launch_scatter_cols(const ImgGeom& g, const ColBuffers& c, const Lor
 cudaError_t launch_em_cols(const ImgGeom& g, const ColBuffers& c, const LorTable& t, SubsetSel s, const void* counts,
                            int counts_dtype, int counts_packed, const float* add, int back, double* partials,
                            int skip_zero, const ColQueue& queue, cudaStream_t st);
+// The full fused kernel of a sampled table (several rays a bin), one partial
+// per col_partials; for n_rs whose lists fit a block's shared memory.
+bool col_rays_fit(const ImgGeom& g, int n_rs);
+cudaError_t launch_em_cols_rays(const ImgGeom& g, const ColBuffers& c, const LorTable& t, SubsetSel s,
+                                const void* counts, int counts_dtype, int counts_packed, const float* add, int back,
+                                double* partials, cudaStream_t st);
 // Bins per tile of the list building (one block each).
 constexpr int kNzTile = 2048;
 // Room for the list of a subset's bins with counts (sparse passes of the
@@ -406,6 +412,7 @@ struct apirl_projector {
   // The column layout (half = 0: none): the fused pass's and the
   // backprojections' image copy and sums, used by one stream at a time.
   apirl::ColBuffers cols;
+  apirl::ColBuffers ray_cols;    // of the passes with several rays a bin (apirl_projector_set_sampling)
   apirl::PlanarBuffers planar;   // 2D
   apirl::ColQueue queue;         // LORs with few counts of a listed pass
   // Column images and sums of the calls that keep no other state in the

@@ -184,7 +184,10 @@ apirl_status apirl_projector_set_shard(apirl_projector* p, int first_sinogram, i
  *   block walks one (angle, r) for all sinograms (7 more images); sensitivities
  *   and geometry images, and passes with an option that speaks of the padded
  *   layouts (L2 window, list order, another accumulation form than plain
- *   atomics), keep to the two.  The launch options below (block size,
+ *   atomics), keep to the two.  Passes with several rays a bin take a column
+ *   layout too (3 more images) where the radial samples are few (their
+ *   crossing lists fit a block's shared memory: 40 KB, 20 (nx + ny + 11) bytes
+ *   a sample); their projections and backprojections walk bin by bin.  The launch options below (block size,
  *   persistent, gather segments) shape the two layouts' kernel; the column
  *   layout's has one shape and takes any setting.
  * APIRL_OPT_KERNEL_TIMING (default 0): record CUDA events around the fused

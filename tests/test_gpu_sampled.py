@@ -172,3 +172,39 @@ def test_sampling_reset_and_validation(oracle):
     P2.set_alpha_precision(True)
     with pytest.raises(ap.ApirlError):
         P2.set_sampling(2, 1, 0)
+
+
+@pytest.mark.parametrize("ns,nas,multi,shard,span", [
+    (2, 2, 1, (0, 23), 1), (3, 1, 0, (3, 16), 1), (3, 1, 0, (3, 15), 1), (2, 1, 1, (0, 9), 3), (20, 1, 0, (0, 23), 1)])
+def test_sampled_pass_layouts(ns, nas, multi, shard, span):
+    """The pass with several rays a bin on the column layout (16 and more
+    sinograms of a shard, crossing lists of the radial samples within a
+    block's shared memory) against the bin by bin walk of the plain layout,
+    which the others keep: the same rays in the same order, so equal estimates
+    and likelihood terms (their FP64 sum to 1e-12), backprojections up to the
+    order of fp32 additions (1e-5).  em_project_backproject adds to what bp
+    holds."""
+    ig, sg = geometry(span)
+    rng = np.random.default_rng(ns + nas + multi + shard[1])
+    x0 = (rng.random(ig.n_voxels, dtype=np.float32) + 0.5).astype(np.float32)
+    m = rng.poisson(2.0, sg.n_bins).astype(np.uint16)
+    add = rng.random(sg.n_bins, dtype=np.float32)
+    sens = (rng.random(ig.n_voxels, dtype=np.float32) + 1).astype(np.float32)
+    got = []
+    for dual in (1, 0):
+        P = ap.SiddonProjector(ig, sg)
+        P.set_option(_lib.APIRL_OPT_DUAL_LAYOUT, dual)
+        P.set_sampling(ns, nas, multi)
+        P.set_shard(*shard)
+        for sub, nsub in ((-1, 1), (3, 7)):
+            x, bp = t(x0), torch.zeros(ig.n_voxels, dtype=torch.float32, device=DEV)
+            lik = torch.zeros(2, dtype=torch.float64, device=DEV)
+            P.em_pass(t(m), x, bp, t(sens), sub, nsub, add=t(add), lik=lik[:1])
+            assert float(bp.abs().max()) == 0.0
+            bp.fill_(0.25)
+            P.em_project_backproject(t(m), t(x0), bp, sub, nsub, add=t(add), lik=lik[1:])
+            got.append([a.cpu().numpy() for a in (x, bp, lik)])
+        P.close()
+    for new, old in zip(got[:2], got[2:]):
+        assert rel(new[0], old[0]) <= 1e-5 and rel(new[1], old[1]) <= 1e-5
+        assert np.all(np.abs(new[2] - old[2]) <= 1e-12 * np.abs(old[2]))
