@@ -150,7 +150,7 @@ __global__ void __launch_bounds__(kColBlock, kColBlocks) k_em_cols(
 // pair, radial sample, axial sample; one running sum): a block keeps one list
 // a radial sample, its lanes take their sinograms' ring pairs in step.  Bound
 // by latency on small images, whose LORs are few: a 64 x 64 x 21 job's subset
-// of 8 with 3 x 2 rays a bin (862 LORs, 91 sinograms) 246 us bin by bin, 146 us
+// of 8 with 3 x 2 rays a bin (862 LORs, 91 sinograms) 246 us bin by bin, 102 us
 // here.
 template <typename CT>
 __global__ void __launch_bounds__(kColBlock, kColBlocks) k_em_cols_rays(

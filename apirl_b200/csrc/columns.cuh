@@ -412,6 +412,7 @@ __device__ __noinline__ void col_walk_checked(const float4 P, const float2 e, co
                                               T* base, V& visit) {
   Walk3 w;
   siddon3_setup(P.x, P.y, e.x, A_SUB(P.z, P.x), A_SUB(P.w, P.y), A_SUB(e.y, e.x), g, w);
+  if (walk_misses(w, g)) return;
   for (int m = 0; m < w.n; m++) {
     bool cx, cy;
     const float an = next_crossing(w, cx, cy);

@@ -81,7 +81,52 @@ __device__ __forceinline__ void siddon3_setup(float p0x, float p0y, float p0z, f
   w.i = imin; w.j = jmin; w.k = kmin;
 }
 
-// Visits the n recorded segments in order: visit(inb, linear_index, length).
+// Whether a walk from cell (i, j) in the plane never enters the image, nx x ny.
+// A ray past a corner of the image starts its walk at the scanner's ring
+// (Siddon.cpp:108-140 clip its entry parameter to [0, 1]) and runs up to twice
+// the ring's radius without a voxel to record.  Such a walk reaches the
+// image's x range at one of its x crossings and leaves it at a later one, y
+// alike: it misses the image where it has left one range before it reaches the
+// other.  The running sums' crossing parameters are taken as first + k *
+// increment; their rounding stays below k 2^-24 of the largest, and 2^-20
+// separates a miss (a doubtful ray is walked, with the same result).  5 % of
+// the rays of a job with 1.3 bins a voxel miss, with up to 280 steps of the
+// bounds-tested walk, the last of a launch: skipping them, the column passes of
+// a 100 x 100 x 41 job 728 -> 693 us, of a 64 x 64 x 21 job with 6 rays a bin
+// 146 -> 102.  (The 2D walk, siddon2_walk, gained nothing and keeps walking.)
+struct AxisSpan {
+  float in, out, doubt_in, doubt_out;
+};
+__device__ __forceinline__ bool axis_span(int i, int inc, int n, float a, float au, AxisSpan& s) {
+  const int to = inc > 0 ? -i : i - (n - 1), past = to + n;  // crossings to the range, and past it
+  s.in = -FLT_MAX;
+  s.out = FLT_MAX;
+  s.doubt_in = s.doubt_out = 0.f;
+  if (inc == 0) return (unsigned)i < (unsigned)n;
+  if (past <= 0) return false;
+  const float rel = 9.5367431640625e-7f;
+  if (to > 0) {
+    s.in = a + (float)(to - 1) * au;
+    s.doubt_in = rel * (float)(to + 4) * fmaxf(fabsf(a), fabsf(s.in));
+  }
+  s.out = a + (float)(past - 1) * au;
+  s.doubt_out = rel * (float)(past + 4) * fmaxf(fabsf(a), fabsf(s.out));
+  return true;
+}
+__device__ __forceinline__ bool walk_misses(int i, int j, int iinc, int jinc, float ax, float ay, float axu, float ayu,
+                                            int nx, int ny) {
+  if (((unsigned)(i + 1) <= (unsigned)(nx + 1)) & ((unsigned)(j + 1) <= (unsigned)(ny + 1))) return false;
+  AxisSpan x, y;
+  if (!axis_span(i, iinc, nx, ax, axu, x) || !axis_span(j, jinc, ny, ay, ayu, y)) return true;
+  return x.in - y.out > x.doubt_in + y.doubt_out || y.in - x.out > y.doubt_in + x.doubt_out;
+}
+template <class W>
+__device__ __forceinline__ bool walk_misses(const W& w, const ImgGeom& g) {
+  return walk_misses(w.i, w.j, w.iinc, w.jinc, w.ax, w.ay, w.axu, w.ayu, g.nx, g.ny);
+}
+
+// Visits the n recorded segments in order: visit(inb, linear_index, length);
+// none of a walk that misses the image.
 // `inb` is the full six-sided bounds test; linear_index = (k*ny + j)*nx + i is
 // only meaningful when inb is true.  Record-then-advance as in Siddon.cpp:310-340.
 template <class V>
@@ -186,6 +231,7 @@ __device__ __forceinline__ float siddon3_gather_pad(Walk3 w, const ImgGeom& g, i
     }
     return acc;
   }
+  if (walk_misses(w, g)) return acc;
   for (int m = 0; m < w.n; m++) {
     bool cx, cy;
     const float an = next_crossing(w, cx, cy);
@@ -282,6 +328,7 @@ __device__ __forceinline__ void siddon3_scatter_pad(Walk3 w, const ImgGeom& g, i
     }
     return;
   }
+  if (walk_misses(w, g)) return;
   for (int m = 0; m < w.n; m++) {
     bool cx, cy;
     const float an = next_crossing(w, cx, cy);
@@ -307,7 +354,7 @@ __device__ __forceinline__ void siddon3_scatter_pad_warp(Walk3 w, const ImgGeom&
                                                          unsigned lim, float r, float* __restrict__ img, bool live) {
   __shared__ float slot[256];
   const int lane = (int)(threadIdx.x & 31), warp0 = (int)threadIdx.x - lane;
-  const int n = live ? w.n : 0;
+  const int n = live && (w.guarded || !walk_misses(w, g)) ? w.n : 0;
   const int nmax = __reduce_max_sync(0xffffffffu, n);
   const int sx = w.iinc * ux, sy = w.jinc * uy, sz = w.kinc * uz;
   int idx = live ? (w.k + kPad) * uz + (w.j + kPad) * uy + (w.i + kPad) * ux : 0;
@@ -351,6 +398,7 @@ __device__ __forceinline__ void siddon3_scatter2_pad(Walk3 w, const ImgGeom& g, 
   const int sx = w.iinc * ux, sy = w.jinc * uy, sz = w.kinc * uz;
   int idx = (w.k + kPad) * uz + (w.j + kPad) * uy + (w.i + kPad) * ux;
   const bool first = r1 != 0.f;
+  if (!w.guarded && walk_misses(w, g)) return;
   for (int m = 0; m < w.n; m++) {
     bool cx, cy;
     const float an = next_crossing(w, cx, cy);
@@ -371,6 +419,7 @@ __device__ __forceinline__ void siddon3_scatter2_pad(Walk3 w, const ImgGeom& g, 
 
 template <class V>
 __device__ __forceinline__ void siddon3_walk(Walk3 w, const ImgGeom& g, V&& visit) {
+  if (walk_misses(w, g)) return;
   const int sx = w.iinc, sy = w.jinc * g.nx, sz = w.kinc * g.nx * g.ny;
   int idx = (w.k * g.ny + w.j) * g.nx + w.i;
   for (int m = 0; m < w.n; m++) {

@@ -165,3 +165,29 @@ def test_project_on_streams_and_in_a_graph(oracle):
     g.replay()
     torch.cuda.synchronize()
     assert bits_equal(out.cpu().numpy(), want[0])
+
+
+@pytest.mark.parametrize("rings,max_rd", [(1, 0), (15, 0), (17, 0), (5, 2)])
+@pytest.mark.parametrize("ring", [70.0, 200.0])
+def test_rays_past_the_image(oracle, rings, max_rd, ring):
+    """Half of the radial bins past the image's corners and sides, angles along
+    the axes and diagonals among them, from a near and a far ring: rays that
+    miss the image record nothing, whichever walk serves them (one sinogram and
+    15: bin by bin; 17 and 19: columns), and those that just touch it all their
+    segments."""
+    ig = ImageGeom(33, 33, 5, 2.0, 2.0, 4.0)
+    sg = Sino3DGeom.span1(16, 131, rings, 66.0, rings * 4.0, ring, max_rd)
+    rng = np.random.default_rng(rings)
+    x0 = (rng.random(ig.n_voxels, dtype=np.float32) + 0.5).astype(np.float32)
+    P = ap.SiddonProjector(ig, sg)
+    est = oracle.project_3d(sg, ig, x0)
+    assert (est.reshape(-1, 131)[:, [0, -1]] == 0).all()
+    assert bits_equal(P.project(t(x0), zeros(est.size)).cpu().numpy(), est)
+    v = rng.random(est.size, dtype=np.float32)
+    want = oracle.backproject_3d(sg, ig, v, threads=1)
+    assert rel(P.backproject(t(v), zeros(ig.n_voxels)).cpu().numpy(), want) <= 1e-5
+    m = rng.poisson(3.0, est.size).astype(np.uint16)
+    add = (rng.random(est.size, dtype=np.float32) + 0.5).astype(np.float32)
+    bp = P.em_project_backproject(t(m), t(x0), zeros(ig.n_voxels), add=t(add))
+    want = oracle.backproject_3d(sg, ig, oracle.inverse_divide(m.astype(np.float32), est + add), threads=1)
+    assert rel(bp.cpu().numpy(), want) <= 1e-5
