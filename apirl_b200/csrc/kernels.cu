@@ -68,14 +68,11 @@ constexpr int kEmMinBlocks = APIRL_EM_MIN_BLOCKS;
 #endif
 
 // Forward projection of one bin (3D), masked gather of the image.
+template <bool SELECT = true>
 __device__ __forceinline__ float ray_sum3(const ImgGeom& g, const float4 L, const float2 z, const float* __restrict__ img,
                                           Walk3& w) {
   siddon3_setup(L.x, L.y, z.x, A_SUB(L.z, L.x), A_SUB(L.w, L.y), A_SUB(z.y, z.x), g, w);
-  float acc = 0.f;
-  siddon3_walk(w, g, [&](bool inb, int idx, float seg) {
-    if (inb) acc = A_ADD(acc, A_MUL(seg, __ldg(img + idx)));
-  });
-  return acc;
+  return siddon3_gather<SELECT>(w, g, img, 0.f);
 }
 
 // Calls f(L, z) for every ray of bin p of a sampled table, in the reference's
@@ -99,9 +96,7 @@ __device__ __forceinline__ float rays_sum3(const ImgGeom& g, const LorTable& t, 
   for_rays(t, p, [&](const float4 L, const float2 z) {
     Walk3 w;
     siddon3_setup(L.x, L.y, z.x, A_SUB(L.z, L.x), A_SUB(L.w, L.y), A_SUB(z.y, z.x), g, w);
-    siddon3_walk(w, g, [&](bool inb, int idx, float seg) {
-      if (inb) acc = A_ADD(acc, A_MUL(seg, __ldg(img + idx)));
-    });
+    acc = siddon3_gather<true>(w, g, img, acc);
   });
   return acc;
 }
@@ -165,7 +160,7 @@ __device__ __forceinline__ double block_sum(double v) {
 }
 
 // ---------------------------------------------------------------------------
-template <bool F64A>
+template <bool F64A, bool SELECT>
 __global__ void __launch_bounds__(kBlock) k_project3(ImgGeom g, LorTable t, SubsetSel s, PreciseGeom pg,
                                                      const float* __restrict__ img, float* __restrict__ out,
                                                      int64_t total) {
@@ -179,7 +174,7 @@ __global__ void __launch_bounds__(kBlock) k_project3(ImgGeom g, LorTable t, Subs
     out[b] = rays_sum3(g, t, p, img);
   } else {
     Walk3 w;
-    out[b] = ray_sum3(g, t.lor[(int64_t)p.a * t.n_r + p.l], t.z[p.g], img, w);
+    out[b] = ray_sum3<SELECT>(g, t.lor[(int64_t)p.a * t.n_r + p.l], t.z[p.g], img, w);
   }
 }
 
@@ -1563,9 +1558,25 @@ cudaError_t launch_project(const ImgGeom& g, const LorTable& t, SubsetSel s, con
                            cudaStream_t st, const PreciseGeom& pg) {
   const int64_t total = (int64_t)t.n_sinos * s.nk * t.n_r;
   if (total == 0) return cudaSuccess;
-  if (t.is3d && pg.enabled) k_project3<true><<<grid_for(total), kBlock, 0, st>>>(g, t, s, pg, img, out, total);
-  else if (t.is3d) k_project3<false><<<grid_for(total), kBlock, 0, st>>>(g, t, s, pg, img, out, total);
-  else k_project2<<<grid_for(total), kBlock, 0, st>>>(g, t, s, img, out, total);
+  if (t.is3d && pg.enabled) {
+    k_project3<true, true><<<grid_for(total), kBlock, 0, st>>>(g, t, s, pg, img, out, total);
+  } else if (t.is3d) {
+    // Few bins wait for their walks' chains of steps, many for the issue
+    // slots (us, step by step before -> select, branch): 22 K bins of a 230 x
+    // 230 slice 83 -> 28, 42; 89 K 71 -> 56, 55; 92 K of a 250 x 250 x 8
+    // image 97 -> 65, 65; 1.5 M 541 -> 619, 525.
+    int dev = 0, sms = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
+    const int small = 64;  // threads: a few warps on every SM
+    if (total <= (int64_t)sms * 512 || t.lor_s)
+      k_project3<false, true><<<(unsigned)((total + small - 1) / small), small, 0, st>>>(g, t, s, pg, img, out, total);
+    else
+      k_project3<false, false><<<grid_for(total), kBlock, 0, st>>>(g, t, s, pg, img, out, total);
+  } else {
+    k_project2<<<grid_for(total), kBlock, 0, st>>>(g, t, s, img, out, total);
+  }
   return cudaGetLastError();
 }
 

@@ -154,26 +154,18 @@ __device__ __forceinline__ float next_crossing(const Walk3& w, bool& cx, bool& c
 
 // One step of a guarded padded walk past its next crossing (x when cx, y
 // when cy, else z): the linear index moves one voxel along that axis and the
-// axis's crossing parameter advances by its increment.  APIRL_STEP_SELECT
-// computes all three candidate parameters and selects (no divergent branch;
-// the same float additions on the same operands, so the walk is unchanged):
-// on B200 0.5 % faster on the listed pass and 4 % slower on the full pass
-// than the branch, so it is off by default.
-#ifndef APIRL_STEP_SELECT
-#define APIRL_STEP_SELECT 0
-#endif
+// axis's crossing parameter advances by its increment.  All three candidate
+// parameters are added up and selected from (the same float additions on the
+// same operands as in a branch, without one that parts the lanes): passes too
+// small to fill the chip wait for this chain.  Against the branch: an EM pass
+// over one sinogram of 143 x 143 62 -> 56 us, listed 221 x 221 102 -> 80, 14
+// sinograms of 250 x 250 x 8 638 -> 628.
 __device__ __forceinline__ void step_pad(Walk3& w, int& idx, bool cx, bool cy, int sx, int sy, int sz) {
-#if APIRL_STEP_SELECT
   const float ax = A_ADD(w.ax, w.axu), ay = A_ADD(w.ay, w.ayu), az = A_ADD(w.az, w.azu);
   idx += cx ? sx : (cy ? sy : sz);
   w.ax = cx ? ax : w.ax;
   w.ay = cy ? ay : w.ay;
   w.az = (cx | cy) ? w.az : az;
-#else
-  if (cx) { idx += sx; w.ax = A_ADD(w.ax, w.axu); }
-  else if (cy) { idx += sy; w.ay = A_ADD(w.ay, w.ayu); }
-  else { idx += sz; w.az = A_ADD(w.az, w.azu); }
-#endif
 }
 
 // Walks over an image padded with a kPad-voxel zero border on every side
@@ -190,8 +182,10 @@ __device__ __forceinline__ void step_pad(Walk3& w, int& idx, bool cx, bool cy, i
 // Otherwise the reference's bounds test is applied.
 // Segments per iteration of the guarded gather: their voxel loads are all
 // issued before any product is added (the additions keep the walk order).
+// Eight: EM passes over one sinogram 56 -> 44 us (143 x 143) and 64 -> 50
+// (180 x 180) against four, 12 no better.
 #ifndef APIRL_GATHER_UNROLL
-#define APIRL_GATHER_UNROLL 4
+#define APIRL_GATHER_UNROLL 8
 #endif
 template <int U = APIRL_GATHER_UNROLL>
 __device__ __forceinline__ float siddon3_gather_pad(Walk3 w, const ImgGeom& g, int ux, int uy, int uz, unsigned lim,
@@ -417,6 +411,30 @@ __device__ __forceinline__ void siddon3_scatter2_pad(Walk3 w, const ImgGeom& g, 
   }
 }
 
+// One step of a bounds-tested walk past its next crossing at an.  SELECT: all
+// three axes' next crossings are added up and selected from, without a branch
+// that parts the lanes (fewer cycles a step); else the branch (fewer
+// instructions).
+template <bool SELECT>
+__device__ __forceinline__ void step_checked(Walk3& w, int& idx, float an, bool cx, bool cy, int sx, int sy, int sz) {
+  w.ac = an;
+  if (SELECT) {
+    const bool cz = !(cx | cy);
+    const float ax = A_ADD(w.ax, w.axu), ay = A_ADD(w.ay, w.ayu), az = A_ADD(w.az, w.azu);
+    w.ax = cx ? ax : w.ax;
+    w.ay = cy ? ay : w.ay;
+    w.az = cz ? az : w.az;
+    w.i += cx ? w.iinc : 0;
+    w.j += cy ? w.jinc : 0;
+    w.k += cz ? w.kinc : 0;
+    idx += cx ? sx : (cy ? sy : sz);
+  } else {
+    if (cx) { w.i += w.iinc; idx += sx; w.ax = A_ADD(w.ax, w.axu); }
+    else if (cy) { w.j += w.jinc; idx += sy; w.ay = A_ADD(w.ay, w.ayu); }
+    else { w.k += w.kinc; idx += sz; w.az = A_ADD(w.az, w.azu); }
+  }
+}
+
 template <class V>
 __device__ __forceinline__ void siddon3_walk(Walk3 w, const ImgGeom& g, V&& visit) {
   if (walk_misses(w, g)) return;
@@ -429,11 +447,38 @@ __device__ __forceinline__ void siddon3_walk(Walk3 w, const ImgGeom& g, V&& visi
     const bool inb = ((unsigned)w.i < (unsigned)g.nx) & ((unsigned)w.j < (unsigned)g.ny) &
                      ((unsigned)w.k < (unsigned)g.nz);
     visit(inb, idx, seg);
-    w.ac = an;
-    if (cx) { w.i += w.iinc; idx += sx; w.ax = A_ADD(w.ax, w.axu); }
-    else if (cy) { w.j += w.jinc; idx += sy; w.ay = A_ADD(w.ay, w.ayu); }
-    else { w.k += w.kinc; idx += sz; w.az = A_ADD(w.az, w.azu); }
+    step_checked<true>(w, idx, an, cx, cy, sx, sy, sz);
   }
+}
+
+// acc + the sum over the walk's segments in the image of length * voxel, in
+// their order.  A batch's voxels are all in flight before its sums (a segment
+// outside the image reads the first voxel and adds nothing).
+template <bool SELECT, int U = 8>
+__device__ __forceinline__ float siddon3_gather(Walk3 w, const ImgGeom& g, const float* __restrict__ img, float acc) {
+  if (walk_misses(w, g)) return acc;
+  const int sx = w.iinc, sy = w.jinc * g.nx, sz = w.kinc * g.nx * g.ny;
+  int idx = (w.k * g.ny + w.j) * g.nx + w.i;
+  for (int m = 0; m < w.n; m += U) {
+    float seg[U], v[U];
+    bool in[U];
+    #pragma unroll
+    for (int u = 0; u < U; u++) {
+      bool cx, cy;
+      const float an = next_crossing(w, cx, cy);
+      seg[u] = A_MUL(A_SUB(an, w.ac), w.L);
+      in[u] = (m + u < w.n) & ((unsigned)w.i < (unsigned)g.nx) & ((unsigned)w.j < (unsigned)g.ny) &
+              ((unsigned)w.k < (unsigned)g.nz);
+      v[u] = __ldg(img + (in[u] ? idx : 0));
+      step_checked<SELECT>(w, idx, an, cx, cy, sx, sy, sz);
+    }
+    #pragma unroll
+    for (int u = 0; u < U; u++) {
+      const float with = A_ADD(acc, A_MUL(seg[u], v[u]));
+      acc = in[u] ? with : acc;
+    }
+  }
+  return acc;
 }
 
 // ---------------------------------------------------------------------------
