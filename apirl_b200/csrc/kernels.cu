@@ -107,7 +107,7 @@ __device__ __forceinline__ void rays_scatter3(const ImgGeom& g, const LorTable& 
   for_rays(t, p, [&](const float4 L, const float2 z) {
     Walk3 w;
     siddon3_setup(L.x, L.y, z.x, A_SUB(L.z, L.x), A_SUB(L.w, L.y), A_SUB(z.y, z.x), g, w);
-    siddon3_walk(w, g, [&](bool inb, int idx, float seg) {
+    siddon3_walk<true>(w, g, [&](bool inb, int idx, float seg) {
       if (!inb) return;
       float val = A_MUL(seg, v);
       if (divide) val = A_DIV(val, e);
@@ -447,7 +447,8 @@ __device__ __forceinline__ void scatter_bin_warp(const ImgGeom& g, const LorTabl
 // (SiddonProjector.cpp:496).
 // b2A / b2T set: the walk also scatters seg into that second padded pair,
 // for every bin (the unweighted image A_s^T 1 beside A_s^T v).
-template <int ACC>
+// SELECT: the scatter's step (step_pad); false for images of ones.
+template <int ACC, bool SELECT>
 __global__ void __launch_bounds__(kBlock, kPersistMinBlocks) k_scatter_persist(
     ImgGeom g, LorTable t, SubsetSel s, const float* __restrict__ vin, int vin_mode, PadBuffers pad, int64_t total,
     unsigned long long* __restrict__ chunk_counter, float* __restrict__ b2A, float* __restrict__ b2T) {
@@ -484,7 +485,7 @@ __global__ void __launch_bounds__(kBlock, kPersistMinBlocks) k_scatter_persist(
         if (b2A)
           siddon3_scatter2_pad(w, g, tr ? py : 1, tr ? 1 : px, uz, pad.lim, v, tr ? pad.bT : pad.bA, tr ? b2T : b2A);
         else
-          siddon3_scatter_pad<ACC>(w, g, tr ? py : 1, tr ? 1 : px, uz, pad.lim, v, tr ? pad.bT : pad.bA,
+          siddon3_scatter_pad<ACC, SELECT>(w, g, tr ? py : 1, tr ? 1 : px, uz, pad.lim, v, tr ? pad.bT : pad.bA,
                                    tr ? pad.eT : pad.eA);
       }
     }
@@ -873,7 +874,7 @@ __global__ void __launch_bounds__(kBlock) k_zero_bins(ImgGeom g, LorTable t, Sub
       if (pad.bA) {
         const bool tr = fabsf(vx) >= fabsf(vy);
         const int px = g.nx + 2 * kPad, py = g.ny + 2 * kPad;
-        siddon3_scatter_pad(w, g, tr ? py : 1, tr ? 1 : px, px * py, pad.lim, 1.f, tr ? pad.bT : pad.bA);
+        siddon3_scatter_pad<0, false>(w, g, tr ? py : 1, tr ? 1 : px, px * py, pad.lim, 1.f, tr ? pad.bT : pad.bA);
       } else {
         siddon3_walk(w, g, [&](bool inb, int idx, float seg) {
           if (inb) red_add_global(img + idx, seg);
@@ -1319,7 +1320,7 @@ __global__ void __launch_bounds__(kBlock) k_scatter_angles(ImgGeom g, LorTable t
     const bool tr = __ldg(tr_of + a) != 0;
     Walk3 w;
     siddon3_setup(L.x, L.y, z.x, A_SUB(L.z, L.x), A_SUB(L.w, L.y), A_SUB(z.y, z.x), g, w);
-    siddon3_scatter_pad(w, g, tr ? py : 1, tr ? 1 : px, px * py, lim, 1.f, per_angle + (int64_t)a * lim);
+    siddon3_scatter_pad<0, false>(w, g, tr ? py : 1, tr ? 1 : px, px * py, lim, 1.f, per_angle + (int64_t)a * lim);
   }
 }
 
@@ -1598,7 +1599,7 @@ cudaError_t launch_backproject_pad(const ImgGeom& g, const LorTable& t, SubsetSe
   const int64_t total = (int64_t)t.n_sinos * s.nk * t.n_r;
   if (total == 0) return cudaSuccess;
   int per_sm = 0, dev = 0, sms = 0;
-  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_scatter_persist<0>, 128, 0);
+  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_scatter_persist<0, false>, 128, 0);
   if (e != cudaSuccess) return e;
   if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
   if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
@@ -1611,13 +1612,16 @@ cudaError_t launch_backproject_pad(const ImgGeom& g, const LorTable& t, SubsetSe
   const int acc = two ? 0 : pad.acc;
   float* none = nullptr;
   if (acc == 1)
-    e = pad_launch(pad, dim3(grid), dim3(128), st, k_scatter_persist<1>, g, t, s, vin, vin_mode, pad, total, counter,
+    e = pad_launch(pad, dim3(grid), dim3(128), st, k_scatter_persist<1, false>, g, t, s, vin, vin_mode, pad, total, counter,
                    none, none);
   else if (acc == 2)
-    e = pad_launch(pad, dim3(grid), dim3(128), st, k_scatter_persist<2>, g, t, s, vin, vin_mode, pad, total, counter,
+    e = pad_launch(pad, dim3(grid), dim3(128), st, k_scatter_persist<2, false>, g, t, s, vin, vin_mode, pad, total, counter,
                    none, none);
+  else if (vin_mode == 0 && !two)
+    e = pad_launch(pad, dim3(grid), dim3(128), st, k_scatter_persist<0, true>, g, t, s, vin, vin_mode, pad, total,
+                   counter, none, none);
   else
-    e = pad_launch(pad, dim3(grid), dim3(128), st, k_scatter_persist<0>, g, t, s, vin, vin_mode, pad, total, counter,
+    e = pad_launch(pad, dim3(grid), dim3(128), st, k_scatter_persist<0, false>, g, t, s, vin, vin_mode, pad, total, counter,
                    two ? pad2.bA : none, two ? pad2.bT : none);
   if (e != cudaSuccess) return e;
   if ((e = cudaGetLastError()) != cudaSuccess) return e;

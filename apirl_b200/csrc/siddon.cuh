@@ -129,7 +129,7 @@ __device__ __forceinline__ bool walk_misses(const W& w, const ImgGeom& g) {
 // none of a walk that misses the image.
 // `inb` is the full six-sided bounds test; linear_index = (k*ny + j)*nx + i is
 // only meaningful when inb is true.  Record-then-advance as in Siddon.cpp:310-340.
-template <class V>
+template <bool SELECT = false, class V>
 __device__ __forceinline__ void siddon3_walk(Walk3 w, const ImgGeom& g, V&& visit);
 
 // The next crossing of a walk, min(ax, ay, az) with the reference's tie order
@@ -160,12 +160,22 @@ __device__ __forceinline__ float next_crossing(const Walk3& w, bool& cx, bool& c
 // small to fill the chip wait for this chain.  Against the branch: an EM pass
 // over one sinogram of 143 x 143 62 -> 56 us, listed 221 x 221 102 -> 80, 14
 // sinograms of 250 x 250 x 8 638 -> 628.
+// Images of ones (sensitivities) keep the branch: sums of equal lengths round
+// with the order in which the lanes' adds arrive, and with the selected step
+// the FP64 likelihood that takes x . A^T 1 moved by 3e-9.
+template <bool SELECT>
 __device__ __forceinline__ void step_pad(Walk3& w, int& idx, bool cx, bool cy, int sx, int sy, int sz) {
-  const float ax = A_ADD(w.ax, w.axu), ay = A_ADD(w.ay, w.ayu), az = A_ADD(w.az, w.azu);
-  idx += cx ? sx : (cy ? sy : sz);
-  w.ax = cx ? ax : w.ax;
-  w.ay = cy ? ay : w.ay;
-  w.az = (cx | cy) ? w.az : az;
+  if (SELECT) {
+    const float ax = A_ADD(w.ax, w.axu), ay = A_ADD(w.ay, w.ayu), az = A_ADD(w.az, w.azu);
+    idx += cx ? sx : (cy ? sy : sz);
+    w.ax = cx ? ax : w.ax;
+    w.ay = cy ? ay : w.ay;
+    w.az = (cx | cy) ? w.az : az;
+  } else {
+    if (cx) { idx += sx; w.ax = A_ADD(w.ax, w.axu); }
+    else if (cy) { idx += sy; w.ay = A_ADD(w.ay, w.ayu); }
+    else { idx += sz; w.az = A_ADD(w.az, w.azu); }
+  }
 }
 
 // Walks over an image padded with a kPad-voxel zero border on every side
@@ -208,7 +218,7 @@ __device__ __forceinline__ float siddon3_gather_pad(Walk3 w, const ImgGeom& g, i
         sa[u] = A_MUL(A_SUB(an, w.ac), w.L);
         ia[u] = idx;
         w.ac = an;
-        step_pad(w, idx, cx, cy, sx, sy, sz);
+        step_pad<true>(w, idx, cx, cy, sx, sy, sz);
       }
       #pragma unroll
       for (int u = 0; u < U; u++) va[u] = __ldg(img + min((unsigned)ia[u], lim - 1u));
@@ -221,7 +231,7 @@ __device__ __forceinline__ float siddon3_gather_pad(Walk3 w, const ImgGeom& g, i
       const float v = __ldg(img + min((unsigned)idx, lim - 1u));
       acc = A_ADD(acc, A_MUL(A_MUL(A_SUB(an, w.ac), w.L), v));
       w.ac = an;
-      step_pad(w, idx, cx, cy, sx, sy, sz);
+      step_pad<true>(w, idx, cx, cy, sx, sy, sz);
     }
     return acc;
   }
@@ -302,7 +312,7 @@ __device__ __forceinline__ void acc_add(float* __restrict__ img, float* __restri
   }
 }
 
-template <int ACC = 0>
+template <int ACC = 0, bool SELECT = true>
 __device__ __forceinline__ void siddon3_scatter_pad(Walk3 w, const ImgGeom& g, int ux, int uy, int uz, unsigned lim,
                                                     float r, float* __restrict__ img,
                                                     float* __restrict__ err = nullptr, int delay = 0) {
@@ -318,7 +328,7 @@ __device__ __forceinline__ void siddon3_scatter_pad(Walk3 w, const ImgGeom& g, i
       const float an = next_crossing(w, cx, cy);
       acc_add<ACC>(img, err, min((unsigned)idx, lim - 1u), A_MUL(A_MUL(A_SUB(an, w.ac), w.L), r));
       w.ac = an;
-      step_pad(w, idx, cx, cy, sx, sy, sz);
+      step_pad<SELECT>(w, idx, cx, cy, sx, sy, sz);
     }
     return;
   }
@@ -435,7 +445,7 @@ __device__ __forceinline__ void step_checked(Walk3& w, int& idx, float an, bool 
   }
 }
 
-template <class V>
+template <bool SELECT, class V>
 __device__ __forceinline__ void siddon3_walk(Walk3 w, const ImgGeom& g, V&& visit) {
   if (walk_misses(w, g)) return;
   const int sx = w.iinc, sy = w.jinc * g.nx, sz = w.kinc * g.nx * g.ny;
@@ -447,7 +457,7 @@ __device__ __forceinline__ void siddon3_walk(Walk3 w, const ImgGeom& g, V&& visi
     const bool inb = ((unsigned)w.i < (unsigned)g.nx) & ((unsigned)w.j < (unsigned)g.ny) &
                      ((unsigned)w.k < (unsigned)g.nz);
     visit(inb, idx, seg);
-    step_checked<true>(w, idx, an, cx, cy, sx, sy, sz);
+    step_checked<SELECT>(w, idx, an, cx, cy, sx, sy, sz);
   }
 }
 
