@@ -30,7 +30,12 @@ namespace {
 // registers).
 constexpr int kColBlock = 256;
 constexpr int kColBlocks = 5;
-constexpr int kColWarps = kColBlock / 32;
+// With several rays a bin and as many lists to make, blocks of up to 16 warps:
+// 271 sinograms of a 46 x 46 x 37 job, 6 rays a bin 120 -> 92 us against 8, 784
+// of 36 x 36 x 64 159 -> 113, 1141 of 80 x 80 x 78 548 -> 494.
+constexpr int kRaysBlock = 512;
+constexpr int kRaysBlocks = 2;
+constexpr int kMaxWarps = kRaysBlock / 32;
 // Blocks of the LORs with few counts.
 constexpr int kColFewBlock = 64;
 constexpr int kColFewBlocks = 20;
@@ -115,7 +120,7 @@ __device__ __forceinline__ int64_t bin_of(const LorTable& t, const SubsetSel& s,
 
 // The LOR's likelihood partial: the sum of the block's terms, warps in order.
 __device__ __forceinline__ void em_partial(double term, unsigned lor, double* __restrict__ partials) {
-  __shared__ double part[kColWarps];
+  __shared__ double part[kMaxWarps];
   #pragma unroll
   for (int o = 16; o > 0; o >>= 1) term += __shfl_down_sync(0xffffffffu, term, o);
   if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = term;
@@ -150,10 +155,10 @@ __global__ void __launch_bounds__(kColBlock, kColBlocks) k_em_cols(
 // pair, radial sample, axial sample; one running sum): a block keeps one list
 // a radial sample, its lanes take their sinograms' ring pairs in step.  Bound
 // by latency on small images, whose LORs are few: a 64 x 64 x 21 job's subset
-// of 8 with 3 x 2 rays a bin (862 LORs, 91 sinograms) 246 us bin by bin, 102 us
+// of 8 with 3 x 2 rays a bin (862 LORs, 91 sinograms) 246 us bin by bin, 100 us
 // here.
 template <typename CT>
-__global__ void __launch_bounds__(kColBlock, kColBlocks) k_em_cols_rays(
+__global__ void __launch_bounds__(kRaysBlock, kRaysBlocks) k_em_cols_rays(
     ImgGeom g, ColDims d, LorTable t, SubsetSel s, const CT* __restrict__ counts, int counts_packed,
     const float* __restrict__ add, const float* __restrict__ img, float* __restrict__ acc, int back,
     double* __restrict__ partials) {
@@ -387,10 +392,10 @@ ColDims dims_of(const ImgGeom& g, const ColBuffers& c) { return ColDims{g.nx, g.
 
 dim3 voxel_grid(const ImgGeom& g) { return dim3((g.nx + 31) / 32, g.ny, (g.nz + 31) / 32); }
 
-// Warps of a block: up to 8, as few as give the same number of rounds over
+// Threads of a block: up to `most`, as few as give the same number of rounds over
 // the sinograms.
-int block_of(const LorTable& t) {
-  const int groups = (t.n_sinos + 31) / 32, rounds = (groups + kColBlock / 32 - 1) / (kColBlock / 32);
+int block_of(const LorTable& t, int most = kColBlock) {
+  const int groups = (t.n_sinos + 31) / 32, rounds = (groups + most / 32 - 1) / (most / 32);
   return (groups + rounds - 1) / rounds * 32;
 }
 
@@ -426,7 +431,7 @@ template <typename CT>
 static cudaError_t em_cols_rays(const ImgGeom& g, const ColBuffers& c, const LorTable& t, SubsetSel s, const CT* counts,
                                 int counts_packed, const float* add, int back, double* partials, cudaStream_t st) {
   if (lors_of(t, s) == 0) return cudaSuccess;
-  k_em_cols_rays<CT><<<(unsigned)lors_of(t, s), block_of(t), t.n_rs * col_smem(g.nx, g.ny), st>>>(
+  k_em_cols_rays<CT><<<(unsigned)lors_of(t, s), block_of(t, kRaysBlock), t.n_rs * col_smem(g.nx, g.ny), st>>>(
       g, dims_of(g, c), t, s, counts, counts_packed, add, c.img, c.acc, back, partials);
   return cudaGetLastError();
 }
