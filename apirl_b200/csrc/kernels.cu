@@ -200,7 +200,8 @@ __device__ __forceinline__ float load_bin(const float* __restrict__ v, int vin_m
   return __ldg(v + b);
 }
 
-template <bool F64A>
+// SELECT: the walk's step (step_checked); false for images of ones.
+template <bool F64A, bool SELECT>
 __global__ void __launch_bounds__(kBlock) k_backproject3(ImgGeom g, LorTable t, SubsetSel s, PreciseGeom pg,
                                                          const float* __restrict__ vin, int vin_mode,
                                                          const float* __restrict__ vest, int divide,
@@ -233,7 +234,7 @@ __global__ void __launch_bounds__(kBlock) k_backproject3(ImgGeom g, LorTable t, 
     const float2 z = t.z[p.g];
     Walk3 w;
     siddon3_setup(L.x, L.y, z.x, A_SUB(L.z, L.x), A_SUB(L.w, L.y), A_SUB(z.y, z.x), g, w);
-    siddon3_walk(w, g, scatter);
+    siddon3_walk<SELECT>(w, g, scatter);
   }
 }
 
@@ -1586,9 +1587,11 @@ cudaError_t launch_backproject(const ImgGeom& g, const LorTable& t, SubsetSel s,
   const int64_t total = (int64_t)t.n_sinos * s.nk * t.n_r;
   if (total == 0) return cudaSuccess;
   if (t.is3d && pg.enabled)
-    k_backproject3<true><<<grid_for(total), kBlock, 0, st>>>(g, t, s, pg, vin, vin_mode, vest, divide, img, total);
+    k_backproject3<true, false><<<grid_for(total), kBlock, 0, st>>>(g, t, s, pg, vin, vin_mode, vest, divide, img, total);
+  else if (t.is3d && vin_mode == 0)
+    k_backproject3<false, true><<<grid_for(total), kBlock, 0, st>>>(g, t, s, pg, vin, vin_mode, vest, divide, img, total);
   else if (t.is3d)
-    k_backproject3<false><<<grid_for(total), kBlock, 0, st>>>(g, t, s, pg, vin, vin_mode, vest, divide, img, total);
+    k_backproject3<false, false><<<grid_for(total), kBlock, 0, st>>>(g, t, s, pg, vin, vin_mode, vest, divide, img, total);
   else k_backproject2<<<grid_for(total), kBlock, 0, st>>>(g, t, s, vin, vin_mode, vest, divide, img, total);
   return cudaGetLastError();
 }

@@ -126,7 +126,7 @@ __device__ __forceinline__ bool walk_misses(const W& w, const ImgGeom& g) {
 }
 
 // Visits the n recorded segments in order: visit(inb, linear_index, length);
-// none of a walk that misses the image.
+// SELECT: step_checked's, and none of a walk that misses the image.
 // `inb` is the full six-sided bounds test; linear_index = (k*ny + j)*nx + i is
 // only meaningful when inb is true.  Record-then-advance as in Siddon.cpp:310-340.
 template <bool SELECT = false, class V>
@@ -160,9 +160,10 @@ __device__ __forceinline__ float next_crossing(const Walk3& w, bool& cx, bool& c
 // small to fill the chip wait for this chain.  Against the branch: an EM pass
 // over one sinogram of 143 x 143 62 -> 56 us, listed 221 x 221 102 -> 80, 14
 // sinograms of 250 x 250 x 8 638 -> 628.
-// Images of ones (sensitivities) keep the branch: sums of equal lengths round
-// with the order in which the lanes' adds arrive, and with the selected step
-// the FP64 likelihood that takes x . A^T 1 moved by 3e-9.
+// Images of ones (sensitivities) keep the branch, and walk the rays that miss
+// the image: sums of equal lengths round with the order in which the lanes'
+// adds arrive, and with the selected step the FP64 likelihood that takes
+// x . A^T 1 moved by 3e-9, without the missing rays by 4e-10.
 template <bool SELECT>
 __device__ __forceinline__ void step_pad(Walk3& w, int& idx, bool cx, bool cy, int sx, int sy, int sz) {
   if (SELECT) {
@@ -332,7 +333,7 @@ __device__ __forceinline__ void siddon3_scatter_pad(Walk3 w, const ImgGeom& g, i
     }
     return;
   }
-  if (walk_misses(w, g)) return;
+  if (SELECT && walk_misses(w, g)) return;
   for (int m = 0; m < w.n; m++) {
     bool cx, cy;
     const float an = next_crossing(w, cx, cy);
@@ -358,7 +359,7 @@ __device__ __forceinline__ void siddon3_scatter_pad_warp(Walk3 w, const ImgGeom&
                                                          unsigned lim, float r, float* __restrict__ img, bool live) {
   __shared__ float slot[256];
   const int lane = (int)(threadIdx.x & 31), warp0 = (int)threadIdx.x - lane;
-  const int n = live && (w.guarded || !walk_misses(w, g)) ? w.n : 0;
+  const int n = live ? w.n : 0;
   const int nmax = __reduce_max_sync(0xffffffffu, n);
   const int sx = w.iinc * ux, sy = w.jinc * uy, sz = w.kinc * uz;
   int idx = live ? (w.k + kPad) * uz + (w.j + kPad) * uy + (w.i + kPad) * ux : 0;
@@ -402,7 +403,6 @@ __device__ __forceinline__ void siddon3_scatter2_pad(Walk3 w, const ImgGeom& g, 
   const int sx = w.iinc * ux, sy = w.jinc * uy, sz = w.kinc * uz;
   int idx = (w.k + kPad) * uz + (w.j + kPad) * uy + (w.i + kPad) * ux;
   const bool first = r1 != 0.f;
-  if (!w.guarded && walk_misses(w, g)) return;
   for (int m = 0; m < w.n; m++) {
     bool cx, cy;
     const float an = next_crossing(w, cx, cy);
@@ -447,7 +447,7 @@ __device__ __forceinline__ void step_checked(Walk3& w, int& idx, float an, bool 
 
 template <bool SELECT, class V>
 __device__ __forceinline__ void siddon3_walk(Walk3 w, const ImgGeom& g, V&& visit) {
-  if (walk_misses(w, g)) return;
+  if (SELECT && walk_misses(w, g)) return;
   const int sx = w.iinc, sy = w.jinc * g.nx, sz = w.kinc * g.nx * g.ny;
   int idx = (w.k * g.ny + w.j) * g.nx + w.i;
   for (int m = 0; m < w.n; m++) {
