@@ -68,11 +68,14 @@ constexpr int kEmMinBlocks = APIRL_EM_MIN_BLOCKS;
 #endif
 
 // Forward projection of one bin (3D), masked gather of the image.
-template <bool SELECT = true>
 __device__ __forceinline__ float ray_sum3(const ImgGeom& g, const float4 L, const float2 z, const float* __restrict__ img,
                                           Walk3& w) {
   siddon3_setup(L.x, L.y, z.x, A_SUB(L.z, L.x), A_SUB(L.w, L.y), A_SUB(z.y, z.x), g, w);
-  return siddon3_gather<SELECT>(w, g, img, 0.f);
+  float acc = 0.f;
+  siddon3_walk(w, g, [&](bool inb, int idx, float seg) {
+    if (inb) acc = A_ADD(acc, A_MUL(seg, __ldg(img + idx)));
+  });
+  return acc;
 }
 
 // Calls f(L, z) for every ray of bin p of a sampled table, in the reference's
@@ -90,13 +93,21 @@ __device__ __forceinline__ void for_rays(const LorTable& t, const BinPos& p, F&&
 
 // Forward projection of one bin over all its rays: one running sum, as the
 // reference increments the zero-filled bin ray after ray (SiddonProjector.cpp:339,419).
+// BATCH: siddon3_gather (projections; the EM pass keeps its pace, step_pad).
+template <bool BATCH>
 __device__ __forceinline__ float rays_sum3(const ImgGeom& g, const LorTable& t, const BinPos& p,
                                            const float* __restrict__ img) {
   float acc = 0.f;
   for_rays(t, p, [&](const float4 L, const float2 z) {
     Walk3 w;
     siddon3_setup(L.x, L.y, z.x, A_SUB(L.z, L.x), A_SUB(L.w, L.y), A_SUB(z.y, z.x), g, w);
-    acc = siddon3_gather<true>(w, g, img, acc);
+    if (BATCH) {
+      acc = siddon3_gather<true>(w, g, img, acc);
+    } else {
+      siddon3_walk(w, g, [&](bool inb, int idx, float seg) {
+        if (inb) acc = A_ADD(acc, A_MUL(seg, __ldg(img + idx)));
+      });
+    }
   });
   return acc;
 }
@@ -107,7 +118,7 @@ __device__ __forceinline__ void rays_scatter3(const ImgGeom& g, const LorTable& 
   for_rays(t, p, [&](const float4 L, const float2 z) {
     Walk3 w;
     siddon3_setup(L.x, L.y, z.x, A_SUB(L.z, L.x), A_SUB(L.w, L.y), A_SUB(z.y, z.x), g, w);
-    siddon3_walk<true>(w, g, [&](bool inb, int idx, float seg) {
+    siddon3_walk(w, g, [&](bool inb, int idx, float seg) {
       if (!inb) return;
       float val = A_MUL(seg, v);
       if (divide) val = A_DIV(val, e);
@@ -171,10 +182,13 @@ __global__ void __launch_bounds__(kBlock) k_project3(ImgGeom g, LorTable t, Subs
     Walk3D w;
     out[b] = ray_sum3d(geom_d(pg), pg.lor[(int64_t)p.a * t.n_r + p.l], pg.z[p.g], img, w);
   } else if (t.lor_s) {
-    out[b] = rays_sum3(g, t, p, img);
+    out[b] = rays_sum3<true>(g, t, p, img);
   } else {
     Walk3 w;
-    out[b] = ray_sum3<SELECT>(g, t.lor[(int64_t)p.a * t.n_r + p.l], t.z[p.g], img, w);
+    const float4 L = t.lor[(int64_t)p.a * t.n_r + p.l];
+    const float2 z = t.z[p.g];
+    siddon3_setup(L.x, L.y, z.x, A_SUB(L.z, L.x), A_SUB(L.w, L.y), A_SUB(z.y, z.x), g, w);
+    out[b] = siddon3_gather<SELECT>(w, g, img, 0.f);
   }
 }
 
@@ -409,7 +423,7 @@ __global__ void __launch_bounds__(kBlock) k_em_pass_rays(ImgGeom g, LorTable t, 
     const int64_t row = counts_packed ? ((int64_t)(p.g - t.g0) * s.nk + p.k) : ((int64_t)p.g * t.n_proj + p.a);
     const int64_t ci = row * t.n_r + p.l;
     const float m = load_count<CT>(counts, ci);
-    float e = rays_sum3(g, t, p, x);
+    float e = rays_sum3<false>(g, t, p, x);
     if (add) e = A_ADD(e, __ldg(add + ci));
     const float r = (m != 0.f && e != 0.f) ? A_DIV(m, e) : 0.f;
     if (lik_mode == 2) { if (r > 0.f) term = (double)m * log((double)r) - (double)r; }

@@ -154,16 +154,14 @@ __device__ __forceinline__ float next_crossing(const Walk3& w, bool& cx, bool& c
 
 // One step of a guarded padded walk past its next crossing (x when cx, y
 // when cy, else z): the linear index moves one voxel along that axis and the
-// axis's crossing parameter advances by its increment.  All three candidate
-// parameters are added up and selected from (the same float additions on the
-// same operands as in a branch, without one that parts the lanes): passes too
-// small to fill the chip wait for this chain.  Against the branch: an EM pass
-// over one sinogram of 143 x 143 62 -> 56 us, listed 221 x 221 102 -> 80, 14
-// sinograms of 250 x 250 x 8 638 -> 628.
-// Images of ones (sensitivities) keep the branch, and walk the rays that miss
-// the image: sums of equal lengths round with the order in which the lanes'
-// adds arrive, and with the selected step the FP64 likelihood that takes
-// x . A^T 1 moved by 3e-9, without the missing rays by 4e-10.
+// axis's crossing parameter advances by its increment.  SELECT: all three
+// candidate parameters are added up and selected from (the same float
+// additions on the same operands, without a branch that parts the lanes):
+// scatters too small to fill the chip wait for this chain (backprojection of a
+// 199 x 199 slice 37 -> 28 us).  Images of ones and EM passes keep the branch:
+// their sums round with the order in which the lanes' adds arrive, which hardly
+// varies from run to run over few sinograms, and the step's pace moved FP64
+// likelihoods by 1e-9 to 3e-9 (EM passes over one slice gained 1.2 - 1.4x).
 template <bool SELECT>
 __device__ __forceinline__ void step_pad(Walk3& w, int& idx, bool cx, bool cy, int sx, int sy, int sz) {
   if (SELECT) {
@@ -193,10 +191,8 @@ __device__ __forceinline__ void step_pad(Walk3& w, int& idx, bool cx, bool cy, i
 // Otherwise the reference's bounds test is applied.
 // Segments per iteration of the guarded gather: their voxel loads are all
 // issued before any product is added (the additions keep the walk order).
-// Eight: EM passes over one sinogram 56 -> 44 us (143 x 143) and 64 -> 50
-// (180 x 180) against four, 12 no better.
 #ifndef APIRL_GATHER_UNROLL
-#define APIRL_GATHER_UNROLL 8
+#define APIRL_GATHER_UNROLL 4
 #endif
 template <int U = APIRL_GATHER_UNROLL>
 __device__ __forceinline__ float siddon3_gather_pad(Walk3 w, const ImgGeom& g, int ux, int uy, int uz, unsigned lim,
@@ -219,7 +215,7 @@ __device__ __forceinline__ float siddon3_gather_pad(Walk3 w, const ImgGeom& g, i
         sa[u] = A_MUL(A_SUB(an, w.ac), w.L);
         ia[u] = idx;
         w.ac = an;
-        step_pad<true>(w, idx, cx, cy, sx, sy, sz);
+        step_pad<false>(w, idx, cx, cy, sx, sy, sz);
       }
       #pragma unroll
       for (int u = 0; u < U; u++) va[u] = __ldg(img + min((unsigned)ia[u], lim - 1u));
@@ -232,11 +228,10 @@ __device__ __forceinline__ float siddon3_gather_pad(Walk3 w, const ImgGeom& g, i
       const float v = __ldg(img + min((unsigned)idx, lim - 1u));
       acc = A_ADD(acc, A_MUL(A_MUL(A_SUB(an, w.ac), w.L), v));
       w.ac = an;
-      step_pad<true>(w, idx, cx, cy, sx, sy, sz);
+      step_pad<false>(w, idx, cx, cy, sx, sy, sz);
     }
     return acc;
   }
-  if (walk_misses(w, g)) return acc;
   for (int m = 0; m < w.n; m++) {
     bool cx, cy;
     const float an = next_crossing(w, cx, cy);
@@ -313,7 +308,7 @@ __device__ __forceinline__ void acc_add(float* __restrict__ img, float* __restri
   }
 }
 
-template <int ACC = 0, bool SELECT = true>
+template <int ACC = 0, bool SELECT = false>
 __device__ __forceinline__ void siddon3_scatter_pad(Walk3 w, const ImgGeom& g, int ux, int uy, int uz, unsigned lim,
                                                     float r, float* __restrict__ img,
                                                     float* __restrict__ err = nullptr, int delay = 0) {

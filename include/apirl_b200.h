@@ -221,7 +221,7 @@ enum {
 };
 /* APIRL_OPT_GATHER_UNROLL (default 0): segments of a walk whose image loads
  * the persistent fused 3D pass issues before it adds any of them: 4, 6 or 8,
- * or 0 for the pass kind's default (6 over a list of bins, 8 over every bin).
+ * or 0 for the pass kind's default (6 over a list of bins, 4 over every bin).
  * Results do not depend on it.  Plain atomics only. */
 /* APIRL_OPT_L2_PERSIST (default 0): 1 = the padded 3D passes launch with an L2
  * access policy window over the projector's padded images and
