@@ -219,6 +219,14 @@ apirl_status check_subset(const apirl_projector* p, int subset, int nsub) {
   return APIRL_OK;
 }
 
+// Waits for the tables and zeros written on the legacy stream: a memset, or a
+// copy from pageable memory, may return before the device has it, and a
+// projector's first pass may run on a stream that does not wait for that one.
+apirl_status settled() {
+  CK(cudaStreamSynchronize(nullptr));
+  return APIRL_OK;
+}
+
 // The padded two-layout buffers of the fused 3D pass, allocated with the
 // projector so that no pass allocates (passes may be captured into CUDA
 // graphs).  Volumes whose padded size does not fit a 32-bit index keep the
@@ -335,6 +343,7 @@ apirl_status finish_create(apirl_projector* p, apirl_projector** out) {
     pl.sumT = pl.sum + copies * lim;
     pl.lim = (unsigned)lim;
   }
+  if (apirl_status st = settled()) return st;
   *out = p;
   return APIRL_OK;
 }
@@ -568,6 +577,7 @@ apirl_status apirl_projector_set_alpha_precision(apirl_projector* p, int mode) {
     p->pg.dx = p->g.dx; p->pg.dy = p->g.dy; p->pg.dz = p->g.dz;
     p->pg.rfov = ((double)p->g.dx * p->g.nx) / 2;
     p->pg.offz = (double)p->g.dz / 2;
+    if (apirl_status st = settled()) return st;
   }
   p->alpha_mode = mode;
   p->pg.enabled = mode == APIRL_ALPHA_F64;
@@ -622,6 +632,7 @@ apirl_status apirl_projector_set_sampling(apirl_projector* p, int n_samples, int
     CK(cudaMalloc(&p->d_zoff[k], rt.zoff.size() * sizeof(int)));
     CK(cudaMemcpy(p->d_zoff[k], rt.zoff.data(), rt.zoff.size() * sizeof(int), cudaMemcpyHostToDevice));
   }
+  if (apirl_status st = settled()) return st;
   for (int k = 0; k < 2; k++) {
     dst[k]->lor_s = p->d_lor_s[k];
     dst[k]->zs = p->d_zs[k];
@@ -997,7 +1008,8 @@ apirl_status apirl_projector_set_option(apirl_projector* p, int option, int valu
       p->dual_layout = value != 0;
       if (p->dual_layout && p->is3d) {
         DEVICE_SCOPE(p->device);
-        return alloc_pad(p);
+        const apirl_status st = alloc_pad(p);
+        return st ? st : settled();
       }
       return APIRL_OK;
     }
@@ -1058,6 +1070,7 @@ apirl_status apirl_projector_set_option(apirl_projector* p, int option, int valu
         CK(cudaMalloc(&p->pad.eT, pv * sizeof(float)));
         CK(cudaMemset(p->pad.eA, 0, pv * sizeof(float)));
         CK(cudaMemset(p->pad.eT, 0, pv * sizeof(float)));
+        if (apirl_status st = settled()) return st;
       }
       p->pad.acc = value;
       return APIRL_OK;
@@ -1344,8 +1357,8 @@ apirl_status backproject_sino_and_ones(apirl_projector* p, SubsetSel ss, const f
     const size_t pv = (size_t)p->pad.lim;
     CK(cudaMalloc(&p->pad2.bA, pv * sizeof(float)));
     CK(cudaMalloc(&p->pad2.bT, pv * sizeof(float)));
-    CK(cudaMemset(p->pad2.bA, 0, pv * sizeof(float)));
-    CK(cudaMemset(p->pad2.bT, 0, pv * sizeof(float)));
+    CK(cudaMemsetAsync(p->pad2.bA, 0, pv * sizeof(float), st));
+    CK(cudaMemsetAsync(p->pad2.bT, 0, pv * sizeof(float), st));
     p->pad2.lim = p->pad.lim;
   }
   CK(launch_backproject_pad(p->g, p->t, ss, vin, vin_mode, img, p->pad, p->d_chunk, st, gimg, p->pad2));

@@ -1,0 +1,43 @@
+"""The calls that the library's host code makes, on a runtime without a GPU
+(fake_gpu.py): what a projector writes is in place before a stream reads it."""
+import pytest
+
+import fake_gpu
+
+
+@pytest.fixture(scope="module")
+def gpu(tmp_path_factory):
+    so = fake_gpu.build(tmp_path_factory.mktemp("fake"))
+    return lambda script: fake_gpu.run(so, script)
+
+
+GEOMS = '''
+G3 = (ImageGeom(32, 32, 21, 2.0, 2.0, 2.0), Sino3DGeom.span1(16, 40, 11, 33.0, 22.0, 100.0, 1))
+G2 = (ImageGeom(32, 32, 1, 2.0, 2.0, 2.0), Sino2DGeom(16, 40, 33.0, 100.0))
+'''
+
+
+def waited(log):
+    """The legacy stream was waited for after the last write on it."""
+    writes = [i for i, l in enumerate(log) if l.split()[:2] in (["memset", "legacy"], ["memcpy", "legacy"])]
+    waits = [i for i, l in enumerate(log) if l.split()[:2] == ["sync", "legacy"]]
+    return bool(writes) and bool(waits) and waits[-1] > writes[-1]
+
+
+@pytest.mark.parametrize("step", ["ap.SiddonProjector(*G3)", "ap.SiddonProjector(*G2)", "P.set_sampling(2, 2)",
+                                  "P.set_alpha_precision(True)",
+                                  "P.set_option(_lib.APIRL_OPT_ACCUMULATE, _lib.APIRL_ACC_COMPENSATED)"])
+def test_tables_and_zeros_are_waited_for(gpu, step):
+    """Non-blocking streams do not wait for the legacy stream, on which tables are copied and buffers cleared."""
+    log = gpu(GEOMS + f"P = ap.SiddonProjector(*G3)\nfake.clear()\n{step}\ndone(fake.log())")
+    assert waited(log), log
+
+
+def test_second_pair_is_cleared_on_the_callers_stream(gpu):
+    log = gpu(GEOMS + '''
+P = ap.SiddonProjector(*G3)
+fake.clear()
+_lib.check(lib.apirl_backproject_and_ones(P.h, D, D, ctypes.c_void_p(1 << 42), -1, 1, S))
+done(fake.log())''')
+    assert any(l.startswith("memset 0x9990") for l in log)
+    assert not any(l.split()[:2] == ["memset", "legacy"] for l in log), log
