@@ -62,3 +62,24 @@ def test_pass_against_oracle(oracle, nx, ny, n_proj, n_r, dtype):
     for s in range(min(2, n_proj)):
         P.em_project_backproject(t(meas), t(x0), bp, s, min(2, n_proj))
     assert rel(bp.cpu().numpy(), x0 + ratio) <= 1e-5
+
+
+def test_image_of_several_slices(oracle):
+    """A 2D pass over a two-slice image: the rays cross the first slice; the
+    other has no backprojection, so its update is x * 0 / sens = 0."""
+    ig, sg = ImageGeom(33, 31, 2, 2.0, 2.0, 1.0), Sino2DGeom(16, 40, 40.0, 400.0)
+    one = ImageGeom(33, 31, 1, 2.0, 2.0, 1.0)
+    n = one.n_voxels
+    rng = np.random.default_rng(3)
+    x0 = (rng.random(ig.n_voxels, dtype=np.float32) + 0.5).astype(np.float32)
+    sens = (rng.random(ig.n_voxels, dtype=np.float32) + 1).astype(np.float32)
+    est = oracle.project_2d(sg, one, x0[:n])
+    meas = rng.poisson(est * 2 + 0.3).astype(np.float32)
+    want = oracle.update(x0[:n], oracle.backproject_2d(sg, one, oracle.inverse_divide(meas, est)), sens[:n],
+                         np.float32(0), False)
+    P = ap.SiddonProjector(ig, sg)
+    x = t(x0)
+    P.em_pass(t(meas), x, torch.zeros(ig.n_voxels, dtype=torch.float32, device=DEV), t(sens), ge=False)
+    got = x.cpu().numpy()
+    assert rel(got[:n], want) <= 1e-5
+    assert not got[n:].any()

@@ -41,3 +41,15 @@ _lib.check(lib.apirl_backproject_and_ones(P.h, D, D, ctypes.c_void_p(1 << 42), -
 done(fake.log())''')
     assert any(l.startswith("memset 0x9990") for l in log)
     assert not any(l.split()[:2] == ["memset", "legacy"] for l in log), log
+
+
+@pytest.mark.parametrize("nz", [1, 2])
+def test_2d_passes_update_every_slice(gpu, nz):
+    """The padded 2D layouts hold one slice; an image of several takes the pass that updates all its voxels."""
+    names = gpu(f'''
+P = ap.SiddonProjector(ImageGeom(32, 32, {nz}, 2.0, 2.0, 2.0), Sino2DGeom(16, 40, 33.0, 100.0))
+fake.clear()
+_lib.check(lib.apirl_em_pass(P.h, D, 0, 0, None, D, D, D, None, 0.0, 0, -1, 1, None, S))
+done(fake.launches())''')
+    assert any("k_planar_update" in n for n in names) == (nz == 1)
+    assert any("k_update" in n for n in names) == (nz == 2)
