@@ -334,7 +334,7 @@ apirl_status finish_create(apirl_projector* p, apirl_projector** out) {
   }
   // (Images of several slices, of which a 2D pass projects the first and updates
   // all, keep to the unpadded pass.)
-  if (!p->is3d && p->g.nz == 1 && apirl::planar_lim(p->g) && (int64_t)p->t.n_proj * p->t.n_r < INT_MAX) {
+  if (!p->is3d && p->g.nz == 1 && apirl::planar_lim(p->g) && (int64_t)p->t.n_proj * p->t.n_r <= INT_MAX - 31) {
     apirl::PlanarBuffers& pl = p->planar;
     const size_t lim = apirl::planar_lim(p->g);
     constexpr int copies = apirl::kPlanarCopies;

@@ -415,9 +415,10 @@ ColBuffers col_layout(const ImgGeom& g, const float* z_ends, int n_ends) {
   const double z0 = ceil(fmax((double)kColSpare, -first) / 2) * 2, slices = fmax((double)g.nz + kColSpare, end) + z0;
   const double floats = (double)(g.nx + 2 * kPad) * (g.ny + 2 * kPad) * (slices + 16);
   // Bounded in bytes and against the image (a long scanner around a short
-  // image), in grid sizes and in the list's shared memory.
+  // image), in grid sizes (a layer more for the likelihood) and in the list's
+  // shared memory.
   if (!(floats < (double)(1 << 30)) || floats > 4.0 * g.nx * g.ny * g.nz + (1 << 22) || g.ny > 65535 ||
-      g.nz > 65535 * 32 || col_smem(g.nx, g.ny) > kColMaxSmem)
+      g.nz > 65534 * 32 || col_smem(g.nx, g.ny) > kColMaxSmem)
     return c;
   c.z0 = (int)z0;
   c.half = (((int)slices + 1) / 2 + 7) / 8 * 8;

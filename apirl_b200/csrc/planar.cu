@@ -221,7 +221,8 @@ __global__ void __launch_bounds__(256) k_planar_update(int nx, int ny, PlanarBuf
 
 unsigned planar_lim(const ImgGeom& g) {
   const int64_t n = (int64_t)(g.nx + 2 * kPad) * (g.ny + 2 * kPad);
-  return n <= ((int64_t)1 << 25) && g.ny < 65535 * 8 ? (unsigned)n : 0u;
+  // (grids of at most 65535 rows, one of them the likelihood's)
+  return n <= ((int64_t)1 << 25) && g.ny <= 65534 * 8 ? (unsigned)n : 0u;
 }
 
 cudaError_t launch_planar_pass(const ImgGeom& g, const LorTable& t, SubsetSel s, const void* counts, int counts_dtype,

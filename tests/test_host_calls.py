@@ -53,3 +53,27 @@ _lib.check(lib.apirl_em_pass(P.h, D, 0, 0, None, D, D, D, None, 0.0, 0, -1, 1, N
 done(fake.launches())''')
     assert any("k_planar_update" in n for n in names) == (nz == 1)
     assert any("k_update" in n for n in names) == (nz == 2)
+
+
+@pytest.mark.parametrize("ny", [65534 * 8, 65534 * 8 + 1, 65535 * 8 - 1])
+def test_tall_2d_images_stay_within_the_grid(gpu, ny):
+    """The update's grid has one row of blocks a tile row of 8 and one for the likelihood, 65535 at most."""
+    log = gpu(f'''
+P = ap.SiddonProjector(ImageGeom(4, {ny}, 1, 2.0, 2.0, 2.0), Sino2DGeom(3, 4, 33.0, 100.0))
+fake.clear()
+st = lib.apirl_em_pass(P.h, D, 0, 0, None, D, D, D, None, 0.0, 0, -1, 1, D, S)
+done([st] + fake.log())''')
+    assert log[0] == 0 and not any(l.startswith("refused") for l in log[1:]), log
+
+
+@pytest.mark.parametrize("nz", [65534 * 32, 65534 * 32 + 1])
+def test_long_images_stay_within_the_grid(gpu, nz):
+    """As above for the column layout's update, whose grid has a layer more than 32 slices each (images of
+    more than 65535 slices that keep to the padded pair have no pass, and had none)."""
+    log = gpu(f'''
+P = ap.SiddonProjector(ImageGeom(8, 8, {nz}, 2.0, 2.0, 0.01), Sino3DGeom.span1(3, 4, 16, 16.0, 500.0, 100.0, 0))
+fake.clear()
+st = lib.apirl_em_pass(P.h, D, 0, 0, None, D, D, D, None, 0.0, 0, -1, 1, D, S)
+done([st] + fake.log())''')
+    cols = any("k_em_cols" in l for l in log[1:])
+    assert cols == (nz == 65534 * 32) and not any(l.startswith("refused") and "k_col" in l for l in log[1:]), log
