@@ -5,6 +5,7 @@
 #include <cstdio>
 #include <cstring>
 #include <string>
+#include <utility>
 #include <vector>
 #include <climits>
 
@@ -173,7 +174,7 @@ bool project_cols(const apirl_projector* p, SubsetSel ss) {
 
 // Forward projection of the subset into d_sino.
 apirl_status project(apirl_projector* p, SubsetSel ss, const float* d_image, float* d_sino, cudaStream_t s) {
-  if (use_cols(p) && project_cols(p, ss)) {
+  if (use_cols(p) && p->col_img[0].buf && project_cols(p, ss)) {
     bool captured = false;
     apirl_status st = capturing(s, &captured);
     if (st) return st;
@@ -252,57 +253,72 @@ apirl_status alloc_pad(apirl_projector* p) {
   return APIRL_OK;
 }
 
-// The column layout's buffers, one block: the passes' image copy and sum, and
+// Device memory for a layout that the projector can do without: *out stays
+// null where there is no room for it.
+apirl_status alloc_spare(void** out, size_t bytes) {
+  const cudaError_t e = cudaMalloc(out, bytes);
+  if (e == cudaSuccess) return APIRL_OK;
+  *out = nullptr;
+  if (e != cudaErrorMemoryAllocation) return cuda_fail(e, "cudaMalloc");
+  (void)cudaGetLastError();  // handled: not left for the next call
+  return APIRL_OK;
+}
+
+// The column layout's buffers, one block: the passes' image copy and sums, and
 // the slots' (see apirl_projector::ColSlot).  All are made here, so that no
-// later call allocates.
+// later call allocates; where they do not fit, without the slots, or none.
 apirl_status alloc_cols(apirl_projector* p) {
-  if (p->cols.half || p->host.n_sinos < apirl::kColMinSinos) return APIRL_OK;
+  if (p->layouts == apirl::Layouts::kPair || p->cols.half || p->host.n_sinos < apirl::kColMinSinos) return APIRL_OK;
   apirl::ColBuffers c = apirl::col_layout(p->g, p->host.z.data(), (int)p->host.z.size());
   if (!c.half) return APIRL_OK;
-  const size_t n = (size_t)c.floats;
-  float* b = nullptr;
-  cudaError_t e = cudaMalloc(&b, 7 * n * sizeof(float));
-  if (e == cudaSuccess) e = cudaMemset(b, 0, 7 * n * sizeof(float));
-  if (e != cudaSuccess) {
-    cudaFree(b);
-    return cuda_fail(e, "column layout buffers");
-  }
-  p->cols.img = b;  // (owned from here on)
   // The queue: its length, items and lists, one block.
   const size_t lors = (size_t)p->t.n_proj * p->t.n_r;
   char* q = nullptr;
-  CK(cudaMalloc(&q, 16 + lors * (sizeof(uint2) + apirl::kColFew * sizeof(uint16_t))));
-  p->queue.n = (unsigned*)q;
+  if (apirl_status st = alloc_spare((void**)&q, 16 + lors * (sizeof(uint2) + apirl::kColFew * sizeof(uint16_t)))) return st;
+  if (!q) return APIRL_OK;
+  p->queue.n = (unsigned*)q;  // (owned from here on)
   p->queue.item = (uint2*)(q + 16);
   p->queue.list = (uint16_t*)(q + 16 + lors * sizeof(uint2));
-  c.img = b;
-  c.acc = b + n;
+  const size_t n = (size_t)c.floats;
+  size_t images = p->layouts == apirl::Layouts::kCalls ? 7 : 3;
+  if (apirl_status st = alloc_spare((void**)&c.img, images * n * sizeof(float))) return st;
+  if (!c.img && images > 3) {
+    images = 3;
+    if (apirl_status st = alloc_spare((void**)&c.img, images * n * sizeof(float))) return st;
+  }
+  if (!c.img) {
+    cudaFree(p->queue.n);
+    p->queue = apirl::ColQueue();
+    return APIRL_OK;
+  }
+  c.acc = c.img + n;
   p->cols = c;
-  p->col_sum[0].buf = b + 3 * n;
+  CK(cudaMemset(c.img, 0, images * n * sizeof(float)));
+  if (images == 3) return APIRL_OK;
+  p->col_sum[0].buf = c.img + 3 * n;
   CK(cudaEventCreateWithFlags(&p->col_sum[0].done, cudaEventDisableTiming));
   for (int k = 0; k < 2; k++) {
-    p->col_img[k].buf = b + (5 + k) * n;
+    p->col_img[k].buf = c.img + (5 + k) * n;
     CK(cudaEventCreateWithFlags(&p->col_img[k].done, cudaEventDisableTiming));
   }
   return APIRL_OK;
 }
 
-// The column layout of a sampled table, whose end points lie up to half a ring
-// beyond the rings': image copy and the two sums.  Without room for it the
-// passes walk bin by bin.
-void alloc_ray_cols(apirl_projector* p, const apirl::RayTables& rt) {
-  if (p->host.n_sinos < apirl::kColMinSinos || !apirl::col_rays_fit(p->g, rt.n_rs)) return;
-  apirl::ColBuffers c = apirl::col_layout(p->g, rt.zs.data(), (int)rt.zs.size());
-  if (!c.half) return;
+// The column layout of a sampled table, whose end points (zs) lie up to half a
+// ring beyond the rings': image copy and the two sums.  Without room for it
+// the passes walk bin by bin.
+apirl_status alloc_ray_cols(apirl_projector* p, int n_rs, const std::vector<float>& zs) {
+  if (p->layouts == apirl::Layouts::kPair || p->host.n_sinos < apirl::kColMinSinos || !apirl::col_rays_fit(p->g, n_rs))
+    return APIRL_OK;
+  apirl::ColBuffers c = apirl::col_layout(p->g, zs.data(), (int)zs.size());
+  if (!c.half) return APIRL_OK;
   const size_t bytes = 3 * (size_t)c.floats * sizeof(float);
-  cudaError_t e = cudaMalloc(&c.img, bytes);
-  if (e == cudaSuccess && (e = cudaMemset(c.img, 0, bytes)) != cudaSuccess) cudaFree(c.img);
-  if (e != cudaSuccess) {
-    (void)cudaGetLastError();  // handled here
-    return;
-  }
+  if (apirl_status st = alloc_spare((void**)&c.img, bytes)) return st;
+  if (!c.img) return APIRL_OK;
   c.acc = c.img + c.floats;
   p->ray_cols = c;
+  CK(cudaMemset(c.img, 0, bytes));
+  return APIRL_OK;
 }
 
 apirl_status finish_create(apirl_projector* p, apirl_projector** out) {
@@ -334,16 +350,18 @@ apirl_status finish_create(apirl_projector* p, apirl_projector** out) {
   }
   // (Images of several slices, of which a 2D pass projects the first and updates
   // all, keep to the unpadded pass.)
-  if (!p->is3d && p->g.nz == 1 && apirl::planar_lim(p->g) && (int64_t)p->t.n_proj * p->t.n_r <= INT_MAX - 31) {
+  if (!p->is3d && p->layouts != apirl::Layouts::kPair && p->g.nz == 1 && apirl::planar_lim(p->g) && (int64_t)p->t.n_proj * p->t.n_r <= INT_MAX - 31) {
     apirl::PlanarBuffers& pl = p->planar;
     const size_t lim = apirl::planar_lim(p->g);
     constexpr int copies = apirl::kPlanarCopies;
-    CK(cudaMalloc(&pl.img, 2 * (1 + copies) * lim * sizeof(float)));
-    CK(cudaMemset(pl.img, 0, 2 * (1 + copies) * lim * sizeof(float)));
-    pl.imgT = pl.img + lim;
-    pl.sum = pl.imgT + lim;
-    pl.sumT = pl.sum + copies * lim;
-    pl.lim = (unsigned)lim;
+    if (apirl_status st = alloc_spare((void**)&pl.img, 2 * (1 + copies) * lim * sizeof(float))) return st;
+    if (pl.img) {
+      CK(cudaMemset(pl.img, 0, 2 * (1 + copies) * lim * sizeof(float)));
+      pl.imgT = pl.img + lim;
+      pl.sum = pl.imgT + lim;
+      pl.sumT = pl.sum + copies * lim;
+      pl.lim = (unsigned)lim;
+    }
   }
   if (apirl_status st = settled()) return st;
   *out = p;
@@ -404,6 +422,53 @@ apirl_status setup_3d(const apirl_image_geom* img, const apirl_sino3d_geom* sino
 }
 }  // namespace apirl
 
+namespace apirl {
+apirl_status create_2d(const apirl_image_geom* img, const apirl_sino2d_geom* sino, int device, Layouts layouts,
+                       apirl_projector** out) {
+  if (!out) return fail(APIRL_ERR_INVALID, "null output pointer");
+  *out = nullptr;
+  if (!valid_img(img)) return fail(APIRL_ERR_INVALID, "invalid image geometry");
+  if (!sino || sino->n_proj <= 0 || sino->n_r <= 0 || !(sino->r_fov > 0) || !(sino->r_scanner > sino->r_fov))
+    return fail(APIRL_ERR_INVALID, "invalid 2D sinogram geometry (need n_proj, n_r > 0 and 0 < r_fov < r_scanner)");
+  if (!walk_bounded(img, sino->r_scanner, 0.f))
+    return fail(APIRL_ERR_INVALID, "voxels too small for the scanner radius (walks above 1e5 segments)");
+  DEVICE_SCOPE(device);
+  apirl_projector* p = new apirl_projector;
+  p->device = device;
+  p->layouts = layouts;
+  p->is3d = 0;
+  p->g = make_img_geom(img->nx, img->ny, img->nz, img->dx, img->dy, img->dz);
+  build_tables_2d(sino->n_proj, sino->n_r, sino->r_fov, sino->r_scanner, p->host);
+  p->t.n_proj = sino->n_proj;
+  p->t.n_r = sino->n_r;
+  p->t.n_sinos = 1;
+  p->t.is3d = 0;
+  apirl_status st = finish_create(p, out);
+  if (st != APIRL_OK) { std::string m = g_err; apirl_projector_destroy(p); g_err = m; }
+  return st;
+}
+
+apirl_status create_3d(const apirl_image_geom* img, const apirl_sino3d_geom* sino, int device, Layouts layouts,
+                       apirl_projector** out) {
+  if (!out) return fail(APIRL_ERR_INVALID, "null output pointer");
+  *out = nullptr;
+  apirl_projector* p = new apirl_projector;
+  apirl_status st = setup_3d(img, sino, p);
+  if (st != APIRL_OK) {
+    delete p;
+    return st;
+  }
+  {
+    DEVICE_SCOPE(device);
+    p->device = device;
+    p->layouts = layouts;
+    st = finish_create(p, out);
+  }
+  if (st != APIRL_OK) { std::string m = g_err; apirl_projector_destroy(p); g_err = m; }
+  return st;
+}
+}  // namespace apirl
+
 extern "C" {
 
 const char* apirl_last_error(void) { return g_err.c_str(); }
@@ -433,26 +498,7 @@ int apirl_sino3d_ring_z(const apirl_sino3d_geom* sino, float* h_z) {
 
 apirl_status apirl_projector_create_2d(const apirl_image_geom* img, const apirl_sino2d_geom* sino, int device,
                                        apirl_projector** out) {
-  if (!out) return fail(APIRL_ERR_INVALID, "null output pointer");
-  *out = nullptr;
-  if (!valid_img(img)) return fail(APIRL_ERR_INVALID, "invalid image geometry");
-  if (!sino || sino->n_proj <= 0 || sino->n_r <= 0 || !(sino->r_fov > 0) || !(sino->r_scanner > sino->r_fov))
-    return fail(APIRL_ERR_INVALID, "invalid 2D sinogram geometry (need n_proj, n_r > 0 and 0 < r_fov < r_scanner)");
-  if (!walk_bounded(img, sino->r_scanner, 0.f))
-    return fail(APIRL_ERR_INVALID, "voxels too small for the scanner radius (walks above 1e5 segments)");
-  DEVICE_SCOPE(device);
-  apirl_projector* p = new apirl_projector;
-  p->device = device;
-  p->is3d = 0;
-  p->g = apirl::make_img_geom(img->nx, img->ny, img->nz, img->dx, img->dy, img->dz);
-  apirl::build_tables_2d(sino->n_proj, sino->n_r, sino->r_fov, sino->r_scanner, p->host);
-  p->t.n_proj = sino->n_proj;
-  p->t.n_r = sino->n_r;
-  p->t.n_sinos = 1;
-  p->t.is3d = 0;
-  apirl_status st = finish_create(p, out);
-  if (st != APIRL_OK) { std::string m = g_err; apirl_projector_destroy(p); g_err = m; }
-  return st;
+  return apirl::create_2d(img, sino, device, apirl::Layouts::kCalls, out);
 }
 
 apirl_status apirl_mmr_lor_table(int n_proj, int n_r, float* h_lor) {
@@ -480,21 +526,7 @@ apirl_status apirl_projector_create_3d_mmr(const apirl_image_geom* img, int n_pr
 
 apirl_status apirl_projector_create_3d(const apirl_image_geom* img, const apirl_sino3d_geom* sino, int device,
                                        apirl_projector** out) {
-  if (!out) return fail(APIRL_ERR_INVALID, "null output pointer");
-  *out = nullptr;
-  apirl_projector* p = new apirl_projector;
-  apirl_status st = apirl::setup_3d(img, sino, p);
-  if (st != APIRL_OK) {
-    delete p;
-    return st;
-  }
-  {
-    DEVICE_SCOPE(device);
-    p->device = device;
-    st = finish_create(p, out);
-  }
-  if (st != APIRL_OK) { std::string m = g_err; apirl_projector_destroy(p); g_err = m; }
-  return st;
+  return apirl::create_3d(img, sino, device, apirl::Layouts::kCalls, out);
 }
 
 void apirl_projector_destroy(apirl_projector* p) {
@@ -619,13 +651,13 @@ apirl_status apirl_projector_set_sampling(apirl_projector* p, int n_samples, int
   p->n_samples = 1; p->n_axial_samples = 1; p->multi_lors = 0;
   if (plain) return APIRL_OK;
   LorTable* dst[2] = {&p->t, &p->t_dab};
+  std::vector<float> zs;  // the passes' end points
   for (int k = 0; k < 2; k++) {
     apirl::RayTables rt;
     if (!apirl::build_rays_3d(p->t.n_proj, p->t.n_r, p->n_rings, p->r_fov, p->axial_fov, p->r_scanner,
                               (int)p->min_rd.size(), p->min_rd.data(), p->max_rd.data(), n_samples, n_axial_samples,
                               multiple_lors_per_bin != 0, k == 1, rt))
       return fail(APIRL_ERR_INVALID, "a sampled ray end point is not finite (sample outside the scanner radius)");
-    if (k == 0) alloc_ray_cols(p, rt);
     if ((int)rt.zoff.size() != p->t.n_sinos + 1) return fail(APIRL_ERR_INVALID, "ring-pair table mismatch");
     CK(cudaMalloc(&p->d_lor_s[k], rt.lor.size() * sizeof(float)));
     CK(cudaMemcpy(p->d_lor_s[k], rt.lor.data(), rt.lor.size() * sizeof(float), cudaMemcpyHostToDevice));
@@ -633,7 +665,9 @@ apirl_status apirl_projector_set_sampling(apirl_projector* p, int n_samples, int
     CK(cudaMemcpy(p->d_zs[k], rt.zs.data(), rt.zs.size() * sizeof(float), cudaMemcpyHostToDevice));
     CK(cudaMalloc(&p->d_zoff[k], rt.zoff.size() * sizeof(int)));
     CK(cudaMemcpy(p->d_zoff[k], rt.zoff.data(), rt.zoff.size() * sizeof(int), cudaMemcpyHostToDevice));
+    if (k == 0) zs = std::move(rt.zs);
   }
+  if (apirl_status st = alloc_ray_cols(p, n_samples, zs)) return st;
   if (apirl_status st = settled()) return st;
   for (int k = 0; k < 2; k++) {
     dst[k]->lor_s = p->d_lor_s[k];
@@ -716,7 +750,7 @@ apirl_status apirl_divide_and_backproject(apirl_projector* p, const float* d_mea
   if (st) return st;
   if (!d_image || !d_meas || !d_est) return fail(APIRL_ERR_INVALID, "null image or sinogram");
   DEVICE_SCOPE(p->device);
-  if (use_cols(p) && !p->t_dab.lor_s) {
+  if (use_cols(p) && p->col_sum[0].buf && !p->t_dab.lor_s) {
     cudaStream_t s = (cudaStream_t)stream;
     bool captured = false;
     if ((st = capturing(s, &captured))) return st;

@@ -55,6 +55,24 @@ apirl_status set_err(apirl_status code, const char* what, cudaError_t e) {
     if (s_ != APIRL_OK) return s_;        \
   } while (0)
 
+// One run of a driver: the layouts its projector may keep, and whether its
+// passes have begun (all device memory is taken before).
+struct Run {
+  apirl::Layouts layouts;
+  bool passes = false;
+};
+// Runs a driver with the passes' own layouts and, where its memory does not
+// fit beside them, again without.
+template <class F>
+apirl_status with_room(F&& driver) {
+  Run run{apirl::Layouts::kPasses};
+  const apirl_status s = driver(run);
+  if (s != APIRL_ERR_OOM || run.passes) return s;
+  (void)cudaGetLastError();  // handled: not left for the next call
+  run.layouts = apirl::Layouts::kPair;
+  return driver(run);
+}
+
 // One EM pass (fused kernel + update) recorded into a graph on `st`.
 // d_zimg set: the sparse pass (apirl_em_pass_sparse) with that zero-count image.
 apirl_status capture_pass(Res& r, apirl_projector* p, const float* d_meas, const float* d_add, float* d_x, float* d_bp,
@@ -152,14 +170,14 @@ namespace {
 
 // h_sens_in: nsubsets given sensitivity images (or NULL: computed);
 // h_sens_out: receives the first n_sens_out of them.
-apirl_status osem_3d(const apirl_image_geom* img, const apirl_sino3d_geom* sino, const float* h_meas,
+apirl_status osem_3d(Run& run, const apirl_image_geom* img, const apirl_sino3d_geom* sino, const float* h_meas,
                      const float* h_mult, const float* h_add, const float* h_init, int iters, int nsubsets,
                      int device, float* h_out, double* h_lik, const float* h_sens_in, float* h_sens_out,
                      int n_sens_out, const apirl_sampling* sampling, int update_positive_sens = 0) {
   if (!h_meas || !h_init || !h_out || iters < 0 || nsubsets <= 0)
     return set_err(APIRL_ERR_INVALID, "apirl_osem_3d arguments", cudaSuccess);
   Res r;
-  DS(apirl_projector_create_3d(img, sino, device, &r.p));
+  DS(apirl::create_3d(img, sino, device, run.layouts, &r.p));
   if (sampling)
     DS(apirl_projector_set_sampling(r.p, sampling->n_samples, sampling->n_axial_samples,
                                     sampling->multiple_lors_per_bin));
@@ -225,6 +243,7 @@ apirl_status osem_3d(const apirl_image_geom* img, const apirl_sino3d_geom* sino,
     DS(capture_pass(r, p, d_meas, d_add, d_x, d_bp, d_sens + nv * s, nullptr, 0.f, update_positive_sens ? 0 : 1, s,
                     nsubsets, d_slot + s,
                     d_zimg ? d_zimg + nv * s : nullptr, d_zadd ? d_zadd + s : nullptr));
+  run.passes = true;
   std::vector<float> h_tmp;
   for (int t = 0; t < iters; t++) {
     for (int s = 0; s < nsubsets; s++) {
@@ -249,13 +268,13 @@ apirl_status osem_3d(const apirl_image_geom* img, const apirl_sino3d_geom* sino,
 }
 
 // h_sens_in: the given sensitivity image (or NULL: computed).
-apirl_status mlem_3d(const apirl_image_geom* img, const apirl_sino3d_geom* sino, const float* h_meas,
+apirl_status mlem_3d(Run& run, const apirl_image_geom* img, const apirl_sino3d_geom* sino, const float* h_meas,
                      const float* h_mult, const float* h_add, const float* h_init, int iters, int device,
                      float* h_out, double* h_lik, const float* h_sens_in, float* h_sens,
                      const apirl_sampling* sampling) {
   if (!h_meas || !h_init || !h_out || iters < 0) return set_err(APIRL_ERR_INVALID, "apirl_mlem_3d arguments", cudaSuccess);
   Res r;
-  DS(apirl_projector_create_3d(img, sino, device, &r.p));
+  DS(apirl::create_3d(img, sino, device, run.layouts, &r.p));
   if (sampling)
     DS(apirl_projector_set_sampling(r.p, sampling->n_samples, sampling->n_axial_samples,
                                     sampling->multiple_lors_per_bin));
@@ -311,6 +330,7 @@ apirl_status mlem_3d(const apirl_image_geom* img, const apirl_sino3d_geom* sino,
   }
   if (d_zimg) DS(apirl::prepare_nz_list(p, apirl_projector_num_bins(p, -1, 1)));
   DS(capture_pass(r, p, d_meas, d_add, d_x, d_bp, d_sens, d_thr, 0.f, 1, -1, 1, d_slot, d_zimg, d_zadd));
+  run.passes = true;
   std::vector<float> h_tmp;
   for (int t = 0; t < iters; t++) {
     DK(cudaGraphLaunch(r.execs[0], r.st));
@@ -400,8 +420,10 @@ extern "C" {
 apirl_status apirl_osem_3d(const apirl_image_geom* img, const apirl_sino3d_geom* sino, const float* h_meas,
                            const float* h_mult, const float* h_add, const float* h_init, int iters, int nsubsets,
                            int device, float* h_out, double* h_lik, float* h_sens0, const apirl_sampling* sampling) {
-  return osem_3d(img, sino, h_meas, h_mult, h_add, h_init, iters, nsubsets, device, h_out, h_lik, nullptr, h_sens0,
-                 1, sampling);
+  return with_room([&](Run& run) {
+    return osem_3d(run, img, sino, h_meas, h_mult, h_add, h_init, iters, nsubsets, device, h_out, h_lik, nullptr,
+                   h_sens0, 1, sampling);
+  });
 }
 
 apirl_status apirl_osem_3d_ex(const apirl_image_geom* img, const apirl_sino3d_geom* sino, const float* h_meas,
@@ -409,22 +431,29 @@ apirl_status apirl_osem_3d_ex(const apirl_image_geom* img, const apirl_sino3d_ge
                               int device, float* h_out, double* h_lik, const apirl_recon_options* opts) {
   const apirl_recon_options o = opts ? *opts : apirl_recon_options{nullptr, nullptr, nullptr, 0, 0};
   const int n_out = o.n_sens_out > 0 && o.n_sens_out < nsubsets ? o.n_sens_out : nsubsets;
-  return osem_3d(img, sino, h_meas, h_mult, h_add, h_init, iters, nsubsets, device, h_out, h_lik, o.h_sens_in,
-                 o.h_sens_out, n_out, o.sampling, o.update_positive_sens);
+  return with_room([&](Run& run) {
+    return osem_3d(run, img, sino, h_meas, h_mult, h_add, h_init, iters, nsubsets, device, h_out, h_lik, o.h_sens_in,
+                   o.h_sens_out, n_out, o.sampling, o.update_positive_sens);
+  });
 }
 
 apirl_status apirl_mlem_3d(const apirl_image_geom* img, const apirl_sino3d_geom* sino, const float* h_meas,
                            const float* h_mult, const float* h_add, const float* h_init, int iters, int device,
                            float* h_out, double* h_lik, float* h_sens, const apirl_sampling* sampling) {
-  return mlem_3d(img, sino, h_meas, h_mult, h_add, h_init, iters, device, h_out, h_lik, nullptr, h_sens, sampling);
+  return with_room([&](Run& run) {
+    return mlem_3d(run, img, sino, h_meas, h_mult, h_add, h_init, iters, device, h_out, h_lik, nullptr, h_sens,
+                   sampling);
+  });
 }
 
 apirl_status apirl_mlem_3d_ex(const apirl_image_geom* img, const apirl_sino3d_geom* sino, const float* h_meas,
                               const float* h_mult, const float* h_add, const float* h_init, int iters, int device,
                               float* h_out, double* h_lik, const apirl_recon_options* opts) {
   const apirl_recon_options o = opts ? *opts : apirl_recon_options{nullptr, nullptr, nullptr, 0, 0};
-  return mlem_3d(img, sino, h_meas, h_mult, h_add, h_init, iters, device, h_out, h_lik, o.h_sens_in, o.h_sens_out,
-                 o.sampling);
+  return with_room([&](Run& run) {
+    return mlem_3d(run, img, sino, h_meas, h_mult, h_add, h_init, iters, device, h_out, h_lik, o.h_sens_in,
+                   o.h_sens_out, o.sampling);
+  });
 }
 
 apirl_status apirl_mlem_2d(const apirl_image_geom* img, const apirl_sino2d_geom* sino, const float* h_meas,

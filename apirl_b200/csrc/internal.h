@@ -377,10 +377,20 @@ cudaError_t launch_sens_batch(const SensJob* d_jobs, int njobs, int64_t nblocks,
 
 typedef int apirl_status;
 struct apirl_image_geom;
+struct apirl_sino2d_geom;
 struct apirl_sino3d_geom;
 
 // Projector object behind the opaque apirl_projector handle.
+namespace apirl {
+// The layouts a projector keeps beside its tables and the padded pair: none;
+// those of the passes; and those of the calls that keep no other state in it
+// (ColSlot).  A layout that the device has no room for is left out, and what
+// it would have served runs as without it.
+enum class Layouts { kPair, kPasses, kCalls };
+}  // namespace apirl
+
 struct apirl_projector {
+  apirl::Layouts layouts = apirl::Layouts::kCalls;
   int device = 0;
   int is3d = 0;
   // The context's persisting-L2 limit before APIRL_OPT_L2_PERSIST raised it
@@ -461,6 +471,10 @@ namespace apirl {
 // The host half of apirl_projector_create_3d: geometry checks and host tables
 // into p (no device work; p->device and the device tables are not set).
 apirl_status setup_3d(const apirl_image_geom* img, const apirl_sino3d_geom* sino, apirl_projector* p);
+apirl_status create_2d(const apirl_image_geom* img, const apirl_sino2d_geom* sino, int device, Layouts layouts,
+                       apirl_projector** out);
+apirl_status create_3d(const apirl_image_geom* img, const apirl_sino3d_geom* sino, int device, Layouts layouts,
+                       apirl_projector** out);
 // Room in p->nz for the list of `total` bins (cudaMalloc: call outside graph
 // capture; a captured sparse pass without room walks every bin's chunk).
 apirl_status prepare_nz_list(apirl_projector* p, int64_t total);

@@ -77,3 +77,96 @@ st = lib.apirl_em_pass(P.h, D, 0, 0, None, D, D, D, None, 0.0, 0, -1, 1, D, S)
 done([st] + fake.log())''')
     cols = any("k_em_cols" in l for l in log[1:])
     assert cols == (nz == 65534 * 32) and not any(l.startswith("refused") and "k_col" in l for l in log[1:]), log
+
+
+ROOM = GEOMS + '''
+G = Sino3DGeom.span1(64, 90, 20, 140.0, 40.0, 200.0, 1)   # enough bins for a projection on the columns
+def em(P):
+    fake.clear()
+    _lib.check(lib.apirl_em_pass(P.h, D, 0, 0, None, D, D, D, None, 0.0, 0, -1, 1, None, S))
+    return [k for k in ("k_em_cols_rays", "k_em_cols", "k_em_pass_rays", "k_em_pass_persist", "k_planar_pass",
+                        "k_em_pass") if any(k in n for n in fake.launches())][0]
+def project(P):
+    fake.clear()
+    _lib.check(lib.apirl_project(P.h, D, D, -1, 1, S))
+    return [k for k in ("k_project_cols", "k_project") if any(k in n for n in fake.launches())][0]
+def under_limits(make, look):
+    P = make(); full = fake.used(); seen = [look(P)]; P.close()
+    for k in range(1, 60):
+        fake.limit(full - full * k // 60)
+        try:
+            P = make()
+        except _lib.ApirlError as e:
+            state = ["oom" if e.code == _lib.APIRL_ERR_OOM else str(e)]
+            assert fake.used() == 0
+            lib.apirl_projector_num_bins(None, 0, 1)
+            _g.cudaGetLastError()
+        else:
+            state = look(P)
+            P.close()
+        assert fake.used() == 0
+        if state != seen[-1]: seen.append(state)
+    return seen
+'''
+
+
+def test_projectors_without_room_for_the_columns(gpu):
+    """Creation takes what fits: all column images, those of the passes, none; each serves every call."""
+    seen = gpu(ROOM + '''
+done(under_limits(lambda: ap.SiddonProjector(ImageGeom(64, 64, 39, 2.0, 2.0, 1.0), G), lambda P: [em(P), project(P)]))''')
+    assert seen == [["k_em_cols", "k_project_cols"], ["k_em_cols", "k_project"], ["k_em_pass_persist", "k_project"], ["oom"]]
+
+
+def test_sampled_projectors_without_room_for_the_columns(gpu):
+    """set_sampling makes its tables first: what fitted without a column layout still does."""
+    seen = gpu(ROOM + '''
+def make():
+    P = ap.SiddonProjector(ImageGeom(64, 64, 39, 2.0, 2.0, 1.0), G)
+    try:
+        P.set_sampling(4, 4)
+    except Exception:
+        P.close()
+        raise
+    return P
+done(under_limits(make, lambda P: [em(P)]))''')
+    assert [s[0] for s in seen if s[0] != "oom"][0] == "k_em_cols_rays"
+    assert ["k_em_pass_rays"] in seen and seen[-1] == ["oom"]
+
+
+def test_2d_projectors_without_room_for_the_padded_layouts(gpu):
+    seen = gpu(ROOM + '''
+done(under_limits(lambda: ap.SiddonProjector(ImageGeom(256, 256, 1, 2.0, 2.0, 1.0), Sino2DGeom(16, 40, 256.0, 400.0)),
+                  lambda P: [em(P)]))''')
+    assert seen == [["k_planar_pass"], ["k_em_pass"], ["oom"]]
+
+
+@pytest.mark.parametrize("iters", [1, 4])
+def test_reconstructions_without_room_for_the_columns(gpu, iters):
+    """A whole reconstruction whose buffers do not fit beside the columns runs on the padded pair."""
+    seen = gpu(ROOM + f'''
+ig, sg = ImageGeom(64, 64, 39, 2.0, 2.0, 1.0), G
+m, x = np.ones(sg.n_bins, np.float32), np.ones(ig.n_voxels, np.float32)
+a = np.full(sg.n_bins, 0.5, np.float32)
+peak = 1 << 40
+def run(limit):
+    fake.limit(limit); fake.clear()
+    try:
+        ap.osem_3d(ig, sg, m, x, {iters}, 4, add=a)
+    except _lib.ApirlError as e:
+        _g.cudaGetLastError()
+        return "oom" if e.code == _lib.APIRL_ERR_OOM else str(e)
+    finally:
+        assert fake.used() == 0
+    return "cols" if any("k_em_cols" in n for n in fake.launches()) else "pair"
+# device bytes by bisection: the least room the run takes on the columns, on the pair
+def least(ok):
+    lo, hi = 0, 1 << 32
+    while hi - lo > 1024:
+        mid = (lo + hi) // 2
+        lo, hi = (lo, mid) if run(mid) in ok else (mid, hi)
+    return hi
+cols, pair = least(["cols"]), least(["cols", "pair"])
+done([run(1 << 40), cols, pair, run(cols - 2048), run(pair - 2048)])''')
+    assert seen[0] == "cols" and seen[3:] == ["pair", "oom"]
+    # the difference is the three column images (and the queue), no more
+    assert seen[1] > seen[2]
