@@ -351,7 +351,11 @@ apirl_status mlem_2d(const apirl_image_geom* img, const apirl_sino2d_geom* sino,
                      float* h_out, double* h_lik, const float* h_sens_in, float* h_sens) {
   if (!h_meas || !h_init || !h_out || iters < 0) return set_err(APIRL_ERR_INVALID, "apirl_mlem_2d arguments", cudaSuccess);
   Res r;
-  DS(apirl_projector_create_2d(img, sino, device, &r.p));
+  // The passes keep to the one unpadded sum: over 60 iterations the changed
+  // order of the float adds on the padded layouts (planar.cu) moved the FP64
+  // likelihoods by up to 1.4e-9 of their value, where runs of one form differ
+  // by 4e-10.  So the projector keeps no padded layouts either.
+  DS(apirl::create_2d(img, sino, device, apirl::Layouts::kPair, &r.p));
   int prev = 0;
   cudaGetDevice(&prev);
   DK(cudaSetDevice(device));
@@ -379,11 +383,6 @@ apirl_status mlem_2d(const apirl_image_geom* img, const apirl_sino2d_geom* sino,
   DK(cudaMemsetAsync(d_sens, 0, nv * sizeof(float), r.st));
   SubsetSel all;
   all.subset = -1; all.nsub = 1; all.nk = sino->n_proj;
-  // The passes keep to the one unpadded sum: over 60 iterations the changed
-  // order of the float adds on the padded layouts (planar.cu) moved the FP64
-  // likelihoods by up to 1.4e-9 of their value, where runs of one form differ
-  // by 4e-10.
-  p->planar.lim = 0;
   // Sensitivity A^T (mult or 1), or the given image (Mlem2d.cpp:95-112).
   if (h_sens_in)
     DK(cudaMemcpyAsync(d_sens, h_sens_in, nv * sizeof(float), cudaMemcpyHostToDevice, r.st));

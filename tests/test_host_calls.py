@@ -170,3 +170,12 @@ done([run(1 << 40), cols, pair, run(cols - 2048), run(pair - 2048)])''')
     assert seen[0] == "cols" and seen[3:] == ["pair", "oom"]
     # the difference is the three column images (and the queue), no more
     assert seen[1] > seen[2]
+
+
+def test_2d_reconstructions_keep_no_layouts_they_do_not_walk(gpu):
+    log = gpu('''
+ig, sg = ImageGeom(128, 128, 1, 2.0, 2.0, 1.0), Sino2DGeom(16, 40, 128.0, 400.0)
+ap.mlem_2d(ig, sg, np.ones(sg.n_bins, np.float32), np.ones(ig.n_voxels, np.float32), 2)
+done(fake.log())''')
+    assert not any("k_planar" in l for l in log)
+    assert not any(l == f"malloc legacy {6 * 132 * 132 * 4}" for l in log) and "memset legacy " not in log, log
