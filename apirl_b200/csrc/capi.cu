@@ -228,140 +228,124 @@ apirl_status settled() {
   return APIRL_OK;
 }
 
-// The padded two-layout buffers of the fused 3D pass, allocated with the
-// projector so that no pass allocates (passes may be captured into CUDA
-// graphs).  Volumes whose padded size does not fit a 32-bit index keep the
-// single unpadded layout.
-apirl_status alloc_pad(apirl_projector* p) {
-  if (p->pad.pA) return APIRL_OK;
-  const int64_t pv = (int64_t)(p->g.nx + 2 * apirl::kPad) * (p->g.ny + 2 * apirl::kPad) * (p->g.nz + 2 * apirl::kPad);
-  if (pv > INT_MAX) return APIRL_OK;
-  // One block for the four images (an L2 access policy window can then
-  // cover them all: APIRL_OPT_L2_PERSIST).
-  float* b = nullptr;
-  cudaError_t e = cudaMalloc(&b, 4 * pv * sizeof(float));
-  if (e == cudaSuccess) e = cudaMemset(b, 0, 4 * pv * sizeof(float));
-  if (e != cudaSuccess) {
-    cudaFree(b);
-    return cuda_fail(e, "padded layout buffers");
+// Places in a device block that is sized before it is taken: a fresh mapping
+// costs about 0.35 ms (0.28 ms to free), whatever its size, so a projector's
+// buffers share one.
+struct Places {
+  size_t bytes = 0;
+  size_t add(size_t n) {
+    const size_t at = bytes;
+    bytes += (n + 511) / 512 * 512;
+    return at;
   }
-  p->pad.pA = b;
-  p->pad.pT = b + pv;
-  p->pad.bA = b + 2 * pv;
-  p->pad.bT = b + 3 * pv;
-  p->pad.lim = (unsigned)pv;
-  return APIRL_OK;
+};
+
+// The block of places() with the layouts that fit: those asked for, else
+// fewer.  *out stays null where not even the last does (APIRL_ERR_OOM).
+template <class F>
+apirl_status take_block(apirl::Layouts& layouts, char** out, F&& places) {
+  for (;;) {
+    const cudaError_t e = cudaMalloc((void**)out, places(layouts).bytes);
+    if (e == cudaSuccess) return APIRL_OK;
+    *out = nullptr;
+    if (e != cudaErrorMemoryAllocation || layouts == apirl::Layouts::kPair) return cuda_fail(e, "projector buffers");
+    (void)cudaGetLastError();  // handled: not left for the next call
+    layouts = layouts == apirl::Layouts::kCalls ? apirl::Layouts::kPasses : apirl::Layouts::kPair;
+  }
 }
 
-// Device memory for a layout that the projector can do without: *out stays
-// null where there is no room for it.
-apirl_status alloc_spare(void** out, size_t bytes) {
-  const cudaError_t e = cudaMalloc(out, bytes);
-  if (e == cudaSuccess) return APIRL_OK;
-  *out = nullptr;
-  if (e != cudaErrorMemoryAllocation) return cuda_fail(e, "cudaMalloc");
-  (void)cudaGetLastError();  // handled: not left for the next call
-  return APIRL_OK;
-}
-
-// The column layout's buffers, one block: the passes' image copy and sums, and
-// the slots' (see apirl_projector::ColSlot).  All are made here, so that no
-// later call allocates; where they do not fit, without the slots, or none.
-apirl_status alloc_cols(apirl_projector* p) {
-  if (p->layouts == apirl::Layouts::kPair || p->cols.half || p->host.n_sinos < apirl::kColMinSinos) return APIRL_OK;
-  apirl::ColBuffers c = apirl::col_layout(p->g, p->host.z.data(), (int)p->host.z.size());
-  if (!c.half) return APIRL_OK;
-  // The queue: its length, items and lists, one block.
-  const size_t lors = (size_t)p->t.n_proj * p->t.n_r;
-  char* q = nullptr;
-  if (apirl_status st = alloc_spare((void**)&q, 16 + lors * (sizeof(uint2) + apirl::kColFew * sizeof(uint16_t)))) return st;
-  if (!q) return APIRL_OK;
-  p->queue.n = (unsigned*)q;  // (owned from here on)
-  p->queue.item = (uint2*)(q + 16);
-  p->queue.list = (uint16_t*)(q + 16 + lors * sizeof(uint2));
-  const size_t n = (size_t)c.floats;
-  size_t images = p->layouts == apirl::Layouts::kCalls ? 7 : 3;
-  if (apirl_status st = alloc_spare((void**)&c.img, images * n * sizeof(float))) return st;
-  if (!c.img && images > 3) {
-    images = 3;
-    if (apirl_status st = alloc_spare((void**)&c.img, images * n * sizeof(float))) return st;
-  }
-  if (!c.img) {
-    cudaFree(p->queue.n);
-    p->queue = apirl::ColQueue();
-    return APIRL_OK;
-  }
-  c.acc = c.img + n;
-  p->cols = c;
-  CK(cudaMemset(c.img, 0, images * n * sizeof(float)));
-  if (images == 3) return APIRL_OK;
-  p->col_sum[0].buf = c.img + 3 * n;
-  CK(cudaEventCreateWithFlags(&p->col_sum[0].done, cudaEventDisableTiming));
-  for (int k = 0; k < 2; k++) {
-    p->col_img[k].buf = c.img + (5 + k) * n;
-    CK(cudaEventCreateWithFlags(&p->col_img[k].done, cudaEventDisableTiming));
-  }
-  return APIRL_OK;
-}
-
-// The column layout of a sampled table, whose end points (zs) lie up to half a
-// ring beyond the rings': image copy and the two sums.  Without room for it
-// the passes walk bin by bin.
-apirl_status alloc_ray_cols(apirl_projector* p, int n_rs, const std::vector<float>& zs) {
-  if (p->layouts == apirl::Layouts::kPair || p->host.n_sinos < apirl::kColMinSinos || !apirl::col_rays_fit(p->g, n_rs))
-    return APIRL_OK;
-  apirl::ColBuffers c = apirl::col_layout(p->g, zs.data(), (int)zs.size());
-  if (!c.half) return APIRL_OK;
-  const size_t bytes = 3 * (size_t)c.floats * sizeof(float);
-  if (apirl_status st = alloc_spare((void**)&c.img, bytes)) return st;
-  if (!c.img) return APIRL_OK;
-  c.acc = c.img + c.floats;
-  p->ray_cols = c;
-  CK(cudaMemset(c.img, 0, bytes));
-  return APIRL_OK;
-}
-
+// The projector's device block: tables and scratch; in 3D the padded
+// two-layout buffers of the fused pass (volumes whose padded size does not fit
+// a 32-bit index keep the single unpadded layout), with kPasses the column
+// layout's image copy, sums and queue, with kCalls the slots'
+// (apirl_projector::ColSlot) too; in 2D the padded slices.  All are made here,
+// so that no later call allocates (passes may be captured into CUDA graphs).
 apirl_status finish_create(apirl_projector* p, apirl_projector** out) {
-  const size_t nl = p->host.lor.size() / 4;
-  CK(cudaMalloc(&p->d_lor, nl * sizeof(float4)));
-  CK(cudaMemcpy(p->d_lor, p->host.lor.data(), nl * sizeof(float4), cudaMemcpyHostToDevice));
-  CK(cudaMalloc(&p->d_z, p->host.z.size() / 2 * sizeof(float2)));
-  CK(cudaMemcpy(p->d_z, p->host.z.data(), p->host.z.size() * sizeof(float), cudaMemcpyHostToDevice));
-  CK(cudaMalloc(&p->d_ok, p->host.ok.size()));
-  CK(cudaMemcpy(p->d_ok, p->host.ok.data(), p->host.ok.size(), cudaMemcpyHostToDevice));
-  p->t.lor = p->d_lor;
-  p->t.z = p->d_z;
-  p->t.ok = p->d_ok;
   SubsetSel all = make_subset(p, -1, 1);
   p->n_partials = apirl::em_pass_blocks(p->t, all);
   const int64_t cp = apirl::col_partials(p->t, all) + apirl::col_dots(p->g);
   if (cp > p->n_partials) p->n_partials = cp;
   const int64_t lb = apirl::likelihood_blocks((int64_t)p->t.n_sinos * p->t.n_proj * p->t.n_r);
   if (lb > p->n_partials) p->n_partials = lb;
-  CK(cudaMalloc(&p->d_partials, p->n_partials * sizeof(double)));
-  CK(cudaMalloc(&p->d_minmax, 2 * sizeof(unsigned)));
-  CK(cudaMalloc(&p->d_scalars, 8 * sizeof(double)));
-  CK(cudaMalloc(&p->d_chunk, sizeof(unsigned long long)));
-  if (p->is3d) CK(apirl::prepare_em_kernels(p->em_block));
-  if (p->is3d && p->dual_layout) {
-    apirl_status st = alloc_pad(p);
-    if (!st) st = alloc_cols(p);
-    if (st) return st;
-  }
+  const int64_t pv64 = (int64_t)(p->g.nx + 2 * apirl::kPad) * (p->g.ny + 2 * apirl::kPad) * (p->g.nz + 2 * apirl::kPad);
+  const size_t pv = p->is3d && pv64 <= INT_MAX ? (size_t)pv64 : 0;
+  apirl::ColBuffers c;
+  if (p->is3d && p->host.n_sinos >= apirl::kColMinSinos)
+    c = apirl::col_layout(p->g, p->host.z.data(), (int)p->host.z.size());
+  const size_t n = c.half ? (size_t)c.floats : 0, lors = (size_t)p->t.n_proj * p->t.n_r;
   // (Images of several slices, of which a 2D pass projects the first and updates
   // all, keep to the unpadded pass.)
-  if (!p->is3d && p->layouts != apirl::Layouts::kPair && p->g.nz == 1 && apirl::planar_lim(p->g) && (int64_t)p->t.n_proj * p->t.n_r <= INT_MAX - 31) {
-    apirl::PlanarBuffers& pl = p->planar;
-    const size_t lim = apirl::planar_lim(p->g);
-    constexpr int copies = apirl::kPlanarCopies;
-    if (apirl_status st = alloc_spare((void**)&pl.img, 2 * (1 + copies) * lim * sizeof(float))) return st;
-    if (pl.img) {
-      CK(cudaMemset(pl.img, 0, 2 * (1 + copies) * lim * sizeof(float)));
-      pl.imgT = pl.img + lim;
-      pl.sum = pl.imgT + lim;
-      pl.sumT = pl.sum + copies * lim;
-      pl.lim = (unsigned)lim;
+  const size_t lim = !p->is3d && p->g.nz == 1 && (int64_t)lors <= INT_MAX - 31 ? apirl::planar_lim(p->g) : 0;
+  constexpr size_t copies = apirl::kPlanarCopies;
+  size_t at_lor, at_z, at_ok, at_partials, at_minmax, at_scalars, at_chunk, at_item, at_list, at_zeros, at_pad, at_col, at_planar;
+  auto places = [&](apirl::Layouts l) {
+    const bool more = l != apirl::Layouts::kPair;
+    Places b;
+    at_lor = b.add(p->host.lor.size() * sizeof(float));
+    at_z = b.add(p->host.z.size() * sizeof(float));
+    at_ok = b.add(p->host.ok.size());
+    at_partials = b.add(p->n_partials * sizeof(double));
+    at_minmax = b.add(2 * sizeof(unsigned));
+    at_scalars = b.add(8 * sizeof(double));
+    at_chunk = b.add(sizeof(unsigned long long) + sizeof(unsigned));  // and the queue's length
+    at_item = b.add(more && n ? lors * sizeof(uint2) : 0);
+    at_list = b.add(more && n ? lors * apirl::kColFew * sizeof(uint16_t) : 0);
+    at_zeros = b.bytes;
+    at_pad = b.add(4 * pv * sizeof(float));
+    at_col = b.add((l == apirl::Layouts::kCalls ? 7 : more ? 3 : 0) * n * sizeof(float));
+    at_planar = b.add(more ? 2 * (1 + copies) * lim * sizeof(float) : 0);
+    return b;
+  };
+  if (apirl_status st = take_block(p->layouts, &p->block, places)) return st;
+  char* const b = p->block;
+  const size_t zeros = places(p->layouts).bytes - at_zeros;
+  p->d_lor = (float4*)(b + at_lor);
+  CK(cudaMemcpy(p->d_lor, p->host.lor.data(), p->host.lor.size() * sizeof(float), cudaMemcpyHostToDevice));
+  p->d_z = (float2*)(b + at_z);
+  CK(cudaMemcpy(p->d_z, p->host.z.data(), p->host.z.size() * sizeof(float), cudaMemcpyHostToDevice));
+  p->d_ok = (uint8_t*)(b + at_ok);
+  CK(cudaMemcpy(p->d_ok, p->host.ok.data(), p->host.ok.size(), cudaMemcpyHostToDevice));
+  p->t.lor = p->d_lor;
+  p->t.z = p->d_z;
+  p->t.ok = p->d_ok;
+  p->d_partials = (double*)(b + at_partials);
+  p->d_minmax = (unsigned*)(b + at_minmax);
+  p->d_scalars = (double*)(b + at_scalars);
+  p->d_chunk = (unsigned long long*)(b + at_chunk);
+  if (zeros) CK(cudaMemset(b + at_zeros, 0, zeros));
+  if (p->is3d) CK(apirl::prepare_em_kernels(p->em_block));
+  if (pv) {
+    // The four images side by side: an L2 access policy window can cover them
+    // all (APIRL_OPT_L2_PERSIST).
+    p->pad.pA = (float*)(b + at_pad);
+    p->pad.pT = p->pad.pA + pv;
+    p->pad.bA = p->pad.pA + 2 * pv;
+    p->pad.bT = p->pad.pA + 3 * pv;
+    p->pad.lim = (unsigned)pv;
+  }
+  if (n && p->layouts != apirl::Layouts::kPair) {
+    c.img = (float*)(b + at_col);
+    c.acc = c.img + n;
+    p->cols = c;
+    p->queue.n = (unsigned*)(p->d_chunk + 1);
+    p->queue.item = (uint2*)(b + at_item);
+    p->queue.list = (uint16_t*)(b + at_list);
+  }
+  if (n && p->layouts == apirl::Layouts::kCalls) {
+    p->col_sum[0].buf = c.img + 3 * n;
+    CK(cudaEventCreateWithFlags(&p->col_sum[0].done, cudaEventDisableTiming));
+    for (int k = 0; k < 2; k++) {
+      p->col_img[k].buf = c.img + (5 + k) * n;
+      CK(cudaEventCreateWithFlags(&p->col_img[k].done, cudaEventDisableTiming));
     }
+  }
+  if (lim && p->layouts != apirl::Layouts::kPair) {
+    apirl::PlanarBuffers& pl = p->planar;
+    pl.img = (float*)(b + at_planar);
+    pl.imgT = pl.img + lim;
+    pl.sum = pl.imgT + lim;
+    pl.sumT = pl.sum + copies * lim;
+    pl.lim = (unsigned)lim;
   }
   if (apirl_status st = settled()) return st;
   *out = p;
@@ -533,13 +517,8 @@ void apirl_projector_destroy(apirl_projector* p) {
   if (!p) return;
   DeviceScope scope(p->device);
   if (p->l2_limit_set) cudaDeviceSetLimit(cudaLimitPersistingL2CacheSize, p->l2_limit_prev);
-  cudaFree(p->d_lor);
-  cudaFree(p->d_z);
-  cudaFree(p->d_ok);
-  cudaFree(p->d_partials);
-  cudaFree(p->d_minmax);
-  cudaFree(p->d_scalars);
-  cudaFree(p->d_chunk);
+  cudaFree(p->block);
+  cudaFree(p->ray_block);
   cudaFree(p->pad2.bA);
   cudaFree(p->pad2.bT);
   cudaFree(p->nz.list);
@@ -547,20 +526,10 @@ void apirl_projector_destroy(apirl_projector* p) {
   cudaFree(p->nz.n_list);
   cudaFree(p->d_lor64);
   cudaFree(p->d_z64);
-  for (int k = 0; k < 2; k++) {
-    cudaFree(p->d_lor_s[k]);
-    cudaFree(p->d_zs[k]);
-    cudaFree(p->d_zoff[k]);
-  }
-  cudaFree(p->cols.img);  // the block of all column buffers
-  cudaFree(p->ray_cols.img);
-  cudaFree(p->queue.n);
-  cudaFree(p->planar.img);
   for (auto& c : p->col_img)
     if (c.done) cudaEventDestroy(c.done);
   for (auto& c : p->col_sum)
     if (c.done) cudaEventDestroy(c.done);
-  cudaFree(p->pad.pA);  // the block of all four padded images
   cudaFree(p->pad.eA);
   cudaFree(p->pad.eT);
   if (p->ev0) cudaEventDestroy(p->ev0);
@@ -636,43 +605,58 @@ apirl_status apirl_projector_set_sampling(apirl_projector* p, int n_samples, int
     return fail(APIRL_ERR_INVALID, "oversampling needs at least 2 radial bins (getDeltaR)");
   DEVICE_SCOPE(p->device);
   // Drop any previous sampled tables.
-  for (int k = 0; k < 2; k++) {
-    cudaFree(p->d_lor_s[k]);
-    cudaFree(p->d_zs[k]);
-    cudaFree(p->d_zoff[k]);
-    p->d_lor_s[k] = nullptr;
-    p->d_zs[k] = nullptr;
-    p->d_zoff[k] = nullptr;
-  }
-  cudaFree(p->ray_cols.img);
+  cudaFree(p->ray_block);
+  p->ray_block = nullptr;
   p->ray_cols = apirl::ColBuffers();
   p->t.lor_s = nullptr; p->t.zs = nullptr; p->t.zoff = nullptr; p->t.n_rs = 1; p->t.n_as = 1;
   p->t_dab = p->t;
   p->n_samples = 1; p->n_axial_samples = 1; p->multi_lors = 0;
   if (plain) return APIRL_OK;
   LorTable* dst[2] = {&p->t, &p->t_dab};
-  std::vector<float> zs;  // the passes' end points
+  apirl::RayTables rt[2];
   for (int k = 0; k < 2; k++) {
-    apirl::RayTables rt;
     if (!apirl::build_rays_3d(p->t.n_proj, p->t.n_r, p->n_rings, p->r_fov, p->axial_fov, p->r_scanner,
                               (int)p->min_rd.size(), p->min_rd.data(), p->max_rd.data(), n_samples, n_axial_samples,
-                              multiple_lors_per_bin != 0, k == 1, rt))
+                              multiple_lors_per_bin != 0, k == 1, rt[k]))
       return fail(APIRL_ERR_INVALID, "a sampled ray end point is not finite (sample outside the scanner radius)");
-    if ((int)rt.zoff.size() != p->t.n_sinos + 1) return fail(APIRL_ERR_INVALID, "ring-pair table mismatch");
-    CK(cudaMalloc(&p->d_lor_s[k], rt.lor.size() * sizeof(float)));
-    CK(cudaMemcpy(p->d_lor_s[k], rt.lor.data(), rt.lor.size() * sizeof(float), cudaMemcpyHostToDevice));
-    CK(cudaMalloc(&p->d_zs[k], rt.zs.size() * sizeof(float)));
-    CK(cudaMemcpy(p->d_zs[k], rt.zs.data(), rt.zs.size() * sizeof(float), cudaMemcpyHostToDevice));
-    CK(cudaMalloc(&p->d_zoff[k], rt.zoff.size() * sizeof(int)));
-    CK(cudaMemcpy(p->d_zoff[k], rt.zoff.data(), rt.zoff.size() * sizeof(int), cudaMemcpyHostToDevice));
-    if (k == 0) zs = std::move(rt.zs);
+    if ((int)rt[k].zoff.size() != p->t.n_sinos + 1) return fail(APIRL_ERR_INVALID, "ring-pair table mismatch");
   }
-  if (apirl_status st = alloc_ray_cols(p, n_samples, zs)) return st;
+  // One block: the tables, and the column layout of the passes (image copy and
+  // two sums), whose end points lie up to half a ring beyond the rings'.
+  // Without room for it, or for so many lists, the passes walk bin by bin.
+  apirl::ColBuffers c;
+  if (p->host.n_sinos >= apirl::kColMinSinos && apirl::col_rays_fit(p->g, n_samples))
+    c = apirl::col_layout(p->g, rt[0].zs.data(), (int)rt[0].zs.size());
+  apirl::Layouts layouts = p->layouts == apirl::Layouts::kPair || !c.half ? apirl::Layouts::kPair : apirl::Layouts::kPasses;
+  size_t at_lor[2], at_zs[2], at_zoff[2], at_col;
+  if (apirl_status st = take_block(layouts, &p->ray_block, [&](apirl::Layouts l) {
+        Places b;
+        for (int k = 0; k < 2; k++) {
+          at_lor[k] = b.add(rt[k].lor.size() * sizeof(float));
+          at_zs[k] = b.add(rt[k].zs.size() * sizeof(float));
+          at_zoff[k] = b.add(rt[k].zoff.size() * sizeof(int));
+        }
+        at_col = b.add(l == apirl::Layouts::kPair ? 0 : 3 * (size_t)c.floats * sizeof(float));
+        return b;
+      }))
+    return st;
+  for (int k = 0; k < 2; k++) {
+    char* const b = p->ray_block;
+    CK(cudaMemcpy(b + at_lor[k], rt[k].lor.data(), rt[k].lor.size() * sizeof(float), cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(b + at_zs[k], rt[k].zs.data(), rt[k].zs.size() * sizeof(float), cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(b + at_zoff[k], rt[k].zoff.data(), rt[k].zoff.size() * sizeof(int), cudaMemcpyHostToDevice));
+  }
+  if (layouts != apirl::Layouts::kPair) {
+    c.img = (float*)(p->ray_block + at_col);
+    c.acc = c.img + c.floats;
+    CK(cudaMemset(c.img, 0, 3 * (size_t)c.floats * sizeof(float)));
+    p->ray_cols = c;
+  }
   if (apirl_status st = settled()) return st;
   for (int k = 0; k < 2; k++) {
-    dst[k]->lor_s = p->d_lor_s[k];
-    dst[k]->zs = p->d_zs[k];
-    dst[k]->zoff = p->d_zoff[k];
+    dst[k]->lor_s = (const float4*)(p->ray_block + at_lor[k]);
+    dst[k]->zs = (const float2*)(p->ray_block + at_zs[k]);
+    dst[k]->zoff = (const int*)(p->ray_block + at_zoff[k]);
     dst[k]->n_rs = n_samples;
     dst[k]->n_as = n_axial_samples;
   }
@@ -1040,15 +1024,7 @@ apirl_status apirl_em_project_backproject(apirl_projector* p, const void* d_coun
 apirl_status apirl_projector_set_option(apirl_projector* p, int option, int value) {
   if (!p) return fail(APIRL_ERR_INVALID, "null projector");
   switch (option) {
-    case APIRL_OPT_DUAL_LAYOUT: {
-      p->dual_layout = value != 0;
-      if (p->dual_layout && p->is3d) {
-        DEVICE_SCOPE(p->device);
-        const apirl_status st = alloc_pad(p);
-        return st ? st : settled();
-      }
-      return APIRL_OK;
-    }
+    case APIRL_OPT_DUAL_LAYOUT: p->dual_layout = value != 0; return APIRL_OK;
     case APIRL_OPT_KERNEL_TIMING: p->timing = value != 0; p->timed = 0; return APIRL_OK;
     case APIRL_OPT_PERSISTENT: p->persistent = value != 0; return APIRL_OK;
     case APIRL_OPT_SPARSE_IMAGE:

@@ -399,6 +399,7 @@ struct apirl_projector {
   size_t l2_limit_prev = 0;
   apirl::ImgGeom g{};
   apirl::HostTables host;
+  char* block = nullptr;         // the device memory of creation: what follows points into it
   float4* d_lor = nullptr;
   float2* d_z = nullptr;
   uint8_t* d_ok = nullptr;
@@ -456,9 +457,7 @@ struct apirl_projector {
   int scanner = 0;               // APIRL_SCANNER_CYLINDRICAL or APIRL_SCANNER_MMR
   int n_samples = 1, n_axial_samples = 1, multi_lors = 0;
   apirl::LorTable t_dab{};
-  float4* d_lor_s[2] = {nullptr, nullptr};
-  float2* d_zs[2] = {nullptr, nullptr};
-  int* d_zoff[2] = {nullptr, nullptr};
+  char* ray_block = nullptr;     // their tables and column layout
 };
 
 // Records `msg` as the calling thread's last error and returns `code`.

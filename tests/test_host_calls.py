@@ -179,3 +179,17 @@ ap.mlem_2d(ig, sg, np.ones(sg.n_bins, np.float32), np.ones(ig.n_voxels, np.float
 done(fake.log())''')
     assert not any("k_planar" in l for l in log)
     assert not any(l == f"malloc legacy {6 * 132 * 132 * 4}" for l in log) and "memset legacy " not in log, log
+
+
+def test_creation_takes_one_block(gpu):
+    """A fresh device mapping costs more than all else in creation: one for a projector, one for its sampled rays."""
+    counts = gpu(GEOMS + '''
+n = []
+def mallocs(make):
+    fake.clear()
+    P = make()
+    n.append(sum(l.startswith("malloc") for l in fake.log()))
+    return P
+P = mallocs(lambda: ap.SiddonProjector(*G3)); mallocs(lambda: P.set_sampling(2, 2)); mallocs(lambda: ap.SiddonProjector(*G2))
+done(n)''')
+    assert counts == [1, 1, 1]
