@@ -1,6 +1,7 @@
 // The C ABI declared in include/apirl_b200.h: projector objects, argument
 // checks, error reporting, and the MLEM / OSEM drivers.
 #include <cuda_runtime.h>
+#include <algorithm>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
@@ -277,7 +278,7 @@ apirl_status finish_create(apirl_projector* p, apirl_projector** out) {
   // all, keep to the unpadded pass.)
   const size_t lim = !p->is3d && p->g.nz == 1 && (int64_t)lors <= INT_MAX - 31 ? apirl::planar_lim(p->g) : 0;
   constexpr size_t copies = apirl::kPlanarCopies;
-  size_t at_lor, at_z, at_ok, at_partials, at_minmax, at_scalars, at_chunk, at_item, at_list, at_zeros, at_pad, at_col, at_planar;
+  size_t at_lor, at_z, at_ok, at_partials, at_minmax, at_scalars, at_chunk, at_item, at_list, at_bins, at_zeros, at_pad, at_col, at_planar;
   auto places = [&](apirl::Layouts l) {
     const bool more = l != apirl::Layouts::kPair;
     Places b;
@@ -287,9 +288,13 @@ apirl_status finish_create(apirl_projector* p, apirl_projector** out) {
     at_partials = b.add(p->n_partials * sizeof(double));
     at_minmax = b.add(2 * sizeof(unsigned));
     at_scalars = b.add(8 * sizeof(double));
-    at_chunk = b.add(sizeof(unsigned long long) + sizeof(unsigned));  // and the queue's length
-    at_item = b.add(more && n ? lors * sizeof(uint2) : 0);
-    at_list = b.add(more && n ? lors * apirl::kColFew * sizeof(uint16_t) : 0);
+    at_chunk = b.add(sizeof(unsigned long long) + 2 * sizeof(unsigned));  // and the queue's numbers
+    const bool queue = more && n;
+    const size_t deferred = std::min<size_t>(lors, apirl::kColDirectLors);
+    at_item = b.add(queue ? deferred * sizeof(uint2) : 0);
+    at_list = b.add(queue ? deferred * apirl::kColFew * sizeof(uint16_t) : 0);
+    const size_t direct = std::min(apirl::col_direct(p->host.n_sinos), p->host.n_sinos);
+    at_bins = b.add(queue && lors > apirl::kColDirectLors ? lors * direct * sizeof(unsigned) : 0);
     at_zeros = b.bytes;
     at_pad = b.add(4 * pv * sizeof(float));
     at_col = b.add((l == apirl::Layouts::kCalls ? 7 : more ? 3 : 0) * n * sizeof(float));
@@ -330,6 +335,7 @@ apirl_status finish_create(apirl_projector* p, apirl_projector** out) {
     p->queue.n = (unsigned*)(p->d_chunk + 1);
     p->queue.item = (uint2*)(b + at_item);
     p->queue.list = (uint16_t*)(b + at_list);
+    p->queue.bins = (unsigned*)(b + at_bins);
   }
   if (n && p->layouts == apirl::Layouts::kCalls) {
     p->col_sum[0].buf = c.img + 3 * n;

@@ -15,6 +15,7 @@
 // one), the scatters by the SM-to-L2 path: 5.1 sectors a reduction of 32 lanes
 // (the pair's rays along r: 10.3), 217 G sectors/s.
 #include <cuda_runtime.h>
+#include <climits>
 #include <cmath>
 #include <cstdint>
 #include "columns_em.cuh"
@@ -39,6 +40,11 @@ constexpr int kMaxWarps = kRaysBlock / 32;
 // Blocks of the LORs with few counts.
 constexpr int kColFewBlock = 64;
 constexpr int kColFewBlocks = 20;
+// Blocks of the bins walked one a lane (small, to spread few of them), and
+// their loads in flight.
+constexpr int kColDirectBlock = 64;
+constexpr int kColDirectBlocks = 16;
+constexpr int kColDirectU = 8;
 // Blocks of the batched pass, whose LORs have from a few to hundreds of
 // counts: ten mixed jobs of 64 - 128 x 1 - 41 slices in 16.7 ms, against 18.0 /
 // 17.6 / 17.8 / 20.4 ms with 64 / 96 / 160 / 256 threads and 18.1 ms at 8 blocks
@@ -208,12 +214,13 @@ __global__ void __launch_bounds__(kRaysBlock, kRaysBlocks) k_em_cols_rays(
 // sinograms with counts and its warps take 32 of them at a time.  skip_zero
 // as lik_term.  A LOR with at most `few` (<= kColFew) counts would leave most
 // of the block's warps idle: it goes to the queue with its list, for the small
-// blocks of k_em_cols_few.
+// blocks of k_em_cols_few; or with at most `direct` its bins go there, for
+// k_em_cols_direct.
 template <typename CT>
 __global__ void __launch_bounds__(kColBlock, kColBlocks) k_em_cols_listed(
     ImgGeom g, ColDims d, LorTable t, SubsetSel s, const CT* __restrict__ counts, int counts_packed,
     const float* __restrict__ add, const float* __restrict__ img, float* __restrict__ acc, int back,
-    double* __restrict__ partials, int skip_zero, int few, ColQueue queue) {
+    double* __restrict__ partials, int skip_zero, int few, int direct, ColQueue queue) {
   __shared__ ColActive act;
   __shared__ unsigned slot;
   const ColLor lor = col_lor(t, s, blockIdx.x);
@@ -224,9 +231,18 @@ __global__ void __launch_bounds__(kColBlock, kColBlocks) k_em_cols_listed(
   for (int g0 = 0; g0 < t.n_sinos; g0 += kColWindow) {
     const int64_t first = bin_of(t, s, lor, g0, counts_packed);
     const int n = col_active(t.n_sinos, g0, [&](int i) { return load_count<CT>(counts, first + i * step); }, act);
-    if (n <= few && t.n_sinos <= kColWindow) {
+    if ((n <= few || n <= direct) && t.n_sinos <= kColWindow) {
       if (n == 0) {
         if (threadIdx.x == 0) partials[blockIdx.x] = 0.0;
+        return;
+      }
+      if (n <= direct) {
+        if (threadIdx.x == 0) {
+          slot = atomicAdd(queue.n + 1, (unsigned)n);
+          partials[blockIdx.x] = 0.0;
+        }
+        __syncthreads();
+        for (int i = threadIdx.x; i < n; i += blockDim.x) queue.bins[slot + i] = blockIdx.x * (unsigned)t.n_sinos + act.list[i];
         return;
       }
       if (threadIdx.x == 0) {
@@ -275,6 +291,43 @@ __global__ void __launch_bounds__(kColFewBlock, kColFewBlocks) k_em_cols_few(
     }
     em_partial(term, item.x, partials);
     __syncthreads();
+  }
+}
+
+// The bins of LORs with too few counts to list the crossings for, a lane each,
+// whose terms are added to their LOR's partial.  Bound by the latency of a step
+// (select and eight loads in flight against branch and four: 16 sinograms of a
+// 256 x 256 image at 0.2 % bins with counts, the pass 141 -> 94 us) where the
+// bins are few, by instruction issue and scattered sectors where they are many.
+template <typename CT>
+__global__ void __launch_bounds__(kColDirectBlock, kColDirectBlocks) k_em_cols_direct(
+    ImgGeom g, ColDims d, LorTable t, SubsetSel s, const CT* __restrict__ counts, int counts_packed,
+    const float* __restrict__ add, const float* __restrict__ img, float* __restrict__ acc, int back,
+    double* __restrict__ partials, int skip_zero, ColQueue queue) {
+  const unsigned bins = queue.n[1], last = (unsigned)d.floats() - 1u;
+  for (unsigned b = blockIdx.x * blockDim.x + threadIdx.x; b < bins; b += gridDim.x * blockDim.x) {
+    const unsigned bin = queue.bins[b], at = bin / (unsigned)t.n_sinos;
+    const ColLor lor = col_lor(t, s, at);
+    const int gl = (int)(bin - at * (unsigned)t.n_sinos);
+    const float4 P = __ldg(t.lor + (int64_t)lor.a * t.n_r + lor.l);
+    const float2 ez = __ldg(t.z + t.g0 + gl);
+    const int64_t ci = bin_of(t, s, lor, gl, counts_packed);
+    const float m = load_count<CT>(counts, ci);
+    ColWalk w;
+    col_setup_xy(P, g, d, w);
+    const ColRay ray(w, col_setup_z(ez, w, g, d));
+    ColGather sum;
+    if (w.listed) sum.acc = col_ray_gather<kColDirectU>(ray, last, img);
+    else col_walk_checked(P, ez, g, d, img, sum);
+    float e = sum.acc;
+    if (add) e = A_ADD(e, __ldg(add + ci));
+    if (e != 0.f) atomicAdd(partials + at, lik_term(m, e, skip_zero));
+    const float q = (m != 0.f && e != 0.f && back) ? A_DIV(m, e) : 0.f;
+    if (q == 0.f) continue;
+    float* const sums = acc + (w.xmain ? d.floats() : 0);
+    ColScatter out{q};
+    if (w.listed) col_ray_scatter(ray, last, q, sums);
+    else col_walk_checked(P, ez, g, d, sums, out);
   }
 }
 
@@ -332,7 +385,7 @@ __global__ void __launch_bounds__(256) k_col_copy(ColDims d, const float* __rest
   __shared__ float tile[32][33];
   __shared__ double part[8];
   const int lx = threadIdx.x, ly = threadIdx.y;
-  if (queue_n && (blockIdx.x | blockIdx.y | blockIdx.z) == 0 && (lx | ly) == 0) *queue_n = 0;
+  if (queue_n && (blockIdx.x | blockIdx.y | blockIdx.z) == 0 && (lx | ly) == 0) queue_n[0] = queue_n[1] = 0;
   double s = col_copy_tile(d, x, img, gimg, blockIdx.x * 32, blockIdx.y, blockIdx.z * 32, lx, ly, tile);
   if (!gimg) return;
   #pragma unroll
@@ -524,12 +577,36 @@ static cudaError_t em_cols(const ImgGeom& g, const ColBuffers& c, const LorTable
   // 41 job: 141 -> 128 us).
   // With so few sinograms that a block has few warps anyway (37 and 19 of a
   // 128 x 128 image: 388 and 358 us with the queue, 304 and 181 without) there
-  // is nothing to defer either.
-  const int few = lors_of(t, s) > 2 * sms * kColBlocks && t.n_sinos > 4 * kColFew && t.n_sinos <= kColWindow ? kColFew
-                                                                                                            : 0;
+  // is nothing to defer to small blocks either.
+  //
+  // A list costs a block about 2600 warp instructions and the walk along it
+  // 250 and 17 a step, whether one lane has a ray or 32; a lane's own walk 300
+  // and some 30 a step for 32 rays together.  So the bins of LORs with up to 32
+  // counts, or 64 where a block of eight warps would take them, are walked one
+  // a lane; of up to 40 sinograms all are (34 of a 256 x 256 image, 70 % bins
+  // with counts: 326 us all listed, 331 us in part, 250 us).  Us of the listed
+  // pass on the padded pair / with every LOR listed / with this, bins with
+  // counts 1 %, 20 %, 70 %: 128 x 128 image, 27,556 LORs of 146 sinograms 177,
+  // 521, 1054 / 433, 567, 744 / 134, 516, 749; of 34 sinograms 122, 186, 318 /
+  // 135, 294, 303 / 73, 164, 259; of 310 sinograms 231, 1001, 2091 / 447, 720,
+  // 1294 / 204, 726, 1294.  Between the two kernels lies the walk of the last
+  // rays, 8 us: below 8000 LORs a pass is too short for it (6889 LORs of 310
+  // sinograms, 64 x 64: 95, 144, 225 us without, 61, 152, 233 with; on the
+  // padded pair 103, 188, 336).
+  const int64_t lors = lors_of(t, s);
+  const bool queued = lors > kColDirectLors && t.n_sinos <= kColWindow && lors * t.n_sinos <= INT_MAX;
+  const int direct = queued ? col_direct(t.n_sinos) : 0;
+  const int few = lors > 2 * sms * kColBlocks && lors <= kColDirectLors && t.n_sinos > 4 * kColFew &&
+                          t.n_sinos <= kColWindow ? kColFew : 0;
   k_em_cols_listed<CT><<<grid, block_of(t), smem, st>>>(g, d, t, s, counts, counts_packed, add, c.img, c.acc, back,
-                                                       partials, skip_zero, few, queue);
-  if ((e = cudaGetLastError()) != cudaSuccess || !few) return e;
+                                                       partials, skip_zero, few, direct, queue);
+  if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  if (direct) {
+    k_em_cols_direct<CT><<<(unsigned)(sms * kColDirectBlocks), kColDirectBlock, 0, st>>>(
+        g, d, t, s, counts, counts_packed, add, c.img, c.acc, back, partials, skip_zero, queue);
+    return cudaGetLastError();
+  }
+  if (!few) return cudaSuccess;
   const unsigned resident = (unsigned)(sms * kColFewBlocks);
   k_em_cols_few<CT><<<grid < resident ? grid : resident, kColFewBlock, smem, st>>>(g, d, t, s, counts, counts_packed, add, c.img,
                                                                         c.acc, back, partials, skip_zero, queue);

@@ -405,6 +405,65 @@ struct ColScatter {
   }
 };
 
+// A lane's own walk over the column layout, for rays of LORs with too few to
+// list the crossings for: the reference's steps (next_crossing), the voxel's
+// place moving by a column or, in z, by the slice changes of WalkZ.  The LOR
+// is one that could be listed: its walk stays within the border in x and y and
+// the columns hold every slice that it can enter; the clamp of the place to
+// the layout is a memory-safety net.  A step selects among all three axes' next
+// crossings: few such rays are under way, and a pass over them waits for this
+// chain (k_em_cols_direct).
+struct ColRay {
+  float ax, ay, az, axu, ayu, azu, ac, len;
+  int at, sx, sy, step, up, n;
+  __device__ __forceinline__ ColRay(const ColWalk& w, const WalkZ& r)
+      : ax(w.ax), ay(w.ay), az(r.az), axu(w.axu), ayu(w.ayu), azu(r.azu), ac(w.amin), len(r.len), at(w.col + r.at),
+        sx(w.sx), sy(w.sy), step(r.step), up(r.up), n(w.n + r.rem) {}
+  __device__ __forceinline__ void next(int& place, float& seg) {
+    const float an = fminf(fminf(ax, ay), az);
+    const bool cx = ax == an, cy = !cx & (ay == an), cz = !(cx | cy);
+    seg = A_MUL(A_SUB(an, ac), len);
+    place = at;
+    ac = an;
+    at += cx ? sx : (cy ? sy : step);
+    step = cz ? up - step : step;
+    const float nx = A_ADD(ax, axu), ny = A_ADD(ay, ayu), nz = A_ADD(az, azu);
+    ax = cx ? nx : ax;
+    ay = cy ? ny : ay;
+    az = cz ? nz : az;
+  }
+};
+template <int U>
+__device__ __forceinline__ float col_ray_gather(ColRay r, unsigned last, const float* __restrict__ img) {
+  float acc = 0.f;
+  int m = 0;
+  for (; m + U <= r.n; m += U) {  // a batch's loads all in flight before its sums
+    int place[U];
+    float seg[U], v[U];
+    #pragma unroll
+    for (int u = 0; u < U; u++) r.next(place[u], seg[u]);
+    #pragma unroll
+    for (int u = 0; u < U; u++) v[u] = __ldg(img + min((unsigned)place[u], last));
+    #pragma unroll
+    for (int u = 0; u < U; u++) acc = A_ADD(acc, A_MUL(seg[u], v[u]));
+  }
+  for (; m < r.n; m++) {
+    int place;
+    float seg;
+    r.next(place, seg);
+    acc = A_ADD(acc, A_MUL(seg, __ldg(img + min((unsigned)place, last))));
+  }
+  return acc;
+}
+__device__ __forceinline__ void col_ray_scatter(ColRay r, unsigned last, float v, float* __restrict__ acc) {
+  for (int m = 0; m < r.n; m++) {
+    int place;
+    float seg;
+    r.next(place, seg);
+    red_add_global(acc + min((unsigned)place, last), A_MUL(seg, v));
+  }
+}
+
 // One ray with the reference's six-sided bounds test, for LORs that are not
 // on the list: visit(place, length) for its segments in the image.
 template <class T, class V>

@@ -59,7 +59,6 @@ __device__ __forceinline__ double em_rays(const ImgGeom& g, const ColDims& d, co
 
 // The block's list of a LOR's sinograms with counts, among kColWindow from
 // g0: list[0 .. n) in order, n returned to every thread.
-constexpr int kColWindow = 2048;
 struct ColActive {
   unsigned mask[kColWindow / 32];
   int first[kColWindow / 32];

@@ -155,13 +155,20 @@ constexpr int kColMinSinos = 16;
 ColBuffers col_layout(const ImgGeom& g, const float* z_ends, int n_ends);
 // Likelihood partials of a column pass.
 int64_t col_partials(const LorTable& t, SubsetSel s);
-// A listed column pass's LORs with few counts: item (LOR of the subset, count)
-// and list (kColFew sinograms of each); room for every LOR.
+// What a listed column pass leaves to a second kernel, because listing a LOR's
+// crossings is not worth its few rays (columns.cu, em_cols, has the rules): of
+// up to kColDirectLors LORs, items (LOR of the subset, count) and lists (kColFew
+// sinograms of each); of more, bins (LOR * n_sinos + sinogram) of those with at
+// most col_direct.  n: the numbers of both.
+constexpr int kColWindow = 2048;  // sinograms that a block looks for counts at a time
 constexpr int kColFew = 64;
+constexpr int kColDirectLors = 8000;
+inline int col_direct(int n_sinos) { return n_sinos > 4 * kColFew ? kColFew : n_sinos <= 40 ? 40 : kColFew / 2; }
 struct ColQueue {
   unsigned* n = nullptr;
   uint2* item = nullptr;
   uint16_t* list = nullptr;
+  unsigned* bins = nullptr;
 };
 // Partials of -x . gimg (launch_col_copy).
 int64_t col_dots(const ImgGeom& g);

@@ -193,3 +193,18 @@ def mallocs(make):
 P = mallocs(lambda: ap.SiddonProjector(*G3)); mallocs(lambda: P.set_sampling(2, 2)); mallocs(lambda: ap.SiddonProjector(*G2))
 done(n)''')
     assert counts == [1, 1, 1]
+
+
+@pytest.mark.parametrize("rings,max_rd,n_proj,want", [(16, 0, 100, "k_em_cols_direct"), (33, 4, 100, "k_em_cols_direct"),
+                                                      (33, 4, 40, "k_em_cols_few"), (16, 0, 40, ""), (46, 45, 100, "")])
+def test_listed_passes_defer_lors_with_few_counts(gpu, rings, max_rd, n_proj, want):
+    """Where a LOR's crossings are listed for few rays, the pass leaves them to a second kernel."""
+    names = gpu(f'''
+P = ap.SiddonProjector(ImageGeom(27, 24, 31, 2.5, 2.5, 2.0), Sino3DGeom.span1({n_proj}, 90, {rings}, 45.0, 64.0, 120.0, {max_rd}))
+P.set_option(_lib.APIRL_OPT_SPARSE_IMAGE, _lib.APIRL_SPARSE_GEOMETRY)
+fake.clear()
+_lib.check(lib.apirl_em_pass_sparse(P.h, D, 0, 0, None, D, D, D, D, None, None, 0.0, 0, -1, 1, None, S))
+done(fake.launches())''')
+    assert any("k_em_cols_listed" in n for n in names)
+    second = [k for k in ("k_em_cols_direct", "k_em_cols_few") if any(k in n for n in names)]
+    assert second == ([want] if want else [])
