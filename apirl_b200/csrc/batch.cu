@@ -6,9 +6,9 @@
 // synchronises its streams while jobs run), then launches one batched EM step:
 // one pass of every running job, or its final likelihood, in four or five
 // launches whatever the number of jobs (image copies and image dot products;
-// the column walk of the jobs with 16 and more sinograms, a block per LOR,
-// beside a persistent walk over the concatenated lists of the other jobs'
-// bins with counts; the likelihood sums; the EM updates).
+// the column walk of the jobs with many counts a LOR, a block per LOR, beside
+// a persistent walk over the concatenated lists of the other jobs' bins with
+// counts; the likelihood sums; the EM updates).
 //
 // * Device memory comes from a private stream-ordered pool that keeps what it
 //   has reserved, so jobs coming and going allocate nothing from the driver
@@ -280,11 +280,12 @@ struct Job {
   int* d_list = nullptr;
   PadBuffers pad;
   ColBuffers cols;               // or these, without lists (cols.half)
+  unsigned long long* d_sq = nullptr;  // of a job that may take either: launch_lor_counts' sum
   std::vector<int64_t> tile_off, list_off;
   std::vector<int> n_list;
   std::vector<double> zero_add;
   // host
-  void* h_stage = nullptr;   // pinned: n_list (nsub ints), zero_add (nsub doubles)
+  void* h_stage = nullptr;   // pinned: n_list (nsub ints), zero_add (nsub doubles), d_sq
   float* h_out = nullptr;    // pinned result image
   double* h_lik = nullptr;   // pinned likelihoods
   cudaEvent_t ev = nullptr;  // end of the current stage's GPU work
@@ -594,7 +595,8 @@ apirl_status geom_for(apirl_batch* b, Job& j, Geom** out) {
 // Layout of a job's page-locked staging block: the subsets' list lengths and
 // additive sums (read back), two sensitivity-walk descriptors (sent).
 size_t stage_zero_add_off(int nsub) { return 8 * (((size_t)nsub * 4 + 7) / 8); }
-size_t stage_sens_off(int nsub) { return 16 * ((stage_zero_add_off(nsub) + (size_t)nsub * 8 + 15) / 16); }
+size_t stage_sq_off(int nsub) { return stage_zero_add_off(nsub) + (size_t)nsub * 8; }
+size_t stage_sens_off(int nsub) { return 16 * ((stage_sq_off(nsub) + 8 + 15) / 16); }
 size_t stage_bytes(int nsub) { return stage_sens_off(nsub) + 2 * sizeof(SensJob); }
 
 // sens[a % nsub] += A_a^T (mult or 1) over the whole sinogram (one walk),
@@ -670,16 +672,14 @@ void release_job(apirl_batch* b, Job& j) {
   b->pool.release(j.d_x, s);
   b->pool.release(j.d_sens, s);
   b->pool.release(j.d_lik, s);
-  b->pool.release(j.d_zero_add, s);
-  b->pool.release(j.d_tiles, s);
   b->pool.release(j.d_nlist, s);
+  b->pool.release(j.d_tiles, s);
   b->pool.release(j.d_list, s);
   b->pool.release(j.pad.pA, s);
   b->pool.release(j.pad.pT, s);
   b->pool.release(j.pad.bA, s);
   b->pool.release(j.pad.bT, s);
-  b->pool.release(j.cols.img, s);
-  b->pool.release(j.cols.acc, s);
+  b->pool.release(j.cols.img, s);  // and the sums behind it
   if (j.set) { j.set->refs--; j.set = nullptr; }
   if (j.geom) { j.geom->refs--; j.geom->last_use = ++b->clock; j.geom = nullptr; }
   b->pinned.put(j.h_stage); j.h_stage = nullptr;
@@ -696,6 +696,50 @@ void destroy_events(Job& j) {
   j.ev = j.alloc_ev = j.up_ev = nullptr;
 }
 
+// The padded copies and list tiles of a job that walks lists, or the column
+// image and sums of one that does not.
+apirl_status pair_layout(apirl_batch* b, Job& j) {
+  cudaStream_t s = b->st;
+  const int64_t pv = padded_voxels(j.img);
+  j.tile_off.assign(j.nsub + 1, 0);
+  for (int k = 0; k < j.nsub; k++)
+    j.tile_off[k + 1] = j.tile_off[k] + n_tiles_of((int64_t)j.geom->t.n_sinos *
+                                                   apirl::subset_nproj(j.sino.n_proj, k, j.nsub) * j.sino.n_r);
+  BK(b->pool.alloc(&j.d_tiles, std::max<int64_t>(j.tile_off[j.nsub], 1), s));
+  float** pads[4] = {&j.pad.pA, &j.pad.pT, &j.pad.bA, &j.pad.bT};
+  for (float** q : pads) {
+    BK(b->pool.alloc(q, pv, s));
+    BK(cudaMemsetAsync(*q, 0, (size_t)pv * 4, s));
+  }
+  j.pad.lim = (unsigned)pv;
+  return APIRL_OK;
+}
+apirl_status column_layout(apirl_batch* b, Job& j) {
+  cudaStream_t s = b->st;
+  ColBuffers c = j.geom->cols;
+  BK(b->pool.alloc(&c.img, 3 * c.floats, s));
+  c.acc = c.img + c.floats;
+  j.cols = c;
+  BK(cudaMemsetAsync(c.img, 0, (size_t)c.floats * 12, s));
+  return APIRL_OK;
+}
+
+// Whether a job that may take either layout takes the columns.  A block of the
+// column walk lists its LOR's crossings for however few bins with counts; the
+// lists' lanes walk a bin each.  Ms an iteration, lists -> columns, of equal
+// jobs on 64 x 64 to 128 x 128 images by the bins with counts of the LORs
+// through the object: 3 (16 sinograms, 8 jobs) 1.2 -> 3.1, 15 (310, 2 jobs) 1.1
+// -> 1.3, 24 (119, 4 jobs) 0.9 -> 1.1, 29 (146, 4 jobs) 1.9 -> 1.9, 45 (65, 4
+// jobs) 1.7 -> 1.7, 62 (310, 2 jobs) 1.9 -> 1.5, 102 (146, 4 jobs) 3.0 -> 2.6.
+// So columns from 40 on, as a bin with counts finds its LOR on average
+// (sq / bins).  Below, a pass loses up to 7 ns a LOR; building a subset's
+// list takes 20 us of launches, the passes over 3000 LORs.
+bool columns_pay(const Job& j, unsigned long long sq, unsigned long long bins) {
+  if (!bins) return false;
+  const double missing = 1.0 - (double)sq / (double)bins / 40.0;
+  return missing * j.iters * j.sino.n_proj / j.nsub * j.sino.n_r <= 3000.0;
+}
+
 // Buffers of an admitted job, from the pool on the compute stream; the upload
 // worker waits for alloc_ev before copying into them.
 apirl_status admit(apirl_batch* b, Job& j) {
@@ -703,7 +747,6 @@ apirl_status admit(apirl_batch* b, Job& j) {
   j.geom->refs++;
   j.geom->last_use = ++b->clock;
   cudaStream_t s = b->st;
-  const int64_t pv = padded_voxels(j.img);
   BK(cudaEventCreateWithFlags(&j.ev, cudaEventDisableTiming));
   BK(cudaEventCreateWithFlags(&j.alloc_ev, cudaEventDisableTiming));
   BK(cudaEventCreateWithFlags(&j.up_ev, cudaEventDisableTiming));
@@ -715,30 +758,13 @@ apirl_status admit(apirl_batch* b, Job& j) {
   if (j.h_add) BK(b->pool.alloc(&j.d_add, j.nbins, s));
   BK(b->pool.alloc(&j.d_x, j.nvox, s));
   BK(b->pool.alloc(&j.d_lik, (int64_t)j.iters * j.nsub + 1, s));
-  BK(b->pool.alloc(&j.d_zero_add, j.nsub, s));
-  if (j.geom->cols.half) {
-    j.cols = j.geom->cols;
-    BK(b->pool.alloc(&j.cols.img, j.cols.floats, s));
-    BK(b->pool.alloc(&j.cols.acc, 2 * j.cols.floats, s));
-    BK(cudaMemsetAsync(j.cols.img, 0, (size_t)j.cols.floats * 4, s));
-    BK(cudaMemsetAsync(j.cols.acc, 0, (size_t)j.cols.floats * 8, s));
-  } else {
-    BK(b->pool.alloc(&j.d_nlist, j.nsub, s));
-    j.tile_off.assign(j.nsub + 1, 0);
-    for (int k = 0; k < j.nsub; k++)
-      j.tile_off[k + 1] = j.tile_off[k] + n_tiles_of((int64_t)j.geom->t.n_sinos *
-                                                     apirl::subset_nproj(j.sino.n_proj, k, j.nsub) * j.sino.n_r);
-    BK(b->pool.alloc(&j.d_tiles, std::max<int64_t>(j.tile_off[j.nsub], 1), s));
-    float* pads[4];
-    for (int k = 0; k < 4; k++) {
-      BK(b->pool.alloc(&pads[k], pv, s));
-      BK(cudaMemsetAsync(pads[k], 0, (size_t)pv * 4, s));
-    }
-    j.pad.pA = pads[0]; j.pad.pT = pads[1]; j.pad.bA = pads[2]; j.pad.bT = pads[3];
-    j.pad.lim = (unsigned)pv;
-  }
+  // n_list, zero_add and sq as in h_stage, to be read back in one copy
+  BK(b->pool.alloc((char**)&j.d_nlist, (int64_t)stage_sens_off(j.nsub), s));
+  BK(cudaMemsetAsync(j.d_nlist, 0, stage_sens_off(j.nsub), s));
+  j.d_zero_add = (double*)((char*)j.d_nlist + stage_zero_add_off(j.nsub));
+  if (j.geom->cols.half) j.d_sq = (unsigned long long*)((char*)j.d_nlist + stage_sq_off(j.nsub));
+  else BS(pair_layout(b, j));
   BK(cudaMemsetAsync(j.d_lik, 0, ((size_t)j.iters * j.nsub + 1) * 8, s));
-  BK(cudaMemsetAsync(j.d_zero_add, 0, (size_t)j.nsub * 8, s));
   j.h_stage = b->pinned.get(stage_bytes(j.nsub));
   j.h_out = (float*)b->pinned.get((size_t)j.nvox * 4);
   j.h_lik = (double*)b->pinned.get(((size_t)j.iters * j.nsub + 1) * 8);
@@ -751,24 +777,30 @@ apirl_status admit(apirl_batch* b, Job& j) {
   return APIRL_OK;
 }
 
-// Counts arrived: the initial image, the per-subset list lengths (of a job
-// that walks lists) and additive sums (read back), the own sensitivity of a
-// job with factors.
+// The tiles of a job's lists (and their lengths, d_nlist).
+apirl_status count_lists(apirl_batch* b, Job& j) {
+  const LorTable& t = j.geom->t;
+  for (int k = 0; k < j.nsub; k++) {
+    SubsetSel ss;
+    ss.subset = k; ss.nsub = j.nsub; ss.nk = apirl::subset_nproj(j.sino.n_proj, k, j.nsub);
+    BK(apirl::launch_nz_count(t, ss, j.d_counts, j.dtype, (int64_t)t.n_sinos * ss.nk * t.n_r,
+                              j.d_tiles + j.tile_off[k], j.d_nlist + k, b->st));
+  }
+  return APIRL_OK;
+}
+
+// Counts arrived: the initial image, the per-subset list lengths (and how the
+// bins with counts share LORs, of a job that may take the columns) and
+// additive sums (read back), the own sensitivity of a job with factors.
 apirl_status start_counting(apirl_batch* b, Job& j) {
   cudaStream_t s = b->st;
   BK(cudaStreamWaitEvent(s, j.up_ev, 0));
   if (!j.h_init) BK(apirl::launch_fill(j.nvox, j.d_x, 1.f, s));
   const LorTable& t = j.geom->t;
-  for (int k = 0; k < j.nsub && !j.cols.half; k++) {
-    SubsetSel ss;
-    ss.subset = k; ss.nsub = j.nsub; ss.nk = apirl::subset_nproj(j.sino.n_proj, k, j.nsub);
-    BK(apirl::launch_nz_count(t, ss, j.d_counts, j.dtype, (int64_t)t.n_sinos * ss.nk * t.n_r,
-                              j.d_tiles + j.tile_off[k], j.d_nlist + k, s));
-  }
+  if (j.d_sq) BK(apirl::launch_lor_counts(t, j.nsub, j.d_counts, j.dtype, j.d_nlist, j.d_sq, s));
+  else BS(count_lists(b, j));
   if (j.d_add) BK(apirl::launch_subset_sums(t, j.nsub, j.d_add, j.d_zero_add, s));
-  if (!j.cols.half) BK(cudaMemcpyAsync(j.h_stage, j.d_nlist, (size_t)j.nsub * 4, cudaMemcpyDeviceToHost, s));
-  BK(cudaMemcpyAsync((char*)j.h_stage + stage_zero_add_off(j.nsub), j.d_zero_add, (size_t)j.nsub * 8,
-                     cudaMemcpyDeviceToHost, s));
+  BK(cudaMemcpyAsync(j.h_stage, j.d_nlist, stage_sens_off(j.nsub), cudaMemcpyDeviceToHost, s));
   if (j.d_mult) {
     // sens_s = A_s^T (factors of subset s), then forcePositive (OsemSinogram3d.cpp:327-346, :115)
     BK(cudaMemsetAsync(j.d_sens, 0, (size_t)j.nvox * j.nsub * 4, s));
@@ -780,17 +812,29 @@ apirl_status start_counting(apirl_batch* b, Job& j) {
   return APIRL_OK;
 }
 
-// List lengths known: the lists themselves, and the shared sensitivity.
+// List lengths known: the layout (of a job that may take either), the lists
+// themselves, and the shared sensitivity.
 apirl_status start_running(apirl_batch* b, Job& j) {
   cudaStream_t s = b->st;
   const double* za = (const double*)((char*)j.h_stage + stage_zero_add_off(j.nsub));
   j.zero_add.assign(za, za + j.nsub);
+  j.n_list.assign((const int*)j.h_stage, (const int*)j.h_stage + j.nsub);
+  if (j.d_sq) {
+    unsigned long long sq = 0, bins = 0;
+    memcpy(&sq, (const char*)j.h_stage + stage_sq_off(j.nsub), 8);
+    for (int n : j.n_list) bins += (unsigned)n;
+    if (columns_pay(j, sq, bins)) {
+      BS(column_layout(b, j));
+    } else {
+      BS(pair_layout(b, j));
+      BS(count_lists(b, j));
+    }
+  }
   int64_t unused;
   if (j.cols.half) {
     // the columns in place of the padded copies and lists
     unused = pads_and_lists(j.img, j.nbins) - 3 * align256(j.cols.floats * 4);
   } else {
-    j.n_list.assign((const int*)j.h_stage, (const int*)j.h_stage + j.nsub);
     j.list_off.assign(j.nsub + 1, 0);
     for (int k = 0; k < j.nsub; k++) j.list_off[k + 1] = j.list_off[k] + j.n_list[k];
     BK(b->pool.alloc(&j.d_list, std::max<int64_t>(j.list_off[j.nsub], 1), s));

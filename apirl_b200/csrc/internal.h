@@ -364,6 +364,10 @@ cudaError_t launch_sum_angles(const float* per_angle, const uint8_t* tr_of, unsi
 cudaError_t launch_sum_images(const float* img, int n_img, int64_t nvox, int nsub, float* out, cudaStream_t st);
 // out[s] = sum over subset s's bins of the additive term (whole-sinogram layout), FP64, fixed order.
 cudaError_t launch_subset_sums(const LorTable& t, int nsub, const float* add, double* out, cudaStream_t st);
+// n[s] += the bins with counts of subset s; *sq += the sum over (angle, r) of
+// their number squared.
+cudaError_t launch_lor_counts(const LorTable& t, int nsub, const void* counts, int dtype, int* n, unsigned long long* sq,
+                              cudaStream_t st);
 
 // Sensitivity of every subset of a job whose sinogram has a multiplicative
 // term, in one pass over its whole sinogram: bin (g, a, l) belongs to subset

@@ -1408,6 +1408,38 @@ __global__ void __launch_bounds__(kBlock) k_subset_sums(LorTable t, int nsub, co
   if (threadIdx.x == 0) out[blockIdx.x] = r;
 }
 
+// Bins with counts of every subset, n[a % nsub], and the sum over (angle, r) of
+// their number squared, *sq: blocks of 32 r of one angle by 16 slices of the
+// sinograms; the counters start at zero.
+constexpr int kLorSlices = 16;
+__global__ void __launch_bounds__(32 * kLorSlices) k_lor_counts(LorTable t, int nsub, const void* __restrict__ counts,
+                                                                int dtype, int* __restrict__ n,
+                                                                unsigned long long* __restrict__ sq) {
+  __shared__ int part[kLorSlices][32];
+  const int groups = (t.n_r + 31) / 32, a = blockIdx.x / groups;
+  const int l = (int)(blockIdx.x - a * groups) * 32 + (threadIdx.x & 31), slice = threadIdx.x >> 5;
+  int c = 0;
+  if (l < t.n_r) {
+    #pragma unroll 4
+    for (int g = slice; g < t.n_sinos; g += kLorSlices)
+      c += load_count_any(counts, dtype, ((int64_t)(t.g0 + g) * t.n_proj + a) * t.n_r + l) != 0.f;
+  }
+  part[slice][threadIdx.x & 31] = c;
+  __syncthreads();
+  if (slice) return;
+  c = 0;
+  #pragma unroll
+  for (int q = 0; q < kLorSlices; q++) c += part[q][threadIdx.x];
+  const int sum = __reduce_add_sync(0xffffffffu, c);
+  unsigned long long s2 = (unsigned long long)c * (unsigned long long)c;
+  #pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s2 += __shfl_down_sync(0xffffffffu, s2, o);
+  if (threadIdx.x == 0 && sum) {
+    atomicAdd(n + a % nsub, sum);
+    atomicAdd(sq, s2);
+  }
+}
+
 inline unsigned grid_for(int64_t total) { return (unsigned)((total + kBlock - 1) / kBlock); }
 
 // Launch of a kernel over the padded layouts: with pad.window
@@ -1926,6 +1958,7 @@ cudaError_t load_batch_kernels() {
       (const void*)k_em_multi,          (const void*)k_multi_copy,         (const void*)k_multi_sum,
       (const void*)k_multi_update,      (const void*)k_scatter_angles,     (const void*)k_sum_angles,
       (const void*)k_sum_images,        (const void*)k_subset_sums,        (const void*)k_sens_batch,
+      (const void*)k_lor_counts,
       (const void*)k_nz_scan,           (const void*)k_nz_tiles<float>,    (const void*)k_nz_tiles<uint16_t>,
       (const void*)k_nz_tiles<uint32_t>, (const void*)k_nz_write<float>,   (const void*)k_nz_write<uint16_t>,
       (const void*)k_nz_write<uint32_t>};
@@ -2053,6 +2086,13 @@ cudaError_t launch_sum_images(const float* img, int n_img, int64_t nvox, int nsu
 cudaError_t launch_subset_sums(const LorTable& t, int nsub, const float* add, double* out, cudaStream_t st) {
   if (nsub <= 0) return cudaSuccess;
   k_subset_sums<<<nsub, kBlock, 0, st>>>(t, nsub, add, out);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_lor_counts(const LorTable& t, int nsub, const void* counts, int dtype, int* n, unsigned long long* sq,
+                              cudaStream_t st) {
+  k_lor_counts<<<(unsigned)((int64_t)t.n_proj * ((t.n_r + 31) / 32)), 32 * kLorSlices, 0, st>>>(t, nsub, counts, dtype,
+                                                                                               n, sq);
   return cudaGetLastError();
 }
 

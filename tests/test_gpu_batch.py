@@ -264,3 +264,27 @@ def test_batch_column_walk(rings, max_rd):
         assert np.array_equal(np.isfinite(img), finite), j.tag
         assert rel(img[finite], solo[finite]) <= 1e-4, j.tag
         assert np.allclose(lik[:-1], solo_lik[:-1], rtol=1e-6), j.tag
+
+
+@pytest.mark.parametrize("rings,max_rd,angles,share", [(21, 20, 20, 0.02), (21, 20, 20, 0.6), (46, 45, 4, 0.01), (46, 45, 4, 0.3)])
+def test_batch_by_counts_a_lor(rings, max_rd, angles, share):
+    """Jobs whose bins with counts are walked by lists or by LORs, as the counts
+    of a LOR say (441 sinograms, and 2116: more than the window in which a
+    block looks for counts): each equals its solo run, beside one of the other kind."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    ig = ap.ImageGeom(24, 27, 2 * rings - 1, 2.08, 2.08, 2.03)
+    sg = ap.Sino3DGeom.span1(angles, 30, rings, 30 * 2.08 / 2, rings * 4.06, 443.0, max_rd)
+    rng = np.random.default_rng(rings)
+    jobs = []
+    for f, dt in ((share, np.uint16), (0.5 * share, np.float32), (0.9 - share, np.uint32)):
+        counts = ((rng.random(sg.n_bins) < f) * (1 + rng.poisson(1.0, sg.n_bins))).astype(dt)
+        jobs.append(Job(ig, sg, counts, 2, 4, update_positive_sens=True))
+    b = Batch(0, budget_bytes=8 << 30)
+    res = b.run_all(jobs)
+    b.close()
+    for j, (img, lik) in zip(jobs, res):
+        solo, solo_lik, _ = ap.osem_3d(ig, sg, j.counts.astype(np.float32), np.ones(ig.n_voxels, np.float32), j.iters,
+                                       j.nsubsets, update_positive_sens=True)
+        assert rel(img, solo) <= 1e-4
+        assert np.allclose(lik, solo_lik, rtol=1e-6)

@@ -208,3 +208,15 @@ done(fake.launches())''')
     assert any("k_em_cols_listed" in n for n in names)
     second = [k for k in ("k_em_cols_direct", "k_em_cols_few") if any(k in n for n in names)]
     assert second == ([want] if want else [])
+
+
+def test_batched_jobs_with_few_counts_take_lists(gpu):
+    """A block a LOR pays from some tens of counts in it on: jobs with fewer (here none) walk lists of their bins."""
+    names = gpu('''
+from apirl_b200.batch import Batch, Job
+ig, sg = ImageGeom(128, 128, 31, 2.0, 2.0, 2.0), Sino3DGeom.span1(160, 160, 16, 160.0, 64.0, 443.0, 0)
+b = Batch(0, 8 << 30)
+b.run_all([Job(ig, sg, np.zeros(sg.n_bins, np.uint16), 10, 8)])
+done(sorted(set(fake.launches())))''')
+    assert any("k_lor_counts" in n for n in names) and any("k_nz_write" in n for n in names)
+    assert not any("k_em_multi_cols" in n for n in names)
