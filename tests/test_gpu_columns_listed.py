@@ -72,3 +72,25 @@ def test_listed_pass(oracle, rings, max_rd, n_proj, n_r, nsub, share, dtype, wit
         P.em_pass_sparse(t(meas), x, zeros(), t(sens), G, sub, nsub, lik=lik, add=t(add) if with_add else None, zero_add=less)
         assert rel(x.cpu().numpy(), want) <= 1e-5
         assert abs(lik.item() - want_lik) <= 1e-6 * max(abs(want_lik), float(np.sum(e64)))
+
+
+@pytest.mark.parametrize("rings,max_rd,n_proj,n_r,nsub", LANES + [(16, 7, 100, 90, 1), (33, 4, 40, 50, 1)])
+@pytest.mark.parametrize("share", [0.0, 0.01, 0.3, 1.0])
+def test_backprojection_of_few_values(oracle, rings, max_rd, n_proj, n_r, nsub, share):
+    """A backprojection leaves LORs without values: empty, sparse and full
+    sinograms (256 of them and more), twice, added to what the image holds."""
+    ig = ImageGeom(27, 24, 2 * rings - 1, 2.5, 2.5, 2.0)
+    sg = Sino3DGeom.span1(n_proj, n_r, rings, 45.0, rings * 4.0, 120.0, max_rd)
+    rng = np.random.default_rng(rings)
+    sub = nsub - 1 if nsub > 1 else -1
+    P = ap.SiddonProjector(ig, sg)
+    n = P.num_bins(sub, nsub)
+    v = ((rng.random(n, dtype=np.float32) + 0.5) * (rng.random(n) < share)).astype(np.float32)
+    want = oracle.backproject_3d(sg, ig, v, sub, nsub, threads=1)
+    x0 = rng.random(ig.n_voxels, dtype=np.float32)
+    for _ in range(2):
+        got = P.backproject(t(v), t(x0), sub, nsub).cpu().numpy().astype(np.float64)
+        if not v.any():
+            assert np.array_equal(got, x0)
+        else:
+            assert np.linalg.norm(got - (x0.astype(np.float64) + want)) <= 1e-5 * np.linalg.norm(want) + 1e-6
