@@ -220,3 +220,14 @@ b.run_all([Job(ig, sg, np.zeros(sg.n_bins, np.uint16), 10, 8)])
 done(sorted(set(fake.launches())))''')
     assert any("k_lor_counts" in n for n in names) and any("k_nz_write" in n for n in names)
     assert not any("k_em_multi_cols" in n for n in names)
+
+
+@pytest.mark.parametrize("n,nsub,cols", [(32, 8, False), (32, 1, True), (64, 8, True)])
+def test_small_divisions_take_one_launch(gpu, n, nsub, cols):
+    nr = int(1.3 * n + 0.5)
+    names = gpu(f'''
+P = ap.SiddonProjector(ImageGeom({n}, {n}, 33, 2.0, 2.0, 2.0), Sino3DGeom.span1({nr}, {nr}, 17, {nr}.0, 68.0, 443.0, 0))
+fake.clear()
+_lib.check(lib.apirl_divide_and_backproject(P.h, D, D, D, 0, {nsub}, S))
+done(fake.launches())''')
+    assert any("k_scatter_cols" in x for x in names) == cols and any("k_backproject3" in x for x in names) != cols
