@@ -114,10 +114,22 @@ bool use_cols(const apirl_projector* p) {
 }
 
 // The fused passes with several rays a bin: on their own column layout where
-// set_sampling made it, from the sinograms on that pay in the plain passes.
-bool use_ray_cols(const apirl_projector* p) {
-  return p->t.lor_s && p->dual_layout && !p->pg.enabled && p->ray_cols.half && p->pad.acc == APIRL_ACC_ATOMIC &&
-         p->t.n_sinos >= apirl::kColMinSinos;
+// set_sampling made it, from the sinograms on that pay in the plain passes.  A
+// block holds a list a radial sample, so wide images and many samples leave
+// few rays in flight on an SM (the blocks that their lists leave room for
+// times the sinograms): over more than 2000 LORs the columns want 224 of them.
+// Us bin by bin -> columns, by rays in flight, 5 % and 90 % bins with counts:
+// 96 (16 sinograms, 64 x 64, 12 samples) 412 -> 887, 758 -> 981; 192 (24, 96 x
+// 96, 6 samples) 732 -> 941, dense 0.88 of the time; 240 (40, 64 x 64, 12) 811
+// -> 968, 0.71; 320 (40, 96 x 96, 6) 0.91 and 0.62; 861 LORs of the first job
+// 0.71 and 0.67.
+bool use_ray_cols(const apirl_projector* p, SubsetSel ss) {
+  if (!(p->t.lor_s && p->dual_layout && !p->pg.enabled && p->ray_cols.half && p->pad.acc == APIRL_ACC_ATOMIC &&
+        p->t.n_sinos >= apirl::kColMinSinos))
+    return false;
+  const size_t smem = p->t.n_rs * apirl::col_list_bytes(p->g) + 1536;  // the block's own and the reserved, too
+  const int64_t blocks = std::min<int64_t>(32, 227 * 1024 / smem);
+  return (int64_t)ss.nk * p->t.n_r <= 2000 || blocks * p->t.n_sinos >= 224;
 }
 
 // A slot for work queued on s until slot_done, which the lock covers: the one
@@ -838,7 +850,7 @@ namespace {
 // The padded pass on the column layout.  It has one launch form: the options
 // of the padded pair's launch (persistent, block size, gather segments) do not
 // change it, an ordered list keeps to the pair.
-bool pass_cols(const apirl_projector* p) { return (use_cols(p) && !p->nz.order) || use_ray_cols(p); }
+bool pass_cols(const apirl_projector* p, SubsetSel ss) { return (use_cols(p) && !p->nz.order) || use_ray_cols(p, ss); }
 const apirl::ColBuffers& pass_layout(const apirl_projector* p) { return p->t.lor_s ? p->ray_cols : p->cols; }
 
 // Before the padded pass: the image into its copy.  After it: the update of x
@@ -846,7 +858,7 @@ const apirl::ColBuffers& pass_layout(const apirl_projector* p) { return p->t.lor
 // carry the likelihood's dot product and sum too.
 apirl_status pass_begin(apirl_projector* p, SubsetSel ss, const float* d_x, const float* d_zimg, double* d_lik,
                         cudaStream_t s) {
-  if (pass_cols(p))
+  if (pass_cols(p, ss))
     CK(apirl::launch_col_copy(p->g, pass_layout(p), d_x, pass_layout(p).img, s, d_lik ? d_zimg : nullptr,
                               p->d_partials + apirl::col_partials(p->t, ss), d_zimg ? p->queue.n : nullptr));
   else
@@ -856,7 +868,7 @@ apirl_status pass_begin(apirl_projector* p, SubsetSel ss, const float* d_x, cons
 apirl_status pass_end(apirl_projector* p, SubsetSel ss, int mode, float* d_x, float* d_bp, const float* d_sens,
                       const float* d_thr, float thr_value, int ge, const float* d_zimg, const double* d_zero_add,
                       double* d_lik, cudaStream_t s) {
-  if (pass_cols(p)) {
+  if (pass_cols(p, ss)) {
     const int64_t lors = (int64_t)ss.nk * p->t.n_r;  // no LORs: no partials written
     const int64_t n = lors ? apirl::col_partials(p->t, ss) + (d_zimg ? apirl::col_dots(p->g) : 0) : 0;
     CK(apirl::launch_col_reduce(p->g, pass_layout(p), pass_layout(p).acc, mode, d_x, d_bp, d_sens, d_thr, thr_value, ge, s,
@@ -882,7 +894,7 @@ apirl_status fused(apirl_projector* p, SubsetSel ss, const void* d_counts, int d
   }
   if (dual && p->t.lor_s) {
     CK(apirl::launch_em_cols_rays(p->g, p->ray_cols, p->t, ss, d_counts, dtype, packed, d_add, 1, p->d_partials, s));
-  } else if (dual && pass_cols(p)) {
+  } else if (dual && pass_cols(p, ss)) {
     CK(apirl::launch_em_cols(p->g, p->cols, p->t, ss, d_counts, dtype, packed, d_add, 1, p->d_partials,
                              d_zimg ? (p->sparse_image ? 2 : 1) : 0, p->queue, s));
   } else if (p->planar.lim) {
@@ -921,7 +933,7 @@ apirl_status apirl_em_pass(apirl_projector* p, const void* d_counts, int counts_
   cudaStream_t s = (cudaStream_t)stream;
   SubsetSel ss = make_subset(p, subset, nsubsets);
   const int64_t nv = (int64_t)p->g.nx * p->g.ny * p->g.nz;
-  if (use_dual(p) || use_ray_cols(p)) {
+  if (use_dual(p) || use_ray_cols(p, ss)) {
     if ((st = pass_begin(p, ss, d_x, nullptr, d_lik, s))) return st;
     st = fused(p, ss, d_counts, counts_dtype, counts_packed, d_add, d_x, d_bp, true, d_lik, s);
     if (st) return st;
@@ -1020,7 +1032,7 @@ apirl_status apirl_em_project_backproject(apirl_projector* p, const void* d_coun
   DEVICE_SCOPE(p->device);
   cudaStream_t s = (cudaStream_t)stream;
   SubsetSel ss = make_subset(p, subset, nsubsets);
-  if (use_dual(p) || use_ray_cols(p)) {
+  if (use_dual(p) || use_ray_cols(p, ss)) {
     if ((st = pass_begin(p, ss, d_x, nullptr, d_lik, s))) return st;
     st = fused(p, ss, d_counts, counts_dtype, counts_packed, d_add, d_x, d_bp, true, d_lik, s);
     if (st) return st;
@@ -1335,7 +1347,7 @@ apirl_status apirl_em_pass_host_async(apirl_projector* p, const void* h_counts_s
 
 namespace apirl {
 apirl_status prepare_nz_list(apirl_projector* p, int64_t total) {
-  if (total <= p->nz.cap || !p->is3d || pass_cols(p)) return APIRL_OK;
+  if (total <= p->nz.cap || !p->is3d || (use_cols(p) && !p->nz.order)) return APIRL_OK;
   DEVICE_SCOPE(p->device);
   cudaFree(p->nz.list);
   cudaFree(p->nz.tiles);

@@ -231,3 +231,18 @@ fake.clear()
 _lib.check(lib.apirl_divide_and_backproject(P.h, D, D, D, 0, {nsub}, S))
 done(fake.launches())''')
     assert any("k_scatter_cols" in x for x in names) == cols and any("k_backproject3" in x for x in names) != cols
+
+
+@pytest.mark.parametrize("rings,ns,nsub,cols", [(16, 12, 1, False), (16, 12, 8, True), (40, 12, 1, True), (16, 3, 1, True)])
+def test_sampled_passes_with_few_rays_in_flight_walk_bin_by_bin(gpu, rings, ns, nsub, cols):
+    names = gpu(f'''
+P = ap.SiddonProjector(ImageGeom(64, 64, 31, 2.0, 2.0, 2.0), Sino3DGeom.span1(83, 83, {rings}, 83.0, 64.0, 443.0, 0))
+P.set_sampling({ns}, 1)
+fake.clear()
+for bp in (0, 1):
+    if bp: _lib.check(lib.apirl_em_project_backproject(P.h, D, 0, 0, None, D, D, 0, {nsub}, None, S))
+    else: _lib.check(lib.apirl_em_pass(P.h, D, 0, 0, None, D, D, D, None, 0.0, 0, 0, {nsub}, D, S))
+done(fake.launches())''')
+    assert sum("k_em_cols_rays" in n for n in names) == (2 if cols else 0)
+    assert sum("k_em_pass_rays" in n for n in names) == (0 if cols else 2)
+    assert any("k_col_" in n for n in names) == cols
