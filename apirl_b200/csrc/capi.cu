@@ -850,7 +850,17 @@ namespace {
 // The padded pass on the column layout.  It has one launch form: the options
 // of the padded pair's launch (persistent, block size, gather segments) do not
 // change it, an ordered list keeps to the pair.
-bool pass_cols(const apirl_projector* p, SubsetSel ss) { return (use_cols(p) && !p->nz.order) || use_ray_cols(p, ss); }
+// A pass over every bin of few sinograms on a wide image pays for lists that
+// serve half a warp and leave few blocks on an SM.  Us on the pair -> columns
+// at 1 %, 20 %, 95 % bins with counts: 320 x 320 image, 16 sinograms 224 -> 355,
+// 284 -> 430, 360 -> 433; 24 sinograms 298 -> 392, 384 -> 461, 481 -> 464; 256 x
+// 256, 18 sinograms 162 -> 187, 196 -> 220, 224 -> 221; 160 x 160, 16 sinograms
+// 197 -> 246, 261 -> 306, 333 -> 310.  The line lies where full data take the
+// same time.
+bool wide_pass(const apirl_projector* p) { return p->g.nx + p->g.ny > 27 * p->t.n_sinos; }
+bool pass_cols(const apirl_projector* p, SubsetSel ss, bool listed) {
+  return (use_cols(p) && (listed ? !p->nz.order : !wide_pass(p))) || use_ray_cols(p, ss);
+}
 const apirl::ColBuffers& pass_layout(const apirl_projector* p) { return p->t.lor_s ? p->ray_cols : p->cols; }
 
 // Before the padded pass: the image into its copy.  After it: the update of x
@@ -858,7 +868,7 @@ const apirl::ColBuffers& pass_layout(const apirl_projector* p) { return p->t.lor
 // carry the likelihood's dot product and sum too.
 apirl_status pass_begin(apirl_projector* p, SubsetSel ss, const float* d_x, const float* d_zimg, double* d_lik,
                         cudaStream_t s) {
-  if (pass_cols(p, ss))
+  if (pass_cols(p, ss, d_zimg != nullptr))
     CK(apirl::launch_col_copy(p->g, pass_layout(p), d_x, pass_layout(p).img, s, d_lik ? d_zimg : nullptr,
                               p->d_partials + apirl::col_partials(p->t, ss), d_zimg ? p->queue.n : nullptr));
   else
@@ -868,7 +878,7 @@ apirl_status pass_begin(apirl_projector* p, SubsetSel ss, const float* d_x, cons
 apirl_status pass_end(apirl_projector* p, SubsetSel ss, int mode, float* d_x, float* d_bp, const float* d_sens,
                       const float* d_thr, float thr_value, int ge, const float* d_zimg, const double* d_zero_add,
                       double* d_lik, cudaStream_t s) {
-  if (pass_cols(p, ss)) {
+  if (pass_cols(p, ss, d_zimg != nullptr)) {
     const int64_t lors = (int64_t)ss.nk * p->t.n_r;  // no LORs: no partials written
     const int64_t n = lors ? apirl::col_partials(p->t, ss) + (d_zimg ? apirl::col_dots(p->g) : 0) : 0;
     CK(apirl::launch_col_reduce(p->g, pass_layout(p), pass_layout(p).acc, mode, d_x, d_bp, d_sens, d_thr, thr_value, ge, s,
@@ -894,7 +904,7 @@ apirl_status fused(apirl_projector* p, SubsetSel ss, const void* d_counts, int d
   }
   if (dual && p->t.lor_s) {
     CK(apirl::launch_em_cols_rays(p->g, p->ray_cols, p->t, ss, d_counts, dtype, packed, d_add, 1, p->d_partials, s));
-  } else if (dual && pass_cols(p, ss)) {
+  } else if (dual && pass_cols(p, ss, d_zimg != nullptr)) {
     CK(apirl::launch_em_cols(p->g, p->cols, p->t, ss, d_counts, dtype, packed, d_add, 1, p->d_partials,
                              d_zimg ? (p->sparse_image ? 2 : 1) : 0, p->queue, s));
   } else if (p->planar.lim) {

@@ -246,3 +246,19 @@ done(fake.launches())''')
     assert sum("k_em_cols_rays" in n for n in names) == (2 if cols else 0)
     assert sum("k_em_pass_rays" in n for n in names) == (0 if cols else 2)
     assert any("k_col_" in n for n in names) == cols
+
+
+@pytest.mark.parametrize("n,rings,cols", [(320, 16, False), (320, 24, True), (256, 18, False), (128, 16, True)])
+def test_full_passes_of_few_sinograms_on_wide_images_take_the_pair(gpu, n, rings, cols):
+    names = gpu(f'''
+P = ap.SiddonProjector(ImageGeom({n}, {n}, 31, 2.0, 2.0, 2.0), Sino3DGeom.span1(20, 83, {rings}, {n}.0, 64.0, 900.0, 0))
+P.set_option(_lib.APIRL_OPT_SPARSE_IMAGE, _lib.APIRL_SPARSE_GEOMETRY)
+fake.clear()
+_lib.check(lib.apirl_em_pass(P.h, D, 0, 0, None, D, D, D, None, 0.0, 0, -1, 1, D, S))
+full = fake.launches()
+fake.clear()
+_lib.check(lib.apirl_em_pass_sparse(P.h, D, 0, 0, None, D, D, D, D, None, None, 0.0, 0, -1, 1, D, S))
+done([full, fake.launches()])''')
+    assert any("k_em_cols" in x for x in names[0]) == cols and any("k_em_pass_persist" in x for x in names[0]) != cols
+    assert any("k_col_" in x for x in names[0]) == cols
+    assert any("k_em_cols_listed" in x for x in names[1])
