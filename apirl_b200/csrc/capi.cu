@@ -309,11 +309,11 @@ apirl_status finish_create(apirl_projector* p, apirl_projector** out) {
     at_scalars = b.add(8 * sizeof(double));
     at_chunk = b.add(sizeof(unsigned long long) + 2 * sizeof(unsigned));  // and the queue's numbers
     const bool queue = more && n;
-    const size_t deferred = std::min<size_t>(lors, apirl::kColDirectLors);
+    const size_t line = (size_t)apirl::col_direct_lors(p->g), deferred = std::min(lors, line);
     at_item = b.add(queue ? deferred * sizeof(uint2) : 0);
     at_list = b.add(queue ? deferred * apirl::kColFew * sizeof(uint16_t) : 0);
     const size_t direct = std::min(apirl::col_direct(p->host.n_sinos), p->host.n_sinos);
-    at_bins = b.add(queue && lors > apirl::kColDirectLors ? lors * direct * sizeof(unsigned) : 0);
+    at_bins = b.add(queue && lors > line ? lors * direct * sizeof(unsigned) : 0);
     at_zeros = b.bytes;
     at_pad = b.add(4 * pv * sizeof(float));
     at_col = b.add((l == apirl::Layouts::kCalls ? 7 : more ? 3 : 0) * n * sizeof(float));

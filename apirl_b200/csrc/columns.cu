@@ -562,7 +562,7 @@ cudaError_t launch_scatter_cols(const ImgGeom& g, const ColBuffers& c, const Lor
   // 605 / 87, 175, 288, 355, 612.  (The listed pass's queue, k_em_cols_direct,
   // gave 50 and 79 us at 5 % of 16 and 34 sinograms, but cost full ones 8 us.)
   // More sinograms have values in most LORs.
-  const int look = lors_of(t, s) > kColDirectLors && t.n_sinos <= kColBlock;
+  const int look = lors_of(t, s) > col_direct_lors(g) && t.n_sinos <= kColBlock;
   k_scatter_cols<<<(unsigned)lors_of(t, s), block_of(t), col_smem(g.nx, g.ny), st>>>(g, dims_of(g, c), t, s, vin, vest,
                                                                                     acc, look);
   return cudaGetLastError();
@@ -605,13 +605,15 @@ static cudaError_t em_cols(const ImgGeom& g, const ColBuffers& c, const LorTable
   // 521, 1054 / 433, 567, 744 / 134, 516, 749; of 34 sinograms 122, 186, 318 /
   // 135, 294, 303 / 73, 164, 259; of 310 sinograms 231, 1001, 2091 / 447, 720,
   // 1294 / 204, 726, 1294.  Between the two kernels lies the walk of the last
-  // rays, 8 us: below 8000 LORs a pass is too short for it (6889 LORs of 310
-  // sinograms, 64 x 64: 95, 144, 225 us without, 61, 152, 233 with; on the
-  // padded pair 103, 188, 336).
-  const int64_t lors = lors_of(t, s);
-  const bool queued = lors > kColDirectLors && t.n_sinos <= kColWindow && lors * t.n_sinos <= INT_MAX;
+  // rays, 8 us: below 8000 LORs, or 1.5e6 LORs times voxels of a row and a
+  // column, a pass is too short for it (6889 LORs of 310 sinograms, 64 x 64: 95,
+  // 144, 225 us without, 61, 152, 233 with; on the padded pair 103, 188, 336;
+  // 6240 of 34 sinograms, 320 x 320: 223, 294, 297 without, 199, 194, 229 with,
+  // 250, 268, 317).
+  const int64_t lors = lors_of(t, s), line = col_direct_lors(g);
+  const bool queued = lors > line && t.n_sinos <= kColWindow && lors * t.n_sinos <= INT_MAX;
   const int direct = queued ? col_direct(t.n_sinos) : 0;
-  const int few = lors > 2 * sms * kColBlocks && lors <= kColDirectLors && t.n_sinos > 4 * kColFew &&
+  const int few = lors > 2 * sms * kColBlocks && lors <= line && t.n_sinos > 4 * kColFew &&
                           t.n_sinos <= kColWindow ? kColFew : 0;
   k_em_cols_listed<CT><<<grid, block_of(t), smem, st>>>(g, d, t, s, counts, counts_packed, add, c.img, c.acc, back,
                                                        partials, skip_zero, few, direct, queue);

@@ -157,12 +157,15 @@ ColBuffers col_layout(const ImgGeom& g, const float* z_ends, int n_ends);
 int64_t col_partials(const LorTable& t, SubsetSel s);
 // What a listed column pass leaves to a second kernel, because listing a LOR's
 // crossings is not worth its few rays (columns.cu, em_cols, has the rules): of
-// up to kColDirectLors LORs, items (LOR of the subset, count) and lists (kColFew
-// sinograms of each); of more, bins (LOR * n_sinos + sinogram) of those with at
-// most col_direct.  n: the numbers of both.
+// up to col_direct_lors LORs, items (LOR of the subset, count) and lists
+// (kColFew sinograms of each); of more, bins (LOR * n_sinos + sinogram) of those
+// with at most col_direct.  n: the numbers of both.
 constexpr int kColWindow = 2048;  // sinograms that a block looks for counts at a time
 constexpr int kColFew = 64;
-constexpr int kColDirectLors = 8000;
+inline int64_t col_direct_lors(const ImgGeom& g) {
+  const int64_t lors = 1500000 / (g.nx + g.ny);
+  return lors < 8000 ? lors : 8000;
+}
 inline int col_direct(int n_sinos) { return n_sinos > 4 * kColFew ? kColFew : n_sinos <= 40 ? 40 : kColFew / 2; }
 struct ColQueue {
   unsigned* n = nullptr;
