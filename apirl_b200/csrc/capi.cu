@@ -861,6 +861,11 @@ bool wide_pass(const apirl_projector* p) { return p->g.nx + p->g.ny > 27 * p->t.
 bool pass_cols(const apirl_projector* p, SubsetSel ss, bool listed) {
   return (use_cols(p) && (listed ? !p->nz.order : !wide_pass(p))) || use_ray_cols(p, ss);
 }
+// Whether the fused pass has one launch form only, which the block size and the
+// gather segments do not change: on the columns, and on the padded 2D layouts.
+bool one_shape(const apirl_projector* p, SubsetSel ss, bool listed) {
+  return p->planar.lim || ((use_dual(p) || p->t.lor_s) && pass_cols(p, ss, listed));
+}
 const apirl::ColBuffers& pass_layout(const apirl_projector* p) { return p->t.lor_s ? p->ray_cols : p->cols; }
 
 // Before the padded pass: the image into its copy.  After it: the update of x
@@ -1138,6 +1143,11 @@ apirl_status apirl_projector_autotune(apirl_projector* p, const void* d_counts, 
                                      int subset, int nsubsets, int repeats, int* best_block, void* stream) {
   apirl_status st = check_em(p, d_counts, counts_dtype, d_x, d_x, subset, nsubsets);
   if (st) return st;
+  if (repeats < 1) repeats = 1;
+  if (one_shape(p, make_subset(p, subset, nsubsets), false)) {  // nothing to choose from
+    if (best_block) *best_block = p->em_block;
+    return APIRL_OK;
+  }
   DEVICE_SCOPE(p->device);
   cudaStream_t s = (cudaStream_t)stream;
   const int64_t nv = (int64_t)p->g.nx * p->g.ny * p->g.nz;
@@ -1151,7 +1161,6 @@ apirl_status apirl_projector_autotune(apirl_projector* p, const void* d_counts, 
   p->timing = 0;
   float best = 1e30f;
   int best_b = p->em_block;
-  if (repeats < 1) repeats = 1;
   for (int c : cands) {
     p->em_block = c;
     CK(cudaMemsetAsync(bp, 0, nv * sizeof(float), s));
@@ -1196,8 +1205,11 @@ apirl_status apirl_projector_autotune_ex(apirl_projector* p, const void* d_count
   cudaEvent_t a = nullptr, b = nullptr;
   cudaError_t ce = cudaEventCreate(&a);
   if (ce == cudaSuccess) ce = cudaEventCreate(&b);
-  const int blocks[] = {64, 96, 128, 192, 256};
-  const int unrolls[] = {4, 6, 8};
+  std::vector<int> blocks{64, 96, 128, 192, 256}, unrolls{4, 6, 8};
+  if (one_shape(p, make_subset(p, subset, nsubsets), d_zimg != nullptr)) {  // the one there is, timed
+    blocks = {p->em_block};
+    unrolls = {p->pad.unroll};
+  }
   const int saved_timing = p->timing, saved_block = p->em_block, saved_unroll = p->pad.unroll;
   p->timing = 0;
   float best = 1e30f;
@@ -1243,7 +1255,7 @@ apirl_status apirl_projector_autotune_ex(apirl_projector* p, const void* d_count
   if (ce != cudaSuccess) return cuda_fail(ce, "autotune");
   if (out) {
     out->block = best_b;
-    out->unroll = best_u;
+    out->unroll = best_u ? best_u : d_zimg ? 6 : 4;  // 0: the pass kind's default
     out->ms = best / repeats;
   }
   return APIRL_OK;

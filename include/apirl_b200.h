@@ -252,7 +252,9 @@ apirl_status apirl_projector_set_option(apirl_projector* p, int option, int valu
 apirl_status apirl_projector_kernel_ms(apirl_projector* p, double* ms);
 /* Autotuner: times the fused kernel (apirl_em_project_backproject, `repeats`
  * runs each, on the caller's counts and image) for block sizes 64..256 and
- * keeps the fastest; its size goes to *best_block.  Allocates one scratch image. */
+ * keeps the fastest; its size goes to *best_block.  Allocates one scratch image.
+ * Where the pass has one launch form (column layout, 2D) the block size in
+ * force goes there and nothing runs. */
 apirl_status apirl_projector_autotune(apirl_projector* p, const void* d_counts, int counts_dtype, const float* d_x,
                                      int subset, int nsubsets, int repeats, int* best_block, void* stream);
 /* The launch shape of the persistent fused 3D pass that runs fastest on this
@@ -262,8 +264,9 @@ apirl_status apirl_projector_autotune(apirl_projector* p, const void* d_counts, 
  * `subset` on `stream`: the sparse pass over the bins with counts when
  * d_zimg is given (the zero-count or geometry image, as APIRL_OPT_SPARSE_IMAGE
  * says), else the full pass; the image is not changed.  The projector keeps
- * the fastest; it goes to *out (block, unroll, ms per pass).  Allocates one
- * scratch image.  No counterpart in the reference, whose block sizes come
+ * the fastest; it goes to *out (block, unroll, ms per pass).  Where the pass
+ * runs on the column layout its launch has one form: that is timed, and the
+ * shape in force goes to *out.  Allocates one scratch image.  No counterpart in the reference, whose block sizes come
  * from its .par files (reconGPU/src/CuMlemSinogram3d.cu:157-170). */
 typedef struct {
   int block;

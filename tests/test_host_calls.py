@@ -262,3 +262,24 @@ done([full, fake.launches()])''')
     assert any("k_em_cols" in x for x in names[0]) == cols and any("k_em_pass_persist" in x for x in names[0]) != cols
     assert any("k_col_" in x for x in names[0]) == cols
     assert any("k_em_cols_listed" in x for x in names[1])
+
+
+def test_autotuner_reports_the_shape_in_force_where_there_is_one(gpu):
+    """Passes on the columns ignore block size and gather segments: neither is chosen from the noise of equal passes."""
+    got = gpu(GEOMS + '''
+G = Sino3DGeom.span1(16, 40, 11, 33.0, 22.0, 100.0, 0)   # 11 sinograms: the padded pair
+out = []
+for sg in (G3[1], G):
+    P = ap.SiddonProjector(G3[0], sg)
+    P.set_option(_lib.APIRL_OPT_SPARSE_IMAGE, _lib.APIRL_SPARSE_GEOMETRY)
+    for z in (D, None):
+        fake.clear()
+        tune, block = _lib.TuneC(), ctypes.c_int()
+        _lib.check(lib.apirl_projector_autotune_ex(P.h, D, 0, D, z, -1, 1, 2, ctypes.byref(tune), S))
+        passes = sum("k_em" in n for n in fake.launches())
+        fake.clear()
+        _lib.check(lib.apirl_projector_autotune(P.h, D, 0, D, -1, 1, 2, ctypes.byref(block), S))
+        out.append([tune.block, tune.unroll, passes, block.value, sum("k_em" in n for n in fake.launches())])
+done(out)''')
+    assert got[:2] == [[128, 6, 3, 128, 0], [128, 4, 3, 128, 0]]
+    assert got[2][2] == got[3][2] == 45 and got[2][4] == got[3][4] == 15
