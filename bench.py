@@ -44,13 +44,12 @@ TOTAL_COUNTS = 5e8
 # within three more passes.  The passes do the same work either way.
 UPDATE_GE = False
 L2_FLUSH_BYTES = 256 << 20
-# DRAM bytes (read + write) per fused-kernel launch of the full workload,
-# mean of the four timed launches captured with ncu --metrics dram__bytes_read.sum,
-# dram__bytes_write.sum (one pass; profiles/k_em_pass_osem3d_256x256x81.md).
-FULL_TRAFFIC_BYTES = 2.603e8
-# The same for the nonzero pass (the default): mean of the three timed
-# launches inside the capture's first 400 launches.
-NONZERO_TRAFFIC_BYTES = 1.498e8
+# DRAM bytes (read + write) of a pass's fused kernels on the full workload, from
+# ncu --metrics dram__bytes_read.sum,dram__bytes_write.sum (one pass):
+# the column walk's (profiles/column_walk.md; the listed pass with the kernel
+# of its queue), and the padded pair's (profiles/k_em_pass_osem3d_256x256x81.md).
+TRAFFIC_BYTES = {("k_em_cols", "full"): 1.395e8, ("k_em_cols_listed", "nonzero"): 1.297e8,
+                 ("k_em_pass_persist", "full"): 2.603e8, ("k_em_pass_persist", "nonzero"): 1.498e8}
 WORKLOAD = ("3D OSEM 256x256x81 image, 41 rings span-1 |rd|<=20: 1261 sinograms x 336 angles x 336 r, "
             "21 subsets, attenuation in sensitivity, 5e8 counts uint32")
 
@@ -179,6 +178,23 @@ def step_bytes(w, s, sparse=False):
     return kern, kern + 20 * w["ig"].n_voxels
 
 
+def walking_kernel(listed, alpha="f32", pair=False):
+    """The fused kernel of a pass: the column walk's, or the padded pair's where
+    an option keeps to it (csrc/capi.cu, pass_cols)."""
+    if alpha != "f32":
+        return "k_em_pass"
+    return "k_em_pass_persist" if pair else "k_em_cols_listed" if listed else "k_em_cols"
+
+
+def keeps_pair(args):
+    return bool(args.l2_persist or args.list_order or args.accumulate != "atomic")
+
+
+def measured_traffic(kernel, pass_form, whole=True):
+    """DRAM bytes of that kernel's launch where they were measured (whole: the full workload), else None."""
+    return TRAFFIC_BYTES.get((kernel, pass_form)) if whole else None
+
+
 def whole_job_value(steps, local_ms, world, dist=None, device=None):
     """Whole-job throughput of `world` replicas that each ran `steps` steps in
     `local_ms` of device time: steps * world / (max over ranks of the time).
@@ -275,7 +291,7 @@ def run_sharded(args):
                        "pass": ("nonzero: each shard walks its bins with counts, its likelihood part from its "
                                 "geometry images A_s^T 1 (set-up)") if nonzero else "full: every bin walked",
                        "update": "x*bp/sens where sens > 0"},
-            "roofline": {"bound": "hbm", "kernel": "k_em_cols on rank 0's shard",
+            "roofline": {"bound": "hbm", "kernel": walking_kernel(nonzero) + " on rank 0's shard",
                          "kernel_ms": statistics.mean(kern), "peak": peak, "unit": "GB/s",
                          "peak_source": f"{peak_kind} hbm_gbs",
                          "achieved": achieved, "frac": achieved / peak, "traffic": None},
@@ -321,7 +337,7 @@ def run_gpu(args):
         best_block = P.autotune(counts, x, 0, NSUB, repeats=2, stream=stream)
     bp.zero_()
     torch.cuda.synchronize(dev)
-    log(f"autotuned fused-kernel block size: {best_block}")
+    log(f"fused-kernel block size (padded pair): {best_block}")
     P.set_option(_l.APIRL_OPT_KERNEL_TIMING, 1)
     P.set_option(_l.APIRL_OPT_PERSISTENT, args.persistent)
     if args.l2_persist:
@@ -358,8 +374,8 @@ def run_gpu(args):
                                                               repeats=2, stream=stream)
         bp.zero_()
         torch.cuda.synchronize(dev)
-        log(f"autotuned listed pass: {best_block} threads per block, {gather_unroll} segments in flight, "
-            f"{tune_ms:.3f} ms")
+        log(f"listed pass: {tune_ms:.3f} ms (shape on the padded pair: {best_block} threads per block, "
+            f"{gather_unroll} segments in flight)")
 
     def zero_images():
         # Per-subset zero-count images of the sparse pass (once per
@@ -434,18 +450,17 @@ def run_gpu(args):
             f_ach = fb / (statistics.mean(fkern) / 1e3) / 1e9
             full_cmp = {"value": f_value, "unit": UNIT, "kernel_ms": statistics.mean(fkern),
                         "roofline_achieved": f_ach, "roofline_frac": f_ach / peaks()[0],
-                        "traffic": FULL_TRAFFIC_BYTES if args.max_ring_diff is None else None,
+                        "traffic": measured_traffic(walking_kernel(False, args.alpha, keeps_pair(args)), "full",
+                                                    args.max_ring_diff is None),
                         "pass": "full: every bin walked, every estimate summed (--pass full)"}
     step_ms = [evs[i][0].elapsed_time(evs[i][1]) for i in range(args.steps)]
     pre_ms = pre[0].elapsed_time(pre[1]) if sparse else 0.0
     value, total_ms = whole_job_value(args.steps, sum(step_ms) + pre_ms, world, dist if world > 1 else None, dev)
 
     kb = [step_bytes(w, s, skipz) for s in subs]
-    # The kernel that walks: the column walk, or the padded pair's where an
-    # option keeps to it (csrc/capi.cu, pass_cols).
-    pair = args.l2_persist or args.list_order or args.accumulate != "atomic"
-    kernel = ("k_em_pass" if args.alpha != "f32" else "k_em_pass_persist" if pair else
-              "k_em_cols" if args.pass_form == "full" else "k_em_cols_listed")
+    kernel = walking_kernel(skipz, args.alpha, keeps_pair(args))
+    traffic = args.traffic_bytes if args.traffic_bytes is not None else \
+        measured_traffic(kernel, args.pass_form, args.max_ring_diff is None)
     kern_bytes = statistics.mean(k for k, _ in kb)
     kern_s = statistics.mean(kern_ms) / 1e3
     peak, peak_kind = peaks()
@@ -553,8 +568,11 @@ def run_gpu(args):
             "scaling": "weak", "vs_baseline": None, "dtype": "f32", "data": "synthetic (seeded phantom, Poisson counts)",
             "config": {"workload": WORKLOAD if args.max_ring_diff is None else
                        WORKLOAD + f" (profiling case: segments |rd| <= {args.max_ring_diff} only)",
-                       "subsets": NSUB, "counts_dtype": "uint32", "em_block": best_block,
-                       "gather_unroll": gather_unroll if gather_unroll is not None else "default (6 listed, 4 full)",
+                       "subsets": NSUB, "counts_dtype": "uint32",
+                       # the column walk's launch has one form
+                       "em_block": None if kernel.startswith("k_em_cols") else best_block,
+                       "gather_unroll": None if kernel.startswith("k_em_cols") else
+                       gather_unroll if gather_unroll is not None else "default (6 listed, 4 full)",
                        "alpha": args.alpha, "persistent": args.persistent, "accumulate": args.accumulate,
                        "l2_persist": bool(args.l2_persist), "list_order": args.list_order,
                        "pass": ("sparse: bins with zero counts not walked, their likelihood terms -x.Z_s from "
@@ -573,9 +591,10 @@ def run_gpu(args):
             "full_pass": full_cmp,
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak,
-                         "traffic": args.traffic_bytes if args.traffic_bytes is not None else
-                         ({"full": FULL_TRAFFIC_BYTES, "nonzero": NONZERO_TRAFFIC_BYTES}.get(args.pass_form)
-                          if args.max_ring_diff is None else None),
+                         "counts": "4 B a forward and 8 B a backward segment, whichever memory serves them (the "
+                                   "images stay in L1 and L2): not a share of the DRAM's bandwidth",
+                         "traffic": traffic,
+                         "dram_frac": None if traffic is None else traffic / kern_s / 1e9 / peak,
                          "kernel": kernel + " (fused projection / ratio / backprojection)",
                          "timing": "CUDA events recorded by the library on the launching stream around the fused "
                                    "kernels",
@@ -1170,7 +1189,7 @@ def main():
     ap_.add_argument("--budget-gb", type=float, default=96.0)
     ap_.add_argument("--traffic-bytes", type=float, default=None,
                      help="DRAM bytes per fused-kernel launch from an ncu capture, reported as roofline.traffic "
-                          f"(default for the full workload: {FULL_TRAFFIC_BYTES:.3g})")
+                          "(default: those measured for the kernel that runs on the full workload)")
     args = ap_.parse_args()
     if args.warmup < 3 and args.impl != "reference":
         args.warmup = 3

@@ -26,3 +26,16 @@ def test_fifo_takes_arrival_order_not_index_order():
     # served as job 1 (0..3), job 2 (3..4), job 0 (5..6)
     assert np.allclose(finish, [6.0, 3.0, 4.0])
     assert np.allclose(lat, [1.0, 3.0, 3.0])
+
+
+def test_traffic_belongs_to_the_kernel_that_ran():
+    """The DRAM bytes printed beside a kernel were measured on that kernel."""
+    assert bench.walking_kernel(True) == "k_em_cols_listed" and bench.walking_kernel(False) == "k_em_cols"
+    assert bench.walking_kernel(True, pair=True) == "k_em_pass_persist"
+    assert bench.walking_kernel(False, alpha="f64") == "k_em_pass"
+    values = [bench.measured_traffic(bench.walking_kernel(f == "nonzero", pair=p), f)
+              for f in ("full", "nonzero") for p in (False, True)]
+    assert len(set(values)) == 4 and all(1e8 < v < 3e8 for v in values)
+    assert bench.measured_traffic("k_em_pass", "full") is None
+    assert bench.measured_traffic(bench.walking_kernel(True), "sparse") is None
+    assert bench.measured_traffic(bench.walking_kernel(True), "nonzero", whole=False) is None
