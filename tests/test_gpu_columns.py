@@ -45,7 +45,8 @@ def _gpu():
     ap.load_library()
 
 
-# image, sinogram: at least 1e7 bins x (nx + ny), so that project takes the columns
+# image, sinogram (their passes and backprojections take the columns; the
+# projections that do are in column_cases.py)
 CASES = {
     "16 sinograms": (ImageGeom(96, 96, 31, 2.08, 2.08, 2.03), Sino3DGeom.span1(40, 90, 16, 99.84, 16 * 4.06, 200.0, 0)),
     "31 sinograms": (ImageGeom(64, 64, 21, 2.08, 2.08, 2.03), Sino3DGeom.span1(36, 80, 11, 66.56, 11 * 4.054, 200.0, 1)),

@@ -83,3 +83,30 @@ def test_image_of_several_slices(oracle):
     got = x.cpu().numpy()
     assert rel(got[:n], want) <= 1e-5
     assert not got[n:].any()
+
+
+def test_pass_with_additive_term(oracle):
+    """An additive term in the counts' layout, whole and packed to a subset."""
+    ig, sg = ImageGeom(33, 40, 1, 2.0, 2.0, 1.0), Sino2DGeom(21, 47, 44.0, 400.0)
+    rng = np.random.default_rng(4)
+    x0 = (rng.random(ig.n_voxels, dtype=np.float32) + 0.5).astype(np.float32)
+    sens = (rng.random(ig.n_voxels, dtype=np.float32) + 1).astype(np.float32)
+    whole = rng.poisson(4.0, 21 * 47).astype(np.float32)
+    add = (rng.random(21 * 47, dtype=np.float32) + 0.1).astype(np.float32)
+    P = ap.SiddonProjector(ig, sg)
+    for sub, nsub, packed in ((-1, 1, False), (1, 3, False), (1, 3, True)):
+        pick = lambda v: v.reshape(21, 47)[max(sub, 0)::nsub].reshape(-1)
+        est = pick((oracle.project_2d(sg, ig, x0) + add).astype(np.float32))
+        m = pick(whole)
+        ratio = np.zeros((21, 47), np.float32)  # the other subsets' bins add nothing
+        ratio[max(sub, 0)::nsub] = oracle.inverse_divide(m, est).reshape(-1, 47)
+        bp = oracle.backproject_2d(sg, ig, ratio.reshape(-1))
+        want = oracle.update(x0, bp, sens, np.float32(0), False)
+        e64 = est[est > 0].astype(np.float64)
+        want_lik = float(np.sum(m[est > 0] * np.log(e64) - e64))
+        x, lik = t(x0), torch.zeros(1, dtype=torch.float64, device=DEV)
+        a, c = (pick(add), m) if packed else (add, whole)
+        P.em_pass(t(c), x, torch.zeros(ig.n_voxels, dtype=torch.float32, device=DEV), t(sens), sub, nsub, add=t(a),
+                  ge=False, counts_packed=packed, lik=lik)
+        assert rel(x.cpu().numpy(), want) <= 1e-5
+        assert abs(lik.item() - want_lik) <= 1e-9 * abs(want_lik)

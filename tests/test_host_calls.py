@@ -283,3 +283,18 @@ for sg in (G3[1], G):
 done(out)''')
     assert got[:2] == [[128, 6, 3, 128, 0], [128, 4, 3, 128, 0]]
     assert got[2][2] == got[3][2] == 45 and got[2][4] == got[3][4] == 15
+
+
+def test_projections_of_the_column_cases_take_the_columns(gpu):
+    got = gpu(f'''
+sys.path.insert(0, {fake_gpu.HERE!r})
+from column_cases import PROJECTED
+out = {{}}
+for name, (ig, sg, sub, nsub) in PROJECTED.items():
+    P = ap.SiddonProjector(ig, sg)
+    fake.clear()
+    _lib.check(lib.apirl_project(P.h, D, D, -1, 1, S))
+    _lib.check(lib.apirl_project(P.h, D, D, sub, nsub, S))
+    out[name] = sum("k_project_cols" in n for n in fake.launches())
+done(out)''')
+    assert got and all(n == 2 for n in got.values()), got
