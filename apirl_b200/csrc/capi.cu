@@ -174,13 +174,18 @@ apirl_status capturing(cudaStream_t s, bool* is) {
 // bins, 19 sinograms 153 -> 123 (columns), 91 sinograms 616 -> 247 (columns);
 // 134 x 134 image, 344 bins, 34 sinograms 285 -> 373 (direct); 82 x 82, 344
 // bins, 47 sinograms 83 -> 92 (direct); 58 x 58, 344 bins, 139 sinograms 175 ->
-// 169 (columns).  Below 1e7 bins times voxels of a row and a column, the copy's
+// 169 (columns).  With one warp a block, the lists of images wider than 160 x
+// 160 leave fewer blocks on an SM than there is room for warps: measured over
+// the estimate 0.98 at 160 x 160, 1.16 at 192 x 192, 1.40 at 224 x 224, 1.57 at
+// 256 x 256 (16 sinograms, all angles, 765 -> 925 us; two warps a block 1.01).
+// Below 1e7 bins times voxels of a row and a column, the copy's
 // launch costs more than the walk gains (48 x 48 image, 57 K bins: 16.5 -> 18.6).
 bool project_cols(const apirl_projector* p, SubsetSel ss) {
   const double side = (double)p->g.nx + p->g.ny;
   if ((double)p->t.n_sinos * ss.nk * p->t.n_r * side < 1e7) return false;
   const double pitch = 2.0 * p->r_fov / p->t.n_r / p->g.dx, steps = 0.65 * side;
-  const double cols = 2600 + (p->t.n_sinos + 31) / 32 * (250 + 17 * steps);
+  const double crowded = p->t.n_sinos <= 32 ? std::max(1.0, side / 323) : 1;
+  const double cols = crowded * (2600 + (p->t.n_sinos + 31) / 32 * (250 + 17 * steps));
   const double direct = p->t.n_sinos / 32.0 * (300 + steps * (26 + 34 * (pitch < 1 ? pitch : 1)));
   return cols <= direct;
 }
@@ -856,10 +861,14 @@ namespace {
 // 284 -> 430, 360 -> 433; 24 sinograms 298 -> 392, 384 -> 461, 481 -> 464; 256 x
 // 256, 18 sinograms 162 -> 187, 196 -> 220, 224 -> 221; 160 x 160, 16 sinograms
 // 197 -> 246, 261 -> 306, 333 -> 310.  The line lies where full data take the
-// same time.
-bool wide_pass(const apirl_projector* p) { return p->g.nx + p->g.ny > 27 * p->t.n_sinos; }
+// same time; in long passes, where neither layout's launches count, at more
+// sinograms (230 x 230, 19 sinograms: 89 K LORs 642 -> 913 us at 5 %, 931 ->
+// 1044 full, 11 K LORs 149 -> 161, 188 -> 180).
+bool wide_pass(const apirl_projector* p, SubsetSel ss) {
+  return p->g.nx + p->g.ny > ((int64_t)ss.nk * p->t.n_r > 20000 ? 20 : 27) * p->t.n_sinos;
+}
 bool pass_cols(const apirl_projector* p, SubsetSel ss, bool listed) {
-  return (use_cols(p) && (listed ? !p->nz.order : !wide_pass(p))) || use_ray_cols(p, ss);
+  return (use_cols(p) && (listed ? !p->nz.order : !wide_pass(p, ss))) || use_ray_cols(p, ss);
 }
 // Whether the fused pass has one launch form only, which the block size and the
 // gather segments do not change: on the columns, and on the padded 2D layouts.

@@ -298,3 +298,26 @@ for name, (ig, sg, sub, nsub) in PROJECTED.items():
     out[name] = sum("k_project_cols" in n for n in fake.launches())
 done(out)''')
     assert got and all(n == 2 for n in got.values()), got
+
+
+def _few_on_wide(n, rings, max_rd, nsub, call):
+    nr = int(1.3 * n + 0.5)
+    return f'''
+P = ap.SiddonProjector(ImageGeom({n}, {n}, 9, 2.0, 2.0, 2.0), Sino3DGeom.span1({nr}, {nr}, {rings}, {nr}.0, 20.0, 443.0, {max_rd}))
+fake.clear()
+_lib.check({call.format(sub=0 if nsub > 1 else -1, nsub=nsub)})
+done(fake.launches())'''
+
+
+@pytest.mark.parametrize("n,rings,max_rd,nsub,cols", [(256, 16, 0, 1, False), (230, 5, 2, 1, False), (256, 24, 0, 1, True),
+                                                      (128, 18, 0, 1, True), (256, 40, 0, 4, True)])
+def test_projections_of_few_sinograms_on_wide_images(gpu, n, rings, max_rd, nsub, cols):
+    names = gpu(_few_on_wide(n, rings, max_rd, nsub, "lib.apirl_project(P.h, D, D, {sub}, {nsub}, S)"))
+    assert any("k_project_cols" in x for x in names) == cols
+
+
+@pytest.mark.parametrize("n,rings,max_rd,nsub,cols", [(230, 5, 2, 1, False), (230, 5, 2, 8, True), (256, 28, 0, 1, True)])
+def test_long_full_passes_of_few_sinograms(gpu, n, rings, max_rd, nsub, cols):
+    names = gpu(_few_on_wide(n, rings, max_rd, nsub,
+                             "lib.apirl_em_pass(P.h, D, 0, 0, None, D, D, D, None, 0.0, 0, {sub}, {nsub}, D, S)"))
+    assert any("k_em_cols" in x for x in names) == cols
