@@ -1404,7 +1404,7 @@ cudaError_t backproject_sino(apirl_projector* p, SubsetSel ss, const float* vin,
   // x . G_s, by 5.6e-8 (one sum) or 1e-8 (two) of its value; the pair's, made
   // once per geometry, by 6e-9.
   if (use_cols(p) && vin_mode == 0) {
-    const cudaError_t e = launch_scatter_cols(p->g, p->cols, p->t, ss, vin, nullptr, p->cols.acc, st);
+    const cudaError_t e = launch_scatter_cols(p->g, p->cols, p->t, ss, vin, nullptr, p->cols.acc, st, p->queue);
     if (e != cudaSuccess) return e;
     return launch_col_reduce(p->g, p->cols, p->cols.acc, 1, nullptr, img, nullptr, nullptr, 0.f, 0, st);
   }

@@ -45,6 +45,7 @@ constexpr int kColFewBlocks = 20;
 constexpr int kColDirectBlock = 64;
 constexpr int kColDirectBlocks = 16;
 constexpr int kColDirectU = 8;
+constexpr int kColDirectBack = 8;  // values of a LOR that a backprojection walks so
 // Blocks of the batched pass, whose LORs have from a few to hundreds of
 // counts: ten mixed jobs of 64 - 128 x 1 - 41 slices in 16.7 ms, against 18.0 /
 // 17.6 / 17.8 / 20.4 ms with 64 / 96 / 160 / 256 threads and 18.1 ms at 8 blocks
@@ -81,16 +82,28 @@ struct ColScatterDivide {
 // bins with v == 0 add nothing) and, with vest, DivideAndBackproject's
 // (:669-683: (seg * v) / e where e != 0, else seg * v).  The ratio v / e is
 // formed once per bin where v and the ratio are far from the ends of the
-// float range, and per segment elsewhere.  look (a thread a sinogram): a LOR
-// without values is left before its crossings are listed.
+// float range, and per segment elsewhere.  look >= 0 (a thread a sinogram): a
+// LOR without values is left before its crossings are listed, and the bins of
+// one with at most `look` go to the queue (k_scatter_cols_direct).
 __global__ void __launch_bounds__(kColBlock, kColBlocks) k_scatter_cols(ImgGeom g, ColDims d, LorTable t, SubsetSel s,
                                                                         const float* __restrict__ vin,
                                                                         const float* __restrict__ vest,
-                                                                        float* __restrict__ acc, int look) {
+                                                                        float* __restrict__ acc, int look,
+                                                                        ColQueue queue) {
   const ColLor lor = col_lor(t, s, blockIdx.x);
-  if (look) {
+  if (look >= 0) {
     const int gl = threadIdx.x;
-    if (!__syncthreads_or(gl < t.n_sinos && __ldg(vin + ((int64_t)gl * s.nk + lor.k) * t.n_r + lor.l) != 0.f)) return;
+    const bool any = gl < t.n_sinos && __ldg(vin + ((int64_t)gl * s.nk + lor.k) * t.n_r + lor.l) != 0.f;
+    const int n = __syncthreads_count(any);
+    if (n == 0) return;
+    if (n <= look) {
+      const unsigned mask = __ballot_sync(0xffffffffu, any), lane = threadIdx.x & 31;
+      unsigned slot = 0;
+      if (lane == 0 && mask) slot = atomicAdd(queue.n + 1, (unsigned)__popc(mask));
+      slot = __shfl_sync(0xffffffffu, slot, 0);
+      if (any) queue.bins[slot + __popc(mask & ((1u << lane) - 1u))] = blockIdx.x * (unsigned)t.n_sinos + gl;
+      return;
+    }
   }
   const float4 P = __ldg(t.lor + (int64_t)lor.a * t.n_r + lor.l);
   col_list(P, g, d);
@@ -121,6 +134,27 @@ __global__ void __launch_bounds__(kColBlock, kColBlocks) k_scatter_cols(ImgGeom 
     ColScatter add{in ? v : 0.f};
     if (w.listed) col_walk(in ? col_setup_z(e, w, g, d) : col_no_ray(), d, acc, add);
     else if (in) col_walk_checked(P, e, g, d, acc, add);
+  }
+}
+
+// A backprojection's queued bins, a lane each.
+__global__ void __launch_bounds__(kColDirectBlock, kColDirectBlocks) k_scatter_cols_direct(
+    ImgGeom g, ColDims d, LorTable t, SubsetSel s, const float* __restrict__ vin, float* __restrict__ acc,
+    ColQueue queue) {
+  const unsigned bins = queue.n[1], last = (unsigned)d.floats() - 1u;
+  for (unsigned b = blockIdx.x * blockDim.x + threadIdx.x; b < bins; b += gridDim.x * blockDim.x) {
+    const unsigned bin = queue.bins[b], at = bin / (unsigned)t.n_sinos;
+    const ColLor lor = col_lor(t, s, at);
+    const int gl = (int)(bin - at * (unsigned)t.n_sinos);
+    const float4 P = __ldg(t.lor + (int64_t)lor.a * t.n_r + lor.l);
+    const float2 ez = __ldg(t.z + t.g0 + gl);
+    const float v = __ldg(vin + ((int64_t)gl * s.nk + lor.k) * t.n_r + lor.l);
+    ColWalk w;
+    col_setup_xy(P, g, d, w);
+    float* const sums = acc + (w.xmain ? d.floats() : 0);
+    ColScatter add{v};
+    if (w.listed) col_ray_scatter(ColRay(w, col_setup_z(ez, w, g, d)), last, v, sums);
+    else col_walk_checked(P, ez, g, d, sums, add);
   }
 }
 
@@ -551,20 +585,34 @@ cudaError_t launch_project_cols(const ImgGeom& g, const ColBuffers& c, const Lor
 }
 
 cudaError_t launch_scatter_cols(const ImgGeom& g, const ColBuffers& c, const LorTable& t, SubsetSel s,
-                                const float* vin, const float* vest, float* acc, cudaStream_t st) {
-  if (lors_of(t, s) == 0) return cudaSuccess;
+                                const float* vin, const float* vest, float* acc, cudaStream_t st,
+                                const ColQueue& queue) {
+  const int64_t lors = lors_of(t, s);
+  if (lors == 0) return cudaSuccess;
   // Looking costs 1.6 us where every LOR has values and many are walked, 2 us
   // of 25 in short calls.  Backprojections of 27,556 LORs of a 128 x 128 image,
   // us on the padded pair / without / with, bins with values 0.2 %, 1 %, 5 %,
   // 20 %, all: 16 sinograms 33, 43, 62, 78, 178 / 60, 66, 84, 97, 99 / 36, 42, 71,
   // 97, 101; 34 sinograms 42, 55, 99, 130, 318 / 82, 102, 141, 157, 184 / 39, 67,
   // 134, 158, 186; 146 sinograms 110, 148, 344, 478, 1296 / 126, 179, 278, 344,
-  // 605 / 87, 175, 288, 355, 612.  (The listed pass's queue, k_em_cols_direct,
-  // gave 50 and 79 us at 5 % of 16 and 34 sinograms, but cost full ones 8 us.)
-  // More sinograms have values in most LORs.
-  const int look = lors_of(t, s) > col_direct_lors(g) && t.n_sinos <= kColBlock;
-  k_scatter_cols<<<(unsigned)lors_of(t, s), block_of(t), col_smem(g.nx, g.ny), st>>>(g, dims_of(g, c), t, s, vin, vest,
-                                                                                    acc, look);
+  // 605 / 87, 175, 288, 355, 612.  More sinograms have values in most LORs.
+  const bool look = lors > col_direct_lors(g) && t.n_sinos <= kColBlock;
+  // The queue, for LORs with up to 8 values (the list serves one walk, whose
+  // reductions cost more lane by lane), costs 6 us more: there it gave 50, 89 and
+  // 79, 141 us at 5 %, 20 % of 16 and 34 sinograms.  It is for long calls, from
+  // 1e7 LORs times voxels of a row and a column on: 89,401 LORs of 19 sinograms,
+  // 230 x 230, 5 % and all: pair 250, 913, without 359, 581, with 173, 588.
+  const bool queued = look && !vest && queue.bins && (double)lors * (g.nx + g.ny) >= 1e7 && lors * t.n_sinos <= INT_MAX;
+  cudaError_t e;
+  if (queued && (e = cudaMemsetAsync(queue.n + 1, 0, sizeof(unsigned), st)) != cudaSuccess) return e;
+  k_scatter_cols<<<(unsigned)lors, block_of(t), col_smem(g.nx, g.ny), st>>>(
+      g, dims_of(g, c), t, s, vin, vest, acc, queued ? kColDirectBack : look ? 0 : -1, queue);
+  if ((e = cudaGetLastError()) != cudaSuccess || !queued) return e;
+  int dev = 0, sms = 0;
+  if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
+  if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
+  k_scatter_cols_direct<<<(unsigned)(sms * kColDirectBlocks), kColDirectBlock, 0, st>>>(g, dims_of(g, c), t, s, vin, acc,
+                                                                                      queue);
   return cudaGetLastError();
 }
 

@@ -185,9 +185,11 @@ cudaError_t launch_col_reduce(const ImgGeom& g, const ColBuffers& c, float* acc,
                               double* lik = nullptr);
 cudaError_t launch_project_cols(const ImgGeom& g, const ColBuffers& c, const LorTable& t, SubsetSel s,
                                 const float* img, float* out, cudaStream_t st);
-// acc += A_s^T v (a subset sinogram); vest: DivideAndBackproject's rule.
+// acc += A_s^T v (a subset sinogram); vest: DivideAndBackproject's rule.  With
+// a queue the bins of LORs with few values may be walked one a lane.
 cudaError_t launch_scatter_cols(const ImgGeom& g, const ColBuffers& c, const LorTable& t, SubsetSel s,
-                                const float* vin, const float* vest, float* acc, cudaStream_t st);
+                                const float* vin, const float* vest, float* acc, cudaStream_t st,
+                                const ColQueue& queue = ColQueue());
 // The fused kernels, one partial per col_partials.  skip_zero as the kernels'
 // (0: every bin is walked); else queue.n is 0 before (launch_col_copy).
 cudaError_t launch_em_cols(const ImgGeom& g, const ColBuffers& c, const LorTable& t, SubsetSel s, const void* counts,

@@ -94,3 +94,19 @@ def test_backprojection_of_few_values(oracle, rings, max_rd, n_proj, n_r, nsub, 
             assert np.array_equal(got, x0)
         else:
             assert np.linalg.norm(got - (x0.astype(np.float64) + want)) <= 1e-5 * np.linalg.norm(want) + 1e-6
+
+
+@pytest.mark.parametrize("rings", [16, 33])
+@pytest.mark.parametrize("share", [0.01, 0.3, 1.0])
+def test_long_backprojection_of_few_values(oracle, rings, share):
+    """Calls so long that the bins of LORs with up to 8 values are queued, some
+    of them past the image, beside LORs with more; twice."""
+    ig = ImageGeom(200, 190, 5, 2.0, 2.0, 2.0)
+    sg = Sino3DGeom.span1(116, 230, rings, 230.0, rings * 0.7, 400.0, 0)
+    rng = np.random.default_rng(rings)
+    v = ((rng.random(sg.n_bins, dtype=np.float32) + 0.5) * (rng.random(sg.n_bins) < share)).astype(np.float32)
+    want = oracle.backproject_3d(sg, ig, v, threads=1)
+    P = ap.SiddonProjector(ig, sg)
+    for _ in range(2):
+        got = P.backproject(t(v), torch.zeros(ig.n_voxels, dtype=torch.float32, device=DEV)).cpu().numpy()
+        assert rel(got, want) <= 1e-5

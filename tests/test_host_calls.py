@@ -321,3 +321,14 @@ def test_long_full_passes_of_few_sinograms(gpu, n, rings, max_rd, nsub, cols):
     names = gpu(_few_on_wide(n, rings, max_rd, nsub,
                              "lib.apirl_em_pass(P.h, D, 0, 0, None, D, D, D, None, 0.0, 0, {sub}, {nsub}, D, S)"))
     assert any("k_em_cols" in x for x in names) == cols
+
+
+@pytest.mark.parametrize("n,rings,n_proj,n_r,want", [(200, 16, 116, 230, True), (200, 257, 116, 230, False), (64, 16, 116, 230, False)])
+def test_long_backprojections_queue_lors_with_few_values(gpu, n, rings, n_proj, n_r, want):
+    log = gpu(f'''
+P = ap.SiddonProjector(ImageGeom({n}, 190, 5, 2.0, 2.0, 2.0), Sino3DGeom.span1({n_proj}, {n_r}, {rings}, 230.0, 11.0, 400.0, 0))
+fake.clear()
+_lib.check(lib.apirl_backproject(P.h, D, D, -1, 1, S))
+done(fake.log())''')
+    assert any("k_scatter_cols_direct" in l for l in log) == want
+    assert any(l.startswith("memset 0x9990") for l in log) == want  # the queue is emptied on the caller's stream
