@@ -28,7 +28,7 @@ namespace {
 // Eight warps, so that a list serves many sinograms, at 5 blocks an SM (48
 // registers): the full pass of that job 1.71 ms, against 1.80 / 1.79 / 1.77 /
 // 2.03 ms with 128 / 192 / 320 / 512 threads and 1.82 ms at 4 blocks (64
-// registers).
+// registers, without the 56 bytes that k_em_cols spills here).
 constexpr int kColBlock = 256;
 constexpr int kColBlocks = 5;
 // With several rays a bin and as many lists to make, blocks of up to 16 warps:

@@ -156,8 +156,9 @@ apirl_status apirl_projector_set_alpha_precision(apirl_projector* p, int mode);
  * width.  Project and Backproject use the oversampled end points when
  * n_samples != 1, DivideAndBackproject unless both counts are 1 (:628), as the
  * reference does.  (1, 1, 0) restores one ray per bin.  Sampled projectors run
- * the fused pass on one unpadded layout; the FP64-alpha mode and the batch
- * engine take one ray per bin. */
+ * the fused pass on a column layout or one unpadded layout
+ * (APIRL_OPT_DUAL_LAYOUT); the FP64-alpha mode and the batch engine take one
+ * ray per bin. */
 #define APIRL_MAX_SAMPLES 64
 apirl_status apirl_projector_set_sampling(apirl_projector* p, int n_samples, int n_axial_samples,
                                          int multiple_lors_per_bin);
@@ -181,15 +182,24 @@ apirl_status apirl_projector_set_shard(apirl_projector* p, int first_sinogram, i
  *   the order of fp32 additions in the backprojection.  Projectors of 16 or
  *   more sinograms (the shard's) run their passes, projections and
  *   backprojections on a third, column layout instead, [y][x][z], in which a
- *   block walks one (angle, r) for all sinograms (7 more images); sensitivities
- *   and geometry images, and passes with an option that speaks of the padded
- *   layouts (L2 window, list order, another accumulation form than plain
- *   atomics), keep to the two.  Passes with several rays a bin take a column
- *   layout too (3 more images) where the radial samples are few (their
- *   crossing lists fit a block's shared memory: 40 KB, 20 (nx + ny + 11) bytes
- *   a sample); their projections and backprojections walk bin by bin.  The launch options below (block size,
- *   persistent, gather segments) shape the two layouts' kernel; the column
- *   layout's has one shape and takes any setting.
+ *   block walks one (angle, r) for all sinograms, where that is faster (not
+ *   for short calls, and not for projections and full passes of few sinograms
+ *   on wide images); sensitivities and geometry images, and passes with an
+ *   option that speaks of the padded layouts (L2 window, list order, another
+ *   accumulation form than plain atomics), keep to the two.  It takes 7 images
+ *   of the column layout, whose columns hold every slice a ray of the scanner
+ *   can enter: about 7 images where the scanner is as long as the image, at
+ *   most 4 images and 4 M floats each (a layout that would need more, or whose
+ *   lists of nx + ny crossings exceed 40 KB, is not made), and a queue of up to
+ *   256 B for each (angle, r).  Creation leaves out what does not fit on the
+ *   device: first 4 of the 7 (projections and DivideAndBackproject then walk bin
+ *   by bin), then the layout.  Passes with several rays a bin take a column
+ *   layout of their own (3 more images) where the radial samples are few (their
+ *   crossing lists, 20 (nx + ny + 11) bytes a sample, fit 40 KB, and enough
+ *   blocks with them an SM); their projections and backprojections walk bin by
+ *   bin.  The launch options below (block size, persistent, gather segments)
+ *   shape the two layouts' kernel; the column layout's has one shape and takes
+ *   any setting.
  * APIRL_OPT_KERNEL_TIMING (default 0): record CUDA events around the fused
  *   kernel of every pass; apirl_projector_kernel_ms returns the last one.
  * APIRL_OPT_EM_BLOCK (default 128): threads per block of the fused kernel
@@ -286,7 +296,12 @@ apirl_status apirl_count_steps(apirl_projector* p, int subset, int nsubsets, int
 apirl_status apirl_project(apirl_projector* p, const float* d_image, float* d_sino, int subset, int nsubsets,
                            void* stream);
 /* SiddonProjector::Backproject: d_image += A^T d_sino (:444-568 for 3D, :34-87
- * for 2D).  Accumulates into d_image, as the reference does. */
+ * for 2D).  Accumulates into d_image, as the reference does.  A sensitivity or
+ * geometry image is better made by the two calls below, as the drivers make
+ * theirs: on the column layout the rounding errors of sums of nearly equal
+ * terms (a sinogram of ones or factors) go the same way LOR by LOR, which
+ * moves a likelihood that holds x . G_s by 1e-8 of its value against their
+ * 6e-9 (the image's own error is 2.2e-7 and 2.15e-7 of its values). */
 apirl_status apirl_backproject(apirl_projector* p, const float* d_sino, float* d_image, int subset, int nsubsets,
                                void* stream);
 /* d_image += A^T 1 over the subset's bins: the sensitivity image without
