@@ -110,3 +110,34 @@ def test_long_backprojection_of_few_values(oracle, rings, share):
     for _ in range(2):
         got = P.backproject(t(v), torch.zeros(ig.n_voxels, dtype=torch.float32, device=DEV)).cpu().numpy()
         assert rel(got, want) <= 1e-5
+
+
+@pytest.mark.parametrize("packed", [False, True])
+@pytest.mark.parametrize("rings,max_rd,n_proj,n_r,nsub", [LANES[1], LANES[3], SMALL[0]])
+def test_zero_count_image_and_packed_counts(oracle, rings, max_rd, n_proj, n_r, nsub, packed):
+    """The same with the zero-count image's likelihood, counts and additive term
+    packed to the subset, and the backprojection alone added to what bp holds."""
+    ig = ImageGeom(27, 24, 2 * rings - 1, 2.5, 2.5, 2.0)
+    sg = Sino3DGeom.span1(n_proj, n_r, rings, 45.0, rings * 4.0, 120.0, max_rd)
+    rng = np.random.default_rng(rings + packed)
+    x0 = (rng.random(ig.n_voxels, dtype=np.float32) + 0.5).astype(np.float32)
+    sub = nsub - 1 if nsub > 1 else -1
+    meas = ((rng.random(sg.n_bins) < 0.05) * (1 + rng.poisson(2.0, sg.n_bins))).astype(np.float32)
+    add = (rng.random(sg.n_bins, dtype=np.float32) + 0.5).astype(np.float32)
+    pick = lambda v: np.ascontiguousarray(v.reshape(sg.n_sinos, n_proj, n_r)[:, max(sub, 0)::nsub, :]).reshape(-1)
+    m, est = pick(meas), (oracle.project_3d(sg, ig, x0, sub, nsub) + pick(add)).astype(np.float32)
+    ratio = oracle.backproject_3d(sg, ig, oracle.inverse_divide(m, est), sub, nsub, threads=1)
+    e64 = est.astype(np.float64)
+    want_lik = float(np.sum(m * np.log(e64) - e64))
+    P = ap.SiddonProjector(ig, sg)
+    zeros = lambda: torch.zeros(ig.n_voxels, dtype=torch.float32, device=DEV)
+    c, a = (t(m), t(pick(add))) if packed else (t(meas), t(add))
+    zimg, zadd = zeros(), torch.zeros(1, dtype=torch.float64, device=DEV)
+    P.zero_count_image(c, zimg, sub, nsub, add=a, zero_add=zadd, counts_packed=packed)
+    x, lik = t(x0), torch.zeros(1, dtype=torch.float64, device=DEV)
+    sens = np.ones(ig.n_voxels, np.float32)
+    P.em_pass_sparse(c, x, zeros(), t(sens), zimg, sub, nsub, add=a, zero_add=zadd, counts_packed=packed, lik=lik)
+    assert rel(x.cpu().numpy(), oracle.update(x0, ratio, sens, np.float32(0), True)) <= 1e-5
+    assert abs(lik.item() - want_lik) <= 1e-6 * max(abs(want_lik), float(np.sum(e64)))
+    bp = P.em_project_backproject(c, t(x0), t(x0), sub, nsub, add=a, counts_packed=packed, zimg=zimg, zero_add=zadd)
+    assert rel(bp.cpu().numpy(), x0.astype(np.float64) + ratio) <= 1e-5
