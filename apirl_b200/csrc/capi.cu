@@ -317,7 +317,7 @@ apirl_status finish_create(apirl_projector* p, apirl_projector** out) {
     const size_t line = (size_t)apirl::col_direct_lors(p->g), deferred = std::min(lors, line);
     at_item = b.add(queue ? deferred * sizeof(uint2) : 0);
     at_list = b.add(queue ? deferred * apirl::kColFew * sizeof(uint16_t) : 0);
-    const size_t direct = std::min(apirl::col_direct(p->host.n_sinos), p->host.n_sinos);
+    const size_t direct = apirl::col_direct_room(p->host.n_sinos);
     at_bins = b.add(queue && lors > line ? lors * direct * sizeof(unsigned) : 0);
     at_zeros = b.bytes;
     at_pad = b.add(4 * pv * sizeof(float));

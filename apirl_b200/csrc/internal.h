@@ -150,6 +150,7 @@ cudaError_t launch_planar_update(const ImgGeom& g, const PlanarBuffers& pl, int 
 // project / backproject / full pass, padded pair -> column walk: 10 sinograms
 // 98 / 128 / 150 -> 120 / 97 / 176, 19: 155 / 186 / 219 -> 123 / 112 / 187,
 // 44: 315 / 398 / 405 -> 179 / 237 / 311, 91: 616 / 787 / 764 -> 247 / 374 / 474.
+// (Projections and full passes ask further: project_cols, wide_pass, capi.cu.)
 constexpr int kColMinSinos = 16;
 // Sizes only; z_ends: the axial end points of the scanner's LORs.
 ColBuffers col_layout(const ImgGeom& g, const float* z_ends, int n_ends);
@@ -167,6 +168,9 @@ inline int64_t col_direct_lors(const ImgGeom& g) {
   return lors < 8000 ? lors : 8000;
 }
 inline int col_direct(int n_sinos) { return n_sinos > 4 * kColFew ? kColFew : n_sinos <= 40 ? 40 : kColFew / 2; }
+// The bins a LOR that a projector of n_sinos makes room for: what any shard of
+// them may queue (40 of up to 40 sinograms is more than 32 of 41 to 256).
+inline int col_direct_room(int n_sinos) { return n_sinos > 4 * kColFew ? kColFew : n_sinos < 40 ? n_sinos : 40; }
 struct ColQueue {
   unsigned* n = nullptr;
   uint2* item = nullptr;

@@ -106,7 +106,9 @@ int apirl_sino3d_ring_z(const apirl_sino3d_geom* sino, float* h_z);
  * (recon/inc/SiddonProjector.h:43-47).  Builds the LOR end-point table on the
  * host with the reference's float expressions
  * (Sinogram2DinCylindrical3Dpet::getPointsFromLor, .cpp:216-266) and keeps it,
- * the per-sinogram ring z and scratch space resident on `device`. */
+ * the per-sinogram ring z, scratch space and the layouts of its passes
+ * (APIRL_OPT_DUAL_LAYOUT; in 2D six padded copies of the slice) resident on
+ * `device`, in one allocation, which leaves out the layouts that do not fit. */
 apirl_status apirl_projector_create_2d(const apirl_image_geom* img, const apirl_sino2d_geom* sino, int device,
                                        apirl_projector** out);
 apirl_status apirl_projector_create_3d(const apirl_image_geom* img, const apirl_sino3d_geom* sino, int device,

@@ -141,3 +141,25 @@ def test_zero_count_image_and_packed_counts(oracle, rings, max_rd, n_proj, n_r, 
     assert abs(lik.item() - want_lik) <= 1e-6 * max(abs(want_lik), float(np.sum(e64)))
     bp = P.em_project_backproject(c, t(x0), t(x0), sub, nsub, add=a, counts_packed=packed, zimg=zimg, zero_add=zadd)
     assert rel(bp.cpu().numpy(), x0.astype(np.float64) + ratio) <= 1e-5
+
+
+@pytest.mark.parametrize("first,n", [(0, 40), (8, 33), (20, 21), (0, 41)])
+def test_shards_with_nearly_every_bin(oracle, first, n):
+    """Shards whose LORs go to the queue whole, of a projector that would queue fewer bins a LOR itself."""
+    ig = ImageGeom(27, 24, 41, 2.5, 2.5, 2.0)
+    sg = Sino3DGeom.span1(100, 90, 41, 45.0, 82.0, 120.0, 0)
+    rng = np.random.default_rng(n)
+    x0 = (rng.random(ig.n_voxels, dtype=np.float32) + 0.5).astype(np.float32)
+    est = oracle.project_3d(sg, ig, x0)
+    meas = (1 + rng.poisson(2.0, sg.n_bins)).astype(np.float32).reshape(41, -1)
+    inside = np.zeros_like(meas)
+    inside[first:first + n] = meas[first:first + n]
+    want = oracle.backproject_3d(sg, ig, oracle.inverse_divide(inside.reshape(-1), est), threads=1)
+    P = ap.SiddonProjector(ig, sg)
+    P.set_option(_lib.APIRL_OPT_SPARSE_IMAGE, _lib.APIRL_SPARSE_GEOMETRY)
+    P.set_shard(first, n)
+    zeros = lambda: torch.zeros(ig.n_voxels, dtype=torch.float32, device=DEV)
+    G = P.backproject_ones(zeros())
+    for _ in range(2):
+        bp = P.em_project_backproject(t(meas.reshape(-1)), t(x0), zeros(), zimg=G)
+        assert rel(bp.cpu().numpy(), want) <= 1e-5

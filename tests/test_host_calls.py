@@ -1,5 +1,8 @@
 """The calls that the library's host code makes, on a runtime without a GPU
 (fake_gpu.py): what a projector writes is in place before a stream reads it."""
+import os
+import subprocess
+
 import pytest
 
 import fake_gpu
@@ -332,3 +335,23 @@ _lib.check(lib.apirl_backproject(P.h, D, D, -1, 1, S))
 done(fake.log())''')
     assert any("k_scatter_cols_direct" in l for l in log) == want
     assert any(l.startswith("memset 0x9990") for l in log) == want  # the queue is emptied on the caller's stream
+
+
+def test_queue_has_room_for_every_shard(tmp_path):
+    exe = str(tmp_path / "queue_room_check")
+    subprocess.run(["g++", "-std=c++17", "-I/usr/local/cuda/include", "-I" + os.path.join(fake_gpu.ROOT, "apirl_b200", "csrc"),
+                    os.path.join(fake_gpu.HERE, "queue_room_check.cpp"), "-o", exe], check=True)
+    r = subprocess.run([exe], capture_output=True, text=True)
+    assert r.returncode == 0, r.stdout
+
+
+def test_queue_is_sized_by_its_room(gpu):
+    """41 sinograms over 9000 LORs: 40 bins a LOR (a shard of 40), 4 bytes each, beyond what 8000 LORs' block has."""
+    sizes = gpu('''
+out = []
+for n_proj in (80, 100):    # 7200 and 9000 LORs: without and with the queue of bins
+    fake.clear()
+    P = ap.SiddonProjector(ImageGeom(27, 24, 31, 2.5, 2.5, 2.0), Sino3DGeom.span1(n_proj, 90, 41, 45.0, 64.0, 120.0, 0))
+    out.append([int(l.split()[2]) for l in fake.log() if l.startswith("malloc")][0])
+done(out)''')
+    assert sizes[1] - sizes[0] >= 9000 * 40 * 4
