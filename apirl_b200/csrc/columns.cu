@@ -82,21 +82,22 @@ struct ColScatterDivide {
 // bins with v == 0 add nothing) and, with vest, DivideAndBackproject's
 // (:669-683: (seg * v) / e where e != 0, else seg * v).  The ratio v / e is
 // formed once per bin where v and the ratio are far from the ends of the
-// float range, and per segment elsewhere.  look >= 0 (a thread a sinogram): a
-// LOR without values is left before its crossings are listed, and the bins of
-// one with at most `look` go to the queue (k_scatter_cols_direct).
+// float range, and per segment elsewhere.  LOOK (a thread a sinogram): a LOR
+// without values is left before its crossings are listed, and the bins of one
+// with at most `few` go to the queue (k_scatter_cols_direct).
+template <bool LOOK>
 __global__ void __launch_bounds__(kColBlock, kColBlocks) k_scatter_cols(ImgGeom g, ColDims d, LorTable t, SubsetSel s,
                                                                         const float* __restrict__ vin,
                                                                         const float* __restrict__ vest,
-                                                                        float* __restrict__ acc, int look,
+                                                                        float* __restrict__ acc, int few,
                                                                         ColQueue queue) {
   const ColLor lor = col_lor(t, s, blockIdx.x);
-  if (look >= 0) {
+  if (LOOK) {
     const int gl = threadIdx.x;
     const bool any = gl < t.n_sinos && __ldg(vin + ((int64_t)gl * s.nk + lor.k) * t.n_r + lor.l) != 0.f;
     const int n = __syncthreads_count(any);
     if (n == 0) return;
-    if (n <= look) {
+    if (n <= few) {
       const unsigned mask = __ballot_sync(0xffffffffu, any), lane = threadIdx.x & 31;
       unsigned slot = 0;
       if (lane == 0 && mask) slot = atomicAdd(queue.n + 1, (unsigned)__popc(mask));
@@ -605,8 +606,9 @@ cudaError_t launch_scatter_cols(const ImgGeom& g, const ColBuffers& c, const Lor
   const bool queued = look && !vest && queue.bins && (double)lors * (g.nx + g.ny) >= 1e7 && lors * t.n_sinos <= INT_MAX;
   cudaError_t e;
   if (queued && (e = cudaMemsetAsync(queue.n + 1, 0, sizeof(unsigned), st)) != cudaSuccess) return e;
-  k_scatter_cols<<<(unsigned)lors, block_of(t), col_smem(g.nx, g.ny), st>>>(
-      g, dims_of(g, c), t, s, vin, vest, acc, queued ? kColDirectBack : look ? 0 : -1, queue);
+  auto kernel = look ? k_scatter_cols<true> : k_scatter_cols<false>;
+  kernel<<<(unsigned)lors, block_of(t), col_smem(g.nx, g.ny), st>>>(g, dims_of(g, c), t, s, vin, vest, acc,
+                                                                   queued ? kColDirectBack : 0, queue);
   if ((e = cudaGetLastError()) != cudaSuccess || !queued) return e;
   int dev = 0, sms = 0;
   if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
